@@ -139,11 +139,13 @@ void f32Exponents(rhgpu_ctx* c) {
    c->f32b.scaleJ = std::ldexp(1.0, c->kJ);
 }
 
+// mover list, sized and called as the fast path's (fastMoverBuffers): between steps only
 int f32MoverBuffers(rhgpu_ctx* c) {
    long long tot = 0;
    for (int s = 0; s < c->ns; ++s) tot += c->f32[s].capOf[c->f32[s].cur];
    const long long want = moverListSize(tot);
    if (want > c->f32b.moverCap) {
+      RH_CUDA(cudaStreamSynchronize(c->stream));
       cudaFree(c->f32b.movers);
       c->f32b.movers = nullptr;
       c->f32b.moverCap = 0;
@@ -333,11 +335,13 @@ int f32RelayoutNext(rhgpu_ctx* c, unsigned mask) {
       if (rc) return rc;
    }
    RH_CUDA(cudaStreamSynchronize(c->stream));
-   return f32MoverBuffers(c);
+   return RHGPU_OK;
 }
 
 int f32Push(rhgpu_ctx* c) {
    int rc = f32Init(c);
+   // a relayout of the last step may have grown the particle storage
+   if (!rc) rc = f32MoverBuffers(c);
    if (rc) return rc;
    c->timestep += 1;
    if (c->P.initial_flow_through_period < c->t && c->useIFT) c->useIFT = 0;

@@ -137,12 +137,15 @@ long long moverListSize(long long slots) {
    return std::max(1LL << 20, std::min(slots / 4, std::max(slots / 16, 1LL << 27)));
 }
 
-// mover list: moverListSize of all slots
+// mover list: moverListSize of all slots. Called between steps only (at an
+// upload or fill and before a push): inside one, the list and the sort buffers
+// hold the movers that a relayout makes room for
 int fastMoverBuffers(rhgpu_ctx* c) {
    long long tot = 0;
    for (int s = 0; s < c->ns; ++s) tot += c->seg[s].capOf[c->seg[s].cur];
    const long long want = moverListSize(tot);
    if (want > c->fb.moverCap) {
+      RH_CUDA(cudaStreamSynchronize(c->stream));
       cudaFree(c->fb.movers);
       c->fb.movers = nullptr;
       c->fb.moverCap = 0;
@@ -269,7 +272,7 @@ int fastRelayoutNext(rhgpu_ctx* c, unsigned mask) {
       if (rc) return rc;
    }
    RH_CUDA(cudaStreamSynchronize(c->stream));
-   return fastMoverBuffers(c);
+   return RHGPU_OK;
 }
 
 int fastUpload(rhgpu_ctx* c, int s, const uint32_t* counts, const double* particles, long long n) {
@@ -479,6 +482,8 @@ int launchPushDeposit(rhgpu_ctx* c, const FastSpecies& FS, const PushParams& pp)
 }
 
 int fastPush(rhgpu_ctx* c) {
+   // a relayout of the last step may have grown the particle storage
+   if (const int rc = fastMoverBuffers(c)) return rc;
    c->timestep += 1;
    if (c->P.initial_flow_through_period < c->t && c->useIFT) c->useIFT = 0;
    PushParams pp;

@@ -371,3 +371,36 @@ def test_chapman_ionosphere_source(lib):
     assert np.all(p[:, 3] * xg + p[:, 4] * yg + p[:, 5] * zg >= 0)
     assert math.isclose(p[0, 6], 1e24 * cfg.dt / 400.0, rel_tol=1e-12)
     assert np.mean(xg > 0) > 0.8
+
+
+@pytest.mark.parametrize("path", [abi.PATH_FAST, abi.PATH_FP32])
+def test_storage_growth_inside_a_step_keeps_the_movers(lib, path):
+    """A source fills an empty species past its storage: the relayout that makes
+    room runs while the step's movers wait to be placed, with enough slots that
+    the mover list would grow too. The run equals one whose storage was reserved
+    before it started, particle for particle."""
+    wind = cf.Population(name="H+", density=N0, velocity=(-U, 0.0, 0.0), temperature=T, ppc=40.0, accelerate=False)
+    src = dataclasses.replace(wind, name="src", ppc=200.0)
+    cfg = dataclasses.replace(box(nx=40, ny=52, nz=52), populations=[wind, src])
+    out = []
+    for reserve in (True, False):
+        ctx = abi.Context(lib, cf.params(cfg), cf.species(cfg))
+        try:
+            ctx.set_path(path)
+            grid = cf.init_grid(cfg)
+            for n in ("faceB", "cellB", "nodeEta"):
+                ctx.upload_array(n, grid[n])
+            ctx.upload_cell_flags(grid["flags"])
+            ctx.fill_uniform(0, wind.density, wind.temperature, wind.velocity, wind.ppc, seed=3)
+            if reserve:
+                ctx.fill_uniform(1, src.density, src.temperature, src.velocity, 60.0, seed=4)
+            ctx.upload_particles(1, np.zeros(cfg.ncells, dtype=np.uint32), np.zeros((0, 7)))
+            ctx.set_injectors(cf.solar_wind_injectors(cfg, seed=5)[1:])
+            ctx.step(6)
+            out.append([ctx.download_particles(s) for s in range(2)] + [ctx.download_array("cellRhoQi")])
+            assert ctx.num_particles(1) == ctx.injection_counters()[1]["macroparticles"] > 500000
+        finally:
+            ctx.close()
+    for (ca, pa), (cb, pb) in zip(out[0][:2], out[1][:2]):
+        assert np.array_equal(ca, cb) and np.array_equal(pa.view(np.uint64), pb.view(np.uint64))
+    assert np.array_equal(out[0][2].view(np.uint64), out[1][2].view(np.uint64))
