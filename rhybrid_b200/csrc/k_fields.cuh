@@ -145,12 +145,12 @@ __global__ void k_ext_bc(GridInfo g, Fields f, FieldParams fp, const int* ext, i
 __global__ void __launch_bounds__(128, 8) k_node_fused(GridInfo g, Fields f, FieldParams fp, unsigned long long* cnt);
 
 // ---- the cell pass, its node stencil in shared memory ------------------------------------------
-// A block of 32 x 4 cells marches NT_Z planes along z; the node layers k - 1
+// A block of 32 x 4 cells marches nzb planes along z; the node layers k - 1
 // and k that a plane of cells reads (nodeJ, nodeRhoQi, nodeE over 33 x 5 nodes
 // from (i0 - 1, j0 - 1)) sit in a ring of three layer slots, the next one
 // copied in with cp.async while the current plane is computed, so every node
 // value is loaded once per block instead of once per cell reading it.
-constexpr int NT_X = 32, NT_Y = 4, NT_Z = 8;
+constexpr int NT_X = 32, NT_Y = 4, NT_Z = 8;   // NT_Z: most planes of a block
 constexpr int NT_LX = NT_X + 1, NT_LY = NT_Y + 1;
 constexpr int CT_ARR = 7;    // nodeJ x 3, nodeRhoQi, nodeE x 3
 constexpr int CT_LAYER = CT_ARR * NT_LY * NT_LX;
@@ -278,14 +278,26 @@ __device__ __forceinline__ void cellFromStencil(const GridInfo& g, const Fields&
    }
 }
 
+// planes per block: fewer than NT_Z while the grid would leave SMs without one
+// resident wave of blocks (8 of 27.7 KB per SM); a plane more per block saves
+// the layer shared with the next block but is a plane more in a serial march.
+// (32^3 cells, 32 blocks of 8 planes: 60 us; 256 blocks of one: 17 us. 61 x 83 x
+// 70 cells: 62 -> 40 us. Grids that fill a wave with 8 planes keep them.)
+inline int cellPlanes(const GridInfo& g) {
+   const long long cols = (long long)((g.nx + NT_X - 1) / NT_X) * ((g.ny + NT_Y - 1) / NT_Y);
+   int nzb = NT_Z;
+   while (nzb > 1 && cols * ((g.nz + nzb - 1) / nzb) < 148 * 8) nzb >>= 1;
+   return nzb;
+}
+
 template <bool FARADAY>
 __global__ void __launch_bounds__(NT_X * NT_Y) k_cell_tiled(GridInfo g, Fields f, FieldParams fp, int useEp,
-                                                            unsigned long long* cnt) {
+                                                            int nzb, unsigned long long* cnt) {
    extern __shared__ __align__(16) double ctLayers[];
    const int tx = threadIdx.x, ty = threadIdx.y;
-   const int i0 = blockIdx.x * NT_X, j0 = blockIdx.y * NT_Y, k0 = blockIdx.z * NT_Z;
+   const int i0 = blockIdx.x * NT_X, j0 = blockIdx.y * NT_Y, k0 = blockIdx.z * nzb;
    const int i = i0 + tx, j = j0 + ty;
-   const int nk = min(NT_Z, g.nz - k0);
+   const int nk = min(nzb, g.nz - k0);
    const bool mine = i < g.nx && j < g.ny;
    ctStage(g, f, ctLayers, i0, j0, k0 - 1);
    ctStage(g, f, ctLayers + CT_LAYER, i0, j0, k0);

@@ -197,13 +197,14 @@ int fieldsAll(rhgpu_ctx* c) {
    c->gridAvgCounter += 1;
    {
       RH_TIME(c, "k_cell_tiled");
-      const dim3 NG((g.nx + NT_X - 1) / NT_X, (g.ny + NT_Y - 1) / NT_Y, (g.nz + NT_Z - 1) / NT_Z);
+      const int nzb = cellPlanes(g);
+      const dim3 NG((g.nx + NT_X - 1) / NT_X, (g.ny + NT_Y - 1) / NT_Y, (g.nz + nzb - 1) / nzb);
       if (smooth)
          k_cell_tiled<false><<<NG, dim3(NT_X, NT_Y), CT_SMEM, c->stream>>>(g, c->f, c->fp, c->P.use_electron_pressure,
-                                                                          c->cntU);
+                                                                          nzb, c->cntU);
       else
          k_cell_tiled<true><<<NG, dim3(NT_X, NT_Y), CT_SMEM, c->stream>>>(g, c->f, c->fp, c->P.use_electron_pressure,
-                                                                         c->cntU);
+                                                                         nzb, c->cntU);
       RH_LAUNCHED(c);
    }
    if (c->next > 0) RH_FIELD_LAUNCH(k_ext_cell_neumann3, EB, 128, g, c->f.cellUe, c->ext, c->next);
