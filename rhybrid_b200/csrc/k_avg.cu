@@ -15,38 +15,15 @@ __global__ void k_deposit_gather_avg(GridInfo g, const double* S, double* nSum, 
    for (int l = 0; l < 3; ++l) vSum[l * N + n] = v[1 + l];
 }
 
-__global__ void k_fast_avg_movers(GridInfo g, FastGeom fg, FastSpecies FS, const Mover* mv, long long n, unsigned mask,
-                                  FastBufs fb) {
-   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= n) return;
-   const Mover& M = mv[t];
-   if (!(M.lx & (MOVER_DEPOSIT | MOVER_AVG)) || !((mask >> M.species) & 1u)) return;
-   moverAdd128<false>(g, fg, FS, M, fb.MMlo, fb.MMhi, fb.scaleR, fb.scaleJ, nullptr);
-}
-
-__global__ void k_fast_avg_gather(GridInfo g, FastGeom fg, FastBufs fb, double hiR, double loR, double hiJ, double loJ,
-                                  double* nSum, double* vSum) {
-   RH_CELL_PROLOGUE
-   const bool bnd = g.per[0] ? (fg.nseg > 1 && i % SEG == 0) : ((i + 1) % SEG == 0);
-   const int gb = g.per[0] ? i / SEG : (i + 1) / SEG;
-   double v[4];
-   for (int qq = 0; qq < 4; ++qq) {
-      const int uyy = dualU(j - (qq & 1), g.ny, g.per[1]);
-      const int uzz = dualU(k - (qq >> 1), g.nz, g.per[2]);
-      const long long row = (long long)uyy + (long long)fg.nd[1] * uzz;
-      const double* rp = fb.RP + (((long long)qq * fg.nrows + row) * g.nx + i) * 4;
-      const double* rb = fb.RPB + (((long long)qq * fg.nrows + row) * fg.nseg + gb) * 4;
-      for (int l = 0; l < 4; ++l) {
-         double r = rp[l];
-         if (bnd) r = r + rb[l];
-         v[l] = qq == 0 ? r : v[l] + r;
-      }
-   }
-   v[0] += fixedToDouble(fb.MMlo[n], fb.MMhi[n], hiR, loR);
-   for (int l = 0; l < 3; ++l) v[1 + l] += fixedToDouble(fb.MMlo[(1 + l) * N + n], fb.MMhi[(1 + l) * N + n], hiJ, loJ);
-   for (int l = 0; l < 4; ++l) { fb.MMlo[l * N + n] = 0ull; fb.MMhi[l * N + n] = 0ull; }
-   nSum[n] += v[0];
-   for (int l = 0; l < 3; ++l) vSum[l * N + n] += v[1 + l];
+__global__ void __launch_bounds__(2 * GA_CELLS)
+k_fast_avg_gather(GridInfo g, FastGeom fg, FastBufs fb, double hiR, double loR, double hiJ, double loJ, double* nSum,
+                  double* vSum) {
+   RH_GATHER_PROLOGUE
+   double* const s0 = (h ? vSum + N : nSum) + n;
+   double* const s1 = (h ? vSum + 2 * N : vSum) + n;
+   const double2 v = gatherMoments<double>(g, fg, fb, i, j, k, h, n, h ? hiJ : hiR, h ? loJ : loR, hiJ, loJ);
+   *s0 += v.x;
+   *s1 += v.y;
 }
 
 __global__ void k_avg_output(long long N, double* nSum, double* vSum, double q, double dV, double inv, double* nOut,

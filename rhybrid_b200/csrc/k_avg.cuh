@@ -15,7 +15,7 @@
 //                          CIC records counting-sorted by dual cell and summed
 //                          per (dual cell, corner) as the push kernel does,
 //                          out as row partials
-//   k_fast_avg_movers      the population's deposits that went through the
+//   k_mover_pass           the population's deposits that went through the
 //                          mover list (left their segment; or deposited in it
 //                          and then removed by a boundary), as exact
 //                          fixed-point sums
@@ -134,14 +134,11 @@ k_fast_avg_deposit(GridInfo gIn, FastGeom fg, FastSpecies FS, unsigned mask, Fas
    segPartialsOut(g, fg, fb, s_rec, row, gseg, u0, u1, a0, a1, a2, a3);
 }
 
-// fast path: the movers of the species in `mask` that were deposited this step
-__global__ void k_fast_avg_movers(GridInfo g, FastGeom fg, FastSpecies FS, const Mover* mv, long long n, unsigned mask,
-                                  FastBufs fb);
-
 // fast path: row partials + fixed-point part added to the population's sums;
 // the fixed-point sums restart
-__global__ void k_fast_avg_gather(GridInfo g, FastGeom fg, FastBufs fb, double hiR, double loR, double hiJ, double loJ,
-                                  double* nSum, double* vSum);
+__global__ void __launch_bounds__(2 * GA_CELLS)
+k_fast_avg_gather(GridInfo g, FastGeom fg, FastBufs fb, double hiR, double loR, double hiJ, double loJ, double* nSum,
+                  double* vSum);
 
 // output step of one population (operator_userdata.cpp:182-211): n = sum/(q dV)*inv,
 // v = current sum / charge sum where the charge sum is positive, else 0; the sums

@@ -4,46 +4,6 @@
 
 namespace rh {
 
-__global__ void k_f32_mig_place(F32Set FS, long long NS, long long nb, const Mover32* mv, const unsigned* order,
-                                const unsigned* bkt, const long long* off, long long n) {
-   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (q >= n) return;
-   const long long b = bkt[q];
-   if (b >= nb) return;
-   const int s = (int)(b / NS);
-   const long long S = b % NS;
-   const F32Species& SS = FS.st[s];
-   const long long pos = SS.base[S] + SS.nxt.cnt[S] + (q - off[b]);
-   const Mover32& M = mv[order[q]];
-   SS.nxt.cell[pos] = M.cell;
-   for (int e = 0; e < 3; ++e) { SS.nxt.o[e][pos] = M.o[e]; SS.nxt.v[e][pos] = M.v[e]; }
-}
-
-__global__ void k_f32_mover_deposit(GridInfo g, FastGeom fg, F32Set FS, F32Bufs fb, long long n) {
-   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= n) return;
-   const Mover32& M = fb.movers[t];
-   if (!(M.lx & MOVER_DEPOSIT)) return;
-   const int s = M.species;
-   const long long row = M.dest / fg.nseg;
-   const int vx = (int)(M.dest % fg.nseg) * SEG + (M.lx & 0xff);
-   const int vy = (int)(row % fg.nd[1]), vz = (int)(row / fg.nd[1]);
-   const int bx = dualB(vx, g.per[0]), by = dualB(vy, g.per[1]), bz = dualB(vz, g.per[2]);
-   float o[3] = {M.o[0], M.o[1], M.o[2]};
-   float w8[8];
-   cicWeightsF(o, FS.wqRel[s], w8);
-   const long long N = g.N;
-   for (int q = 0; q < 8; ++q) {
-      int dxc = bx + (q & 1), dyc = by + ((q >> 1) & 1), dzc = bz + ((q >> 2) & 1);
-      if (!wrapc(dxc, g.nx, g.per[0]) || !wrapc(dyc, g.ny, g.per[1]) || !wrapc(dzc, g.nz, g.per[2])) continue;
-      const long long dc = cidx(g, dxc, dyc, dzc);
-      add128(&fb.MMlo[dc], &fb.MMhi[dc], (double)w8[q], fb.scaleR);
-      for (int l = 0; l < 3; ++l)
-         add128(&fb.MMlo[(1 + l) * N + dc], &fb.MMhi[(1 + l) * N + dc], (double)(w8[q] * M.v[l]), fb.scaleJ);
-      fb.touched[dc] = 1;
-   }
-}
-
 __global__ void k_f32_cell_keys(FastGeom fg, F32Buf B, const long long* base, const long long* first, unsigned* key,
                                 unsigned long long* slots) {
    const long long S = blockIdx.x;

@@ -71,9 +71,8 @@ struct Mover32 {
 struct F32Bufs {
    float* RP;                  // 4 planes x nrows x nx x 4
    float* RPB;                 // 4 planes x nrows x nseg x 4
-   unsigned long long* MMlo;   // 4 x N (shared with the FP64 fast path)
+   unsigned long long* MMlo;   // N x 4 (shared with the FP64 fast path)
    unsigned long long* MMhi;
-   unsigned char* touched;
    const unsigned char* segInner;   // per segment: an obstacle cell within reach (shared with the fast path)
    Mover32* movers;
    unsigned long long* nmovers;
@@ -474,65 +473,38 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
    }
 }
 
-// mover order[q] to slot q - off[bucket] after its bucket's stayers (bucket nb: not placed)
-__global__ void k_f32_mig_place(F32Set FS, long long NS, long long nb, const Mover32* mv, const unsigned* order,
-                                const unsigned* bkt, const long long* off, long long n);
+// corner o's four deposits of one mover (k_mover_pass): cicWeightsF's products, in its order
+__device__ __forceinline__ void moverTerms(const GridInfo&, const F32Set& FS, const Mover32& M, int o, double t[4]) {
+   float f[3];
+   for (int a = 0; a < 3; ++a) {
+      const float w = M.o[a] + 0.5f - (float)halfSf(M.o[a]);
+      f[a] = (o >> a) & 1 ? w : 1.0f - w;
+   }
+   const float w = f[0] * f[1] * f[2] * FS.wqRel[M.species];
+   t[0] = (double)w;
+   for (int l = 0; l < 3; ++l) t[1 + l] = (double)(w * M.v[l]);
+}
+__device__ __forceinline__ void placeMover(const F32Species& SS, long long slot, const Mover32& M) {
+   SS.nxt.cell[slot] = M.cell;
+#pragma unroll
+   for (int e = 0; e < 3; ++e) { SS.nxt.o[e][slot] = M.o[e]; SS.nxt.v[e][slot] = M.v[e]; }
+}
 
-// CIC contributions of the particles that left their segment, exact fixed-point sums
-__global__ void k_f32_mover_deposit(GridInfo g, FastGeom fg, F32Set FS, F32Bufs fb, long long n);
-
-// cell moments: four row partials (+ boundary partials) + fixed-point part, times (w q)_0 / dV
+// cell moments: gatherMoments times (w q)_0 / dV, and the rho clamp
 template <bool GC>   // GC: also count the rho clamp per cell (grid counters on)
-__global__ void k_f32_gather(GridInfo g, Fields f, FastGeom fg, F32Bufs fb, double hiR, double loR, double hiJ,
-                             double loJ, double scale, double minRho, unsigned long long* cnt) {
-   RH_CELL_PROLOGUE
-   const bool bnd = g.per[0] ? (fg.nseg > 1 && i % SEG == 0) : ((i + 1) % SEG == 0);
-   const int gb = g.per[0] ? i / SEG : (i + 1) / SEG;
-   // every load first (one wait for memory), the same sums in the same order
-   float4 rp[4];
-   float rb[4][4];
-#pragma unroll
-   for (int qq = 0; qq < 4; ++qq) {
-      const int uyy = dualU(j - (qq & 1), g.ny, g.per[1]);
-      const int uzz = dualU(k - (qq >> 1), g.nz, g.per[2]);
-      const long long row = (long long)uyy + (long long)fg.nd[1] * uzz;
-      rp[qq] = *reinterpret_cast<const float4*>(fb.RP + (((long long)qq * fg.nrows + row) * g.nx + i) * 4);
-      if (bnd) {
-         const float* pb = fb.RPB + (((long long)qq * fg.nrows + row) * fg.nseg + gb) * 4;
-#pragma unroll
-         for (int l = 0; l < 4; ++l) rb[qq][l] = pb[l];
-      }
-   }
-   const unsigned tw = fb.touched[n];
-   unsigned long long mlo[4], mhi[4];
-#pragma unroll
-   for (int l = 0; l < 4; ++l) { mlo[l] = fb.MMlo[l * N + n]; mhi[l] = fb.MMhi[l * N + n]; }
-   double v[4];
-#pragma unroll
-   for (int qq = 0; qq < 4; ++qq) {
-      const float rv[4] = {rp[qq].x, rp[qq].y, rp[qq].z, rp[qq].w};
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-         float r = rv[l];
-         if (bnd) r = r + rb[qq][l];
-         v[l] = qq == 0 ? (double)r : v[l] + (double)r;
-      }
-   }
-   if (tw) {
-      v[0] += fixedToDouble(mlo[0], mhi[0], hiR, loR);
-      for (int l = 0; l < 3; ++l) v[1 + l] += fixedToDouble(mlo[1 + l], mhi[1 + l], hiJ, loJ);
-   }
-   // every cell's sums cleared for the next step, touched or not: whole sectors
-   // written (a warp writing only its touched cells leaves partly written
-   // sectors, which cost a read-modify-write each; 0.48 -> 0.17 ms per step)
-   for (int l = 0; l < 4; ++l) { fb.MMlo[l * N + n] = 0ull; fb.MMhi[l * N + n] = 0ull; }
-   double rho = v[0] * scale;
-   bool clamp = false;
-   if (rho < minRho) { rho = minRho; clamp = true; }
+__global__ void __launch_bounds__(2 * GA_CELLS)
+k_f32_gather(GridInfo g, Fields f, FastGeom fg, F32Bufs fb, double hiR, double loR, double hiJ, double loJ,
+             double scale, double minRho, unsigned long long* cnt) {
+   RH_GATHER_PROLOGUE
+   double2 v = gatherMoments<float>(g, fg, fb, i, j, k, h, n, h ? hiJ : hiR, h ? loJ : loR, hiJ, loJ);
+   v.x *= scale;
+   v.y *= scale;
+   const bool clamp = h == 0 && v.x < minRho;
+   if (clamp) v.x = minRho;
    countIf(clamp, &cnt[CNT_MIN_CELL_RHO]);
    if (GC) gridCount(f, GC_CELL_MIN_RHOQI, N, n, clamp);
-   f.cellRho[n] = rho;
-   for (int l = 0; l < 3; ++l) f.cellJi[l * N + n] = v[1 + l] * scale;
+   (h ? f.cellJi + N : f.cellRho)[n] = v.x;
+   (h ? f.cellJi + 2 * N : f.cellJi)[n] = v.y;
 }
 
 // ---- upload / download / relayout ----------------------------------------------------------

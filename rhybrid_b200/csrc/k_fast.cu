@@ -4,47 +4,50 @@
 
 namespace rh {
 
-__global__ void k_fast_mover_deposit(GridInfo g, FastGeom fg, FastSpecies FS, FastBufs fb, long long n) {
-   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= n) return;
-   const Mover& M = fb.movers[t];
-   if (!(M.lx & MOVER_DEPOSIT)) return;
-   moverAdd128<true>(g, fg, FS, M, fb.MMlo, fb.MMhi, fb.scaleR, fb.scaleJ, fb.touched);
-}
-
-__global__ void k_fast_fold_boundary(GridInfo g, FastGeom fg, FastBufs fb) {
-   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   const long long nrows = fg.nrows;
-   if (t >= 16 * nrows * fg.nseg) return;
-   const int m = (int)(t & 3);
-   const long long e = t >> 2;                    // (qq, row, gseg)
-   const int gseg = (int)(e % fg.nseg);
-   const long long qr = e / fg.nseg;              // qq * nrows + row
-   if (!(g.per[0] ? fg.nseg > 1 : gseg >= 1)) return;
-   const int x = g.per[0] ? gseg * SEG : gseg * SEG - 1;
-   if (x >= g.nx) return;
-   double* rp = fb.RP + (qr * g.nx + x) * 4 + m;
-   *rp = *rp + fb.RPB[e * 4 + m];
-}
-
-__global__ void k_fast_mig_place(FastSpecies FS, long long NS, long long nb, const Mover* mv, const unsigned* order,
-                                 const unsigned* bkt, const long long* off, long long n) {
-   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (q >= n) return;
-   const long long b = bkt[q];
-   if (b >= nb) return;
-   const int s = (int)(b / NS);
-   const long long S = b % NS;
-   const SegSpecies& SS = FS.st[s];
-   const long long pos = SS.base[S] + SS.nxt.cnt[S] + (q - off[b]);
-   const Mover& M = mv[order[q]];
-   for (int e = 0; e < 7; ++e) SS.nxt.a[e][pos] = M.s[e];
-   SS.nxt.lx[pos] = (unsigned char)(M.lx & 0xff);
-}
-
 __global__ void k_mig_large_list(const int* inc, long long nb, unsigned* large, int* nlarge) {
    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (b < nb && inc[b] > MIG_SMALL) large[atomicAdd(nlarge, 1)] = (unsigned)b;
+   if (b < nb && inc[b] > MIG_RANK) large[atomicAdd(nlarge, 1)] = (unsigned)b;
+}
+
+__global__ void __launch_bounds__(MIG_LARGE_THREADS) k_mig_order_large(const int* inc, const long long* off,
+                                                                        unsigned long long* klist, unsigned* vlist,
+                                                                        const unsigned* large, const int* nlarge) {
+   __shared__ unsigned long long skey[MIG_LARGE];
+   __shared__ unsigned sval[MIG_LARGE];
+   const int n = *nlarge;
+   for (int q = blockIdx.x; q < n; q += gridDim.x) {
+      const unsigned b = large[q];
+      const int k = inc[b];
+      unsigned long long* const kl = klist + off[b];
+      unsigned* const vl = vlist + off[b];
+      int m = 1;
+      while (m < k) m <<= 1;
+      for (int i = threadIdx.x; i < m; i += MIG_LARGE_THREADS) {
+         skey[i] = i < k ? kl[i] : ~0ull;
+         sval[i] = i < k ? vl[i] : ~0u;
+      }
+      __syncthreads();
+      for (int size = 2; size <= m; size <<= 1) {
+         for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int i = threadIdx.x; i < m; i += MIG_LARGE_THREADS) {
+               const int j = i ^ stride;
+               if (j > i) {
+                  const bool up = (i & size) == 0;
+                  const unsigned long long ki = skey[i], kj = skey[j];
+                  const unsigned vi = sval[i], vj = sval[j];
+                  const bool gt = ki > kj || (ki == kj && vi > vj);
+                  if (gt == up) {
+                     skey[i] = kj; skey[j] = ki;
+                     sval[i] = vj; sval[j] = vi;
+                  }
+               }
+            }
+            __syncthreads();
+         }
+      }
+      for (int i = threadIdx.x; i < k; i += MIG_LARGE_THREADS) vl[i] = sval[i];
+      __syncthreads();
+   }
 }
 
 __global__ void k_fast_seg_of(GridInfo g, FastGeom fg, const double* aos, const int* pcell, long long n,

@@ -28,9 +28,10 @@
 //                        corner, moment) in FP64, one thread per (dual cell,
 //                        corner). Particles that leave the segment go to the
 //                        mover list.
-//   k_fast_mover_deposit the movers' CIC contributions as exact 128-bit
-//                        fixed-point sums (order-independent)
-//   k_mig_*, k_fast_mig_place  placement of the movers after the stayers of their
+//   k_mover_pass         the movers' CIC contributions as exact 128-bit
+//                        fixed-point sums (order-independent), and their count
+//                        per destination
+//   k_mig_*              placement of the movers after the stayers of their
 //                        destination segment, in (source segment, index) order
 //   k_fast_gather        cell moments from the four row partials (+ the segment
 //                        boundary partial) + the fixed-point part, then /dV and
@@ -84,12 +85,19 @@ constexpr int MOVER_DEPOSIT = 1 << 8;   // deposits its CIC contributions (fixed
 constexpr int MOVER_PLACE = 1 << 9;     // is stored in the destination segment
 constexpr int MOVER_AVG = 1 << 10;      // removed after its in-segment deposit: population averages only
 
+// state of a step's migration, read back by the host once per step
+struct MigCtl {
+   unsigned long long nm;       // movers of the step (may exceed the list: an error)
+   unsigned long long placed;   // list positions given to destinations
+   unsigned over;               // bit s: arrivals of species s do not fit some segment
+   int maxInc;                  // most arrivals of one destination, where above MIG_RANK
+};
+
 struct FastBufs {
    double* RP;                 // row partials: 4 planes x nrows x nx x 4
    double* RPB;                // segment-boundary partials: 4 planes x nrows x nseg x 4
-   unsigned long long* MMlo;   // 4 x N
-   unsigned long long* MMhi;   // 4 x N
-   unsigned char* touched;     // byte per cell: MM nonzero this step
+   unsigned long long* MMlo;   // N x 4: a cell's four sums in one 32-byte sector
+   unsigned long long* MMhi;   // N x 4
    const unsigned char* segInner;   // per segment: an obstacle (RHGPU_FLAG_INNER_PARTICLE) cell within reach
    Mover* movers;
    unsigned long long* nmovers;
@@ -780,103 +788,269 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
    segPartialsOut(g, fg, fb, sh.rec, row, gseg, u0, u1, a0, a1, a2, a3);
 }
 
-// CIC contributions of the particles that left their segment, as exact fixed-point sums (MM)
-// one mover's CIC contributions as exact fixed-point sums into lo/hi (4 x N),
-// marking the touched cells (TOUCH)
-template <bool TOUCH>
-__device__ __forceinline__ void moverAdd128(const GridInfo& g, const FastGeom& fg, const FastSpecies& FS, const Mover& M,
-                                            unsigned long long* lo, unsigned long long* hi, double scaleR, double scaleJ,
-                                            unsigned char* touched) {
-   const int s = M.species;
-   const long long row = M.dest / fg.nseg;
-   const int vx = (int)(M.dest % fg.nseg) * SEG + (M.lx & 0xff);
-   const int vy = (int)(row % fg.nd[1]), vz = (int)(row / fg.nd[1]);
-   const int bx = dualB(vx, g.per[0]), by = dualB(vy, g.per[1]), bz = dualB(vz, g.per[2]);
-   double st[7];
-   for (int a = 0; a < 7; ++a) st[a] = M.s[a];
-   double w8[8];
-   cicWeightsLocal(st[0], st[1], st[2], st[6] * FS.sp[s].q, g, w8);
-   const long long N = g.N;
-   for (int o = 0; o < 8; ++o) {
-      int dxc = bx + (o & 1), dyc = by + ((o >> 1) & 1), dzc = bz + ((o >> 2) & 1);
-      if (!wrapc(dxc, g.nx, g.per[0]) || !wrapc(dyc, g.ny, g.per[1]) || !wrapc(dzc, g.nz, g.per[2])) continue;
-      const long long dc = cidx(g, dxc, dyc, dzc);
-      add128(&lo[dc], &hi[dc], w8[o], scaleR);
-      for (int l = 0; l < 3; ++l) add128(&lo[(1 + l) * N + dc], &hi[(1 + l) * N + dc], w8[o] * st[3 + l], scaleJ);
-      if (TOUCH) touched[dc] = 1;   // a plain byte store: every writer stores the same value
+// corner o's four deposits (charge, current) of one mover: the weight products
+// of cicWeightsLocal, in its order
+__device__ __forceinline__ void moverTerms(const GridInfo& g, const FastSpecies& FS, const Mover& M, int o, double t[4]) {
+   const double dx = g.dx, x = M.s[0], y = M.s[1], z = M.s[2];
+   const double x0 = (halfS(x, dx) - 1 + 0.5) * dx, y0 = (halfS(y, dx) - 1 + 0.5) * dx, z0 = (halfS(z, dx) - 1 + 0.5) * dx;
+   const double w_x = divDx(x - x0, g), w_y = divDx(y - y0, g), w_z = divDx(z - z0, g);
+   const double fx = o & 1 ? w_x : 1 - w_x, fy = o & 2 ? w_y : 1 - w_y, fz = o & 4 ? w_z : 1 - w_z;
+   t[0] = fx * fy * fz * (M.s[6] * FS.sp[M.species].q);
+   for (int l = 0; l < 3; ++l) t[1 + l] = t[0] * M.s[3 + l];
+}
+
+// One pass over the movers: the contributions of those whose flags meet `need`
+// (species in smask) as exact fixed-point sums into lo / hi, and, with inc, the
+// arrivals counted per destination, rank[m] being a mover's place in that count
+// (in any order; k_mig_place orders them).
+//
+// A warp takes four movers, one lane per corner; the 16 x 8 terms go through
+// shared memory so that each of four atomics of the warp covers one mover, the
+// four sums of a cell on adjacent lanes (one 32-byte sector, two for corners
+// adjacent in x). The pass is bound by those returning atomics: one thread per
+// mover with its 32 atomics in a row over four planes took 0.30 ms for 2.9e6
+// movers of the Mars run and 30-39 us for the few thousand of a 32^3 box, where
+// the chain of one thread is all there is.
+constexpr int MP_THREADS = 256;
+template <class MV, class SET>
+__global__ void __launch_bounds__(MP_THREADS)
+k_mover_pass(GridInfo g, FastGeom fg, SET FS, const MV* mv, const MigCtl* ctl, long long cap, int need, unsigned smask,
+             unsigned long long* lo, unsigned long long* hi, double scaleR, double scaleJ, int* inc, unsigned* rank) {
+   __shared__ long long term[MP_THREADS / 32][32][4];
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o = lane & 7;
+   const long long nm = min((long long)ctl->nm, cap);
+   const long long step = (long long)gridDim.x * (MP_THREADS / 8);
+   for (long long m0 = ((long long)blockIdx.x * (MP_THREADS / 32) + warp) * 4; m0 < nm; m0 += step) {
+      const long long m = m0 + (lane >> 3);
+      const MV& M = mv[m < nm ? m : m0];
+      const int flags = m < nm ? M.lx : 0;
+      const int dest = (int)M.dest;
+      if (inc && o == 0 && (flags & MOVER_PLACE)) rank[m] = (unsigned)atomicAdd(&inc[M.species * (int)fg.NS + dest], 1);
+      int dc = -1;
+      if ((flags & need) && ((smask >> M.species) & 1u)) {
+         const int row = dest / fg.nseg;
+         const int vx = (dest - row * fg.nseg) * SEG + (flags & 0xff);
+         const int vz = row / fg.nd[1], vy = row - vz * fg.nd[1];
+         int cx = dualB(vx, g.per[0]) + (o & 1), cy = dualB(vy, g.per[1]) + ((o >> 1) & 1), cz = dualB(vz, g.per[2]) + (o >> 2);
+         if (wrapc(cx, g.nx, g.per[0]) && wrapc(cy, g.ny, g.per[1]) && wrapc(cz, g.nz, g.per[2])) {
+            dc = (int)cidx(g, cx, cy, cz);
+            double t[4];
+            moverTerms(g, FS, M, o, t);
+            term[warp][lane][0] = __double2ll_rn(t[0] * scaleR);
+#pragma unroll
+            for (int l = 1; l < 4; ++l) term[warp][lane][l] = __double2ll_rn(t[l] * scaleJ);
+         }
+      }
+      __syncwarp();
+      unsigned long long old[4];
+      long long iv[4], at[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+         const int src = 8 * r + (lane >> 2);
+         const int d = __shfl_sync(0xffffffffu, dc, src);
+         at[r] = d < 0 ? -1 : 4LL * d + (lane & 3);
+         if (d >= 0) {
+            iv[r] = term[warp][src][lane & 3];
+            old[r] = atomicAdd(&lo[at[r]], (unsigned long long)iv[r]);
+         }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+         if (at[r] < 0) continue;
+         const unsigned long long h = (iv[r] < 0 ? ~0ull : 0ull) + (old[r] + (unsigned long long)iv[r] < old[r] ? 1ull : 0ull);
+         if (h) atomicAdd(&hi[at[r]], h);
+      }
+      __syncwarp();
    }
 }
 
-__global__ void k_fast_mover_deposit(GridInfo g, FastGeom fg, FastSpecies FS, FastBufs fb, long long n);
+// Two threads per cell, two moments each (charge and Jx, Jy and Jz): a cell's
+// four row partials and fixed-point sums are one vector per thread, consecutive
+// over a warp's 16 cells. The fixed-point sums are cleared after the gather by a
+// fill (fixedClear), not here: a kernel that reads and writes them in place
+// moves the same bytes but took 0.13 to 1.08 ms on the Mars run (3.07e6 cells,
+// FP32 and FP64 form), depending on its vector width and resident warps, where
+// the gather and the fill together take 0.13 (FP32) and 0.15 (FP64).
+constexpr int GA_CELLS = 64;   // cells of a block of 128 threads, consecutive in x
+inline dim3 gatherGrid(const GridInfo& g) { return dim3((g.nx + GA_CELLS - 1) / GA_CELLS, g.ny, g.nz); }
+#define RH_GATHER_PROLOGUE                                        \
+   const int i = blockIdx.x * GA_CELLS + (threadIdx.x >> 1);      \
+   const int h = threadIdx.x & 1;                                 \
+   const int j = blockIdx.y, k = blockIdx.z;                      \
+   if (i >= g.nx) return;                                         \
+   const long long n = cidx(g, i, j, k);                          \
+   const long long N = g.N;
 
-// the segment-boundary partials folded into the row partials of their cells
-// (RP += RPB, the addition the gather would make): the gather then reads four
-// row partials per cell and nothing else
-__global__ void k_fast_fold_boundary(GridInfo g, FastGeom fg, FastBufs fb);
+template <class T> struct Vec2;
+template <> struct Vec2<double> { using type = double2; };
+template <> struct Vec2<float> { using type = float2; };
 
-// destination moments: four row partials (boundary partials folded in) +
-// fixed-point part, then finalize. The touched mark, the four row partials
-// (16-byte loads) and the fixed-point sums are all requested before any sum:
-// most cells are touched by some mover, and waiting for the touched mark
-// before loading the sums would add a second dependent round trip.
-template <bool GC>   // GC: also count the rho clamp per cell (grid counters on)
-__global__ void k_fast_gather(GridInfo g, Fields f, FastGeom fg, FastBufs fb, double hiR, double loR, double hiJ,
-                              double loJ, double minRho, unsigned long long* cnt) {
-   RH_CELL_PROLOGUE
-   const unsigned tw = fb.touched[n];
-   double2 rp[4][2];
+// moments 2h and 2h + 1 of cell (i, j, k): the four row partials, each with its
+// segment's boundary partial where the cell's other dual cell is in another
+// segment, and the fixed-point part (scales hi/lo S0, S1). A cell that no mover
+// touched adds +0.0, which changes no sum here (a sum of products started at
+// +0.0 is never -0.0).
+template <class T, class B>
+__device__ __forceinline__ double2 gatherMoments(const GridInfo& g, const FastGeom& fg, const B& fb, int i, int j, int k,
+                                                 int h, long long n, double hiS0, double loS0, double hiS1, double loS1) {
+   using V = typename Vec2<T>::type;
+   const bool bnd = g.per[0] ? (fg.nseg > 1 && i % SEG == 0) : ((i + 1) % SEG == 0);
+   const int gb = g.per[0] ? i / SEG : (i + 1) / SEG;
+   V r[4], rb[4];
 #pragma unroll
    for (int qq = 0; qq < 4; ++qq) {
       const int uyy = dualU(j - (qq & 1), g.ny, g.per[1]);
       const int uzz = dualU(k - (qq >> 1), g.nz, g.per[2]);
-      const long long row = (long long)uyy + (long long)fg.nd[1] * uzz;
-      const double2* p2 = reinterpret_cast<const double2*>(fb.RP + (((long long)qq * fg.nrows + row) * g.nx + i) * 4);
-      rp[qq][0] = p2[0];
-      rp[qq][1] = p2[1];
+      const long long row = (long long)qq * fg.nrows + uyy + (long long)fg.nd[1] * uzz;
+      r[qq] = reinterpret_cast<const V*>(fb.RP)[(row * g.nx + i) * 2 + h];
+      if (bnd) rb[qq] = reinterpret_cast<const V*>(fb.RPB)[(row * fg.nseg + gb) * 2 + h];
    }
-   double v[4] = {rp[0][0].x, rp[0][0].y, rp[0][1].x, rp[0][1].y};
+   const ulonglong2 lo = reinterpret_cast<const ulonglong2*>(fb.MMlo)[2 * n + h];
+   const ulonglong2 hi = reinterpret_cast<const ulonglong2*>(fb.MMhi)[2 * n + h];
+   double2 v = make_double2(0.0, 0.0);
 #pragma unroll
-   for (int qq = 1; qq < 4; ++qq) {
-      v[0] = v[0] + rp[qq][0].x;
-      v[1] = v[1] + rp[qq][0].y;
-      v[2] = v[2] + rp[qq][1].x;
-      v[3] = v[3] + rp[qq][1].y;
+   for (int qq = 0; qq < 4; ++qq) {
+      if (bnd) { r[qq].x = r[qq].x + rb[qq].x; r[qq].y = r[qq].y + rb[qq].y; }
+      v.x = qq == 0 ? (double)r[0].x : v.x + (double)r[qq].x;
+      v.y = qq == 0 ? (double)r[0].y : v.y + (double)r[qq].y;
    }
-   unsigned long long mlo[4], mhi[4];
-#pragma unroll
-   for (int l = 0; l < 4; ++l) {
-      mlo[l] = fb.MMlo[l * N + n];
-      mhi[l] = fb.MMhi[l * N + n];
-   }
-   if (tw) {
-      v[0] += fixedToDouble(mlo[0], mhi[0], hiR, loR);
-      for (int l = 0; l < 3; ++l) v[1 + l] += fixedToDouble(mlo[1 + l], mhi[1 + l], hiJ, loJ);
-   }
-   // every cell's sums cleared for the next step, touched or not: whole sectors
-   // written (a warp writing only its touched cells leaves partly written
-   // sectors, which cost a read-modify-write each; 0.48 -> 0.17 ms per step)
-   for (int l = 0; l < 4; ++l) { fb.MMlo[l * N + n] = 0ull; fb.MMhi[l * N + n] = 0ull; }
-   double rho = v[0] / g.dV;
-   bool clamp = false;
-   if (rho < minRho) { rho = minRho; clamp = true; }
+   v.x += fixedToDouble(lo.x, hi.x, hiS0, loS0);
+   v.y += fixedToDouble(lo.y, hi.y, hiS1, loS1);
+   return v;
+}
+
+// destination moments: gatherMoments, then /dV and the rho clamp
+template <bool GC>   // GC: also count the rho clamp per cell (grid counters on)
+__global__ void __launch_bounds__(2 * GA_CELLS)
+k_fast_gather(GridInfo g, Fields f, FastGeom fg, FastBufs fb, double hiR, double loR, double hiJ, double loJ,
+              double minRho, unsigned long long* cnt) {
+   RH_GATHER_PROLOGUE
+   double2 v = gatherMoments<double>(g, fg, fb, i, j, k, h, n, h ? hiJ : hiR, h ? loJ : loR, hiJ, loJ);
+   v.x /= g.dV;
+   v.y /= g.dV;
+   const bool clamp = h == 0 && v.x < minRho;
+   if (clamp) v.x = minRho;
    countIf(clamp, &cnt[CNT_MIN_CELL_RHO]);
    if (GC) gridCount(f, GC_CELL_MIN_RHOQI, N, n, clamp);
-   f.cellRho[n] = rho;
-   for (int l = 0; l < 3; ++l) f.cellJi[l * N + n] = v[1 + l] / g.dV;
+   (h ? f.cellJi + N : f.cellRho)[n] = v.x;
+   (h ? f.cellJi + 2 * N : f.cellJi)[n] = v.y;
 }
 
 // ---- mover placement ------------------------------------------------------------------------
-template <class MV>
-__global__ void k_fast_mig_count(const MV* mv, long long n, long long NS, int* inc) {
-   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= n || !(mv[t].lx & MOVER_PLACE)) return;
-   atomicAdd(&inc[(long long)mv[t].species * NS + mv[t].dest], 1);
+// The arrivals of a destination (species, segment) bucket are stored after its
+// stayers in the order of their mover keys (source segment, index in it). Each
+// bucket's arrivals are listed together (k_mig_buckets gives every bucket a
+// stretch of the list, in whatever order the buckets come, and k_mig_list fills
+// it), and a mover's place is the number of smaller keys in its bucket, which
+// k_mig_place counts, one thread per list position, so that a warp reads the
+// same one or two buckets. The three kernels do nothing when the step needs the
+// host (no room in a segment, or a bucket above MIG_RANK arrivals), which reads
+// MigCtl after it has launched the rest of the step and then relays out, orders
+// the large buckets one block each (k_mig_order_large) or, past MIG_LARGE, all
+// movers by two radix sorts (by key, then stably by bucket), and places.
+// (Counts, a scan over all buckets, a second counting pass, one thread ordering
+// each bucket and two host round trips in between took 83-93 us for the 32^3 box
+// and 0.26 ms for the Mars run.)
+constexpr int MIG_RANK = 256;     // arrivals of a bucket whose order is found by counting
+constexpr int MIG_LARGE = 2048;   // arrivals one block orders in shared memory (k_mig_order_large)
+
+// every bucket with arrivals: its stretch of the list (one reservation per
+// warp), whether its segment has room, and the size of the buckets above MIG_RANK
+template <class SET>
+__global__ void k_mig_buckets(SET FS, int NS, const int* inc, long long* off, MigCtl* ctl) {
+   const int b = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+   const int k = b < FS.ns * NS ? inc[b] : 0;
+   int x = k;
+#pragma unroll
+   for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+   }
+   unsigned long long base = 0;
+   if (lane == 31 && x > 0) base = atomicAdd(&ctl->placed, (unsigned long long)x);
+   base = __shfl_sync(0xffffffffu, base, 31);
+   if (k == 0) return;
+   off[b] = (long long)base + (x - k);
+   const int s = b / NS, S = b - s * NS;
+   if (FS.st[s].base[S] + FS.st[s].nxt.cnt[S] + k > FS.st[s].base[S + 1]) atomicOr(&ctl->over, 1u << s);
+   if (k > MIG_RANK) atomicMax(&ctl->maxInc, k);
 }
-// Placement order of the arrivals of a destination (species, segment) bucket:
-// by mover key (source segment, index in it). The movers are sorted by key and
-// then, stably, by bucket (radix sorts on the host side); these kernels prepare
-// the sort keys, check the room of every bucket, place the movers (one thread
-// each) after the bucket's stayers, and add the arrivals to the counts.
+// the step needs the host before its movers can be placed
+__device__ __forceinline__ bool migHeld(const MigCtl* ctl, long long cap, int force) {
+   return (long long)ctl->nm > cap || (!force && (ctl->over != 0 || ctl->maxInc > MIG_RANK));
+}
+template <class MV>
+__global__ void k_mig_list(const MV* mv, const MigCtl* ctl, long long cap, int force, int NS, const long long* off,
+                           const unsigned* rank, unsigned long long* klist, unsigned* vlist) {
+   if (migHeld(ctl, cap, force)) return;
+   const long long nm = (long long)ctl->nm;
+   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nm; t += (long long)gridDim.x * blockDim.x) {
+      if (!(mv[t].lx & MOVER_PLACE)) continue;
+      const long long q = off[mv[t].species * NS + (int)mv[t].dest] + rank[t];
+      klist[q] = mv[t].key;
+      vlist[q] = (unsigned)t;
+   }
+}
+// one mover into a slot of its destination's next buffer
+__device__ __forceinline__ void placeMover(const SegSpecies& SS, long long slot, const Mover& M) {
+#pragma unroll
+   for (int e = 0; e < 7; ++e) SS.nxt.a[e][slot] = M.s[e];
+   SS.nxt.lx[slot] = (unsigned char)(M.lx & 0xff);
+}
+template <class MV, class SET>
+__global__ void k_mig_place(SET FS, const MV* mv, const MigCtl* ctl, long long cap, int force, int NS, const int* inc,
+                            const long long* off, const unsigned long long* klist, const unsigned* vlist) {
+   if (migHeld(ctl, cap, force)) return;
+   const long long n = (long long)ctl->placed;
+   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+      const unsigned t = vlist[q];
+      const MV& M = mv[t];
+      const int S = (int)M.dest, b = M.species * NS + S;
+      const int k = inc[b];
+      const long long first = off[b];
+      long long before = q - first;   // a bucket above MIG_RANK is in order already
+      if (k <= MIG_RANK) {
+         const unsigned long long key = klist[q];
+         before = 0;
+         for (int j = 0; j < k; ++j) {
+            const unsigned long long kj = klist[first + j];
+            before += kj < key || (kj == key && vlist[first + j] < t) ? 1 : 0;
+         }
+      }
+      const auto& SS = FS.st[M.species];
+      placeMover(SS, SS.base[S] + SS.nxt.cnt[S] + before, M);
+   }
+}
+// the arrivals added to the segments' counts, and cleared for the next step
+template <class SET>
+__global__ void k_mig_counts(SET FS, const MigCtl* ctl, long long cap, int force, int NS, int* inc) {
+   if (migHeld(ctl, cap, force)) return;
+   const int b = blockIdx.x * blockDim.x + threadIdx.x;
+   if (b >= FS.ns * NS || inc[b] == 0) return;
+   FS.st[b / NS].nxt.cnt[b % NS] += inc[b];
+   inc[b] = 0;
+}
+// whether every species has room for its arrivals (after a relayout)
+template <class SET>
+__global__ void k_mig_check(SET FS, int NS, const int* inc, MigCtl* ctl) {
+   const int b = blockIdx.x * blockDim.x + threadIdx.x;
+   if (b >= FS.ns * NS || inc[b] == 0) return;
+   const int s = b / NS, S = b - s * NS;
+   if (FS.st[s].base[S] + FS.st[s].nxt.cnt[S] + inc[b] > FS.st[s].base[S + 1]) atomicOr(&ctl->over, 1u << s);
+}
+
+// the buckets with more than MIG_RANK arrivals, appended to large[] (count in *nlarge)
+__global__ void k_mig_large_list(const int* inc, long long nb, unsigned* large, int* nlarge);
+
+// each bucket of large[] (at most MIG_LARGE arrivals) ordered by one block: its
+// stretch of the list sorted bitonically by (key, mover index) in shared memory
+constexpr int MIG_LARGE_THREADS = 256;
+__global__ void __launch_bounds__(MIG_LARGE_THREADS) k_mig_order_large(const int* inc, const long long* off,
+                                                                        unsigned long long* klist, unsigned* vlist,
+                                                                        const unsigned* large, const int* nlarge);
+
+// the radix order: sort keys of every mover (bucket nb: not placed), and mover
+// order[q] to slot q - off[bucket] after its bucket's stayers
 template <class MV>
 __global__ void k_mig_sort_keys(const MV* mv, long long n, long long NS, long long nb, unsigned long long* key,
                                 unsigned* val, unsigned* bkt) {
@@ -886,113 +1060,17 @@ __global__ void k_mig_sort_keys(const MV* mv, long long n, long long NS, long lo
    val[t] = (unsigned)t;
    bkt[t] = (mv[t].lx & MOVER_PLACE) ? (unsigned)((long long)mv[t].species * NS + mv[t].dest) : (unsigned)nb;
 }
-template <class SET>
-__global__ void k_mig_check(SET FS, long long NS, const int* inc, int* overflow) {
-   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (b >= (long long)FS.ns * NS || inc[b] == 0) return;
-   const int s = (int)(b / NS);
-   const long long S = b % NS;
-   // one bit per species whose arrivals do not fit (relaid alone)
-   if (FS.st[s].base[S] + FS.st[s].nxt.cnt[S] + inc[b] > FS.st[s].base[S + 1]) atomicOr((unsigned*)overflow, 1u << s);
-}
-template <class SET>
-__global__ void k_mig_counts(SET FS, long long NS, int* inc) {
-   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (b >= (long long)FS.ns * NS || inc[b] == 0) return;
-   FS.st[(int)(b / NS)].nxt.cnt[b % NS] += inc[b];
-   inc[b] = 0;
-}
-// small buckets: the arrivals of each bucket listed (in any order) at off[b] by
-// k_mig_bucket, then one thread per bucket orders them by key (insertion sort)
-// into order[], the same order as the sorts
-template <class MV>
-__global__ void k_mig_bucket(const MV* mv, long long n, long long NS, const long long* off, int* fill,
-                             unsigned* list) {
-   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (t >= n || !(mv[t].lx & MOVER_PLACE)) return;
-   const long long b = (long long)mv[t].species * NS + mv[t].dest;
-   const int k = atomicAdd(&fill[b], 1);
-   list[off[b] + k] = (unsigned)t;
-}
-constexpr int MIG_SMALL = 64;     // arrivals a bucket's own thread orders
-constexpr int MIG_LARGE = 2048;   // arrivals one block orders in shared memory (k_mig_order_large)
-template <class MV>
-__global__ void k_mig_order_small(const MV* mv, long long nb, const int* inc, const long long* off, unsigned* list,
-                                  unsigned* bkt) {
-   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+template <class MV, class SET>
+__global__ void k_mig_place_order(SET FS, int NS, long long nb, const MV* mv, const unsigned* order, const unsigned* bkt,
+                                  const long long* off, long long n) {
+   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+   if (q >= n) return;
+   const long long b = bkt[q];
    if (b >= nb) return;
-   const int k = inc[b];
-   if (k > MIG_SMALL) return;   // k_mig_order_large
-   unsigned* bk = list + off[b];
-   for (int a = 1; a < k; ++a) {
-      const unsigned t = bk[a];
-      const unsigned long long key = mv[t].key;
-      int c = a;
-      for (; c > 0 && mv[bk[c - 1]].key > key; --c) bk[c] = bk[c - 1];
-      bk[c] = t;
-   }
-   for (int a = 0; a < k; ++a) bkt[off[b] + a] = (unsigned)b;
+   const int s = (int)b / NS, S = (int)b - s * NS;
+   const auto& SS = FS.st[s];
+   placeMover(SS, SS.base[S] + SS.nxt.cnt[S] + (q - off[b]), mv[order[q]]);
 }
-
-// the buckets with more than MIG_SMALL arrivals, appended to large[] (count in *nlarge)
-__global__ void k_mig_large_list(const int* inc, long long nb, unsigned* large, int* nlarge);
-
-// each bucket of large[] (at most MIG_LARGE arrivals) ordered by one block: its
-// arrivals' (key, mover index) sorted bitonically in shared memory, the order
-// the radix sorts give (by key; equal keys by mover index)
-constexpr int MIG_LARGE_THREADS = 256;
-template <class MV>
-__global__ void __launch_bounds__(MIG_LARGE_THREADS) k_mig_order_large(const MV* mv, const int* inc, const long long* off,
-                                                                        unsigned* list, unsigned* bkt,
-                                                                        const unsigned* large, const int* nlarge) {
-   __shared__ unsigned long long skey[MIG_LARGE];
-   __shared__ unsigned sval[MIG_LARGE];
-   const int n = *nlarge;
-   for (int q = blockIdx.x; q < n; q += gridDim.x) {
-      const unsigned b = large[q];
-      const int k = inc[b];
-      unsigned* bk = list + off[b];
-      int m = 1;
-      while (m < k) m <<= 1;
-      for (int i = threadIdx.x; i < m; i += MIG_LARGE_THREADS) {
-         if (i < k) {
-            skey[i] = mv[bk[i]].key;
-            sval[i] = bk[i];
-         } else {
-            skey[i] = ~0ull;
-            sval[i] = ~0u;
-         }
-      }
-      __syncthreads();
-      for (int size = 2; size <= m; size <<= 1) {
-         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = threadIdx.x; i < m; i += MIG_LARGE_THREADS) {
-               const int j = i ^ stride;
-               if (j > i) {
-                  const bool up = (i & size) == 0;
-                  const unsigned long long ki = skey[i], kj = skey[j];
-                  const unsigned vi = sval[i], vj = sval[j];
-                  const bool gt = ki > kj || (ki == kj && vi > vj);
-                  if (gt == up) {
-                     skey[i] = kj; skey[j] = ki;
-                     sval[i] = vj; sval[j] = vi;
-                  }
-               }
-            }
-            __syncthreads();
-         }
-      }
-      for (int i = threadIdx.x; i < k; i += MIG_LARGE_THREADS) {
-         bk[i] = sval[i];
-         bkt[off[b] + i] = b;
-      }
-      __syncthreads();
-   }
-}
-
-// mover order[q] to slot q - off[bucket] after its bucket's stayers (bucket nb: not placed)
-__global__ void k_fast_mig_place(FastSpecies FS, long long NS, long long nb, const Mover* mv, const unsigned* order,
-                                 const unsigned* bkt, const long long* off, long long n);
 
 // ---- upload / download / relayout support -----------------------------------------------------
 // segment and dual x (in the segment) of each uploaded particle (records grouped by cell)

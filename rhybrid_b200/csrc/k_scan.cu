@@ -46,19 +46,4 @@ __global__ void k_scan_add(long long* out, long long n, const long long* offs) {
    if (i < n) out[i] += offs[i / SCAN_TILE];
 }
 
-__global__ void k_max_int(const int* a, long long n, int* mx) {
-   __shared__ int wmax[8];
-   int m = 0;
-   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-      m = max(m, a[i]);
-#pragma unroll
-   for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-   if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-   __syncthreads();
-   if (threadIdx.x == 0) {
-      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = max(m, wmax[w]);
-      atomicMax(mx, m);
-   }
-}
-
 }  // namespace rh

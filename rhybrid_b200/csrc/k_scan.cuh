@@ -1,7 +1,6 @@
-// Exclusive prefix sums of 64-bit counts and the maximum of 32-bit counts:
-// the bookkeeping of the particle storage (cell and segment layouts, the
-// migration's arrival offsets). Integer sums, so any order gives the same
-// result; these replace library scans on the per-step path.
+// Exclusive prefix sums of 64-bit counts: the bookkeeping of the particle
+// storage (cell and segment layouts). Integer sums, so any order gives the
+// same result.
 //
 // A scan of n values in place: tiles of SCAN_TILE values (SCAN_THREADS threads
 // x SCAN_PER consecutive values each) are scanned by one block each, their
@@ -23,8 +22,5 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_tile(const long long* in,
 
 // out[i] += offs[tile of i]
 __global__ void k_scan_add(long long* out, long long n, const long long* offs);
-
-// *mx = max(*mx, a[0..n)) (*mx cleared by the caller)
-__global__ void k_max_int(const int* a, long long n, int* mx);
 
 }  // namespace rh

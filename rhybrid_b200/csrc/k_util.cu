@@ -25,10 +25,6 @@ __global__ void k_int_to64(const int* in, long long n, long long* out) {
    if (t == n) out[n] = 0;
 }
 
-__global__ void k_fill_u32(unsigned* a, long long n, unsigned v) {
-   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-   if (p < n) a[p] = v;
-}
 __global__ void k_gather_u32(const unsigned* src, const unsigned* idx, long long n, unsigned* dst) {
    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
    if (p < n) dst[p] = src[idx[p]];

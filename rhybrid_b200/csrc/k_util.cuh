@@ -14,8 +14,6 @@ __global__ void k_fill_pcell(long long N, const long long* start, int* pcell);
 __global__ void k_iota(unsigned* v, long long n);
 // out[t] = in[t] as 64 bits, out[n] = 0
 __global__ void k_int_to64(const int* in, long long n, long long* out);
-// a[p] = v
-__global__ void k_fill_u32(unsigned* a, long long n, unsigned v);
 // dst[p] = src[idx[p]]
 __global__ void k_gather_u32(const unsigned* src, const unsigned* idx, long long n, unsigned* dst);
 

@@ -333,12 +333,10 @@ int rhgpu_create(const rhgpu_params* params, int32_t n_species, const rhgpu_spec
    alloc((void**)&c->fb.RPB, sizeof(double) * 16 * fg.nrows * fg.nseg);
    alloc((void**)&c->fb.MMlo, sizeof(unsigned long long) * 4 * N);
    alloc((void**)&c->fb.MMhi, sizeof(unsigned long long) * 4 * N);
-   alloc((void**)&c->fb.touched, (size_t)N + 16);
    alloc((void**)&c->segInnerDev, (size_t)NS + 16);
    c->fb.segInner = c->segInnerDev;
-   alloc((void**)&c->fb.nmovers, sizeof(unsigned long long));
+   alloc((void**)&c->mig, sizeof(MigCtl));
    alloc((void**)&c->finc, sizeof(int) * nb);
-   alloc((void**)&c->ffill, sizeof(int) * nb);
    alloc((void**)&c->fmaxInc, sizeof(int));
    alloc((void**)&c->fcap, sizeof(long long) * (NS + 1));
    alloc((void**)&c->ffirst, sizeof(long long) * (NS + 1));
@@ -349,7 +347,13 @@ int rhgpu_create(const rhgpu_params* params, int32_t n_species, const rhgpu_spec
    alloc((void**)&c->fover, 2 * sizeof(unsigned long long));
    alloc((void**)&c->diagPart, sizeof(double) * DIAG_BLOCKS * DIAG_FS);
    if (!rc) {
-      // MM starts at zero; the gather clears it after reading
+      c->fb.nmovers = &c->mig->nm;
+      if (cudaMallocHost((void**)&c->migHost, sizeof(MigCtl)) != cudaSuccess ||
+          cudaEventCreateWithFlags(&c->migEvent, cudaEventDisableTiming) != cudaSuccess)
+         rc = fail(RHGPU_ERR_NOMEM, "create: migration state");
+   }
+   if (!rc) {
+      // MM starts at zero; cleared again after every gather
       if (cudaMemset(c->fb.MMlo, 0, sizeof(unsigned long long) * 4 * N) != cudaSuccess ||
           cudaMemset(c->fb.MMhi, 0, sizeof(unsigned long long) * 4 * N) != cudaSuccess ||
           cudaMemset(c->fb.RPB, 0, sizeof(double) * 16 * fg.nrows * fg.nseg) != cudaSuccess ||
@@ -420,11 +424,13 @@ int rhgpu_destroy(rhgpu_ctx* c) {
       cudaFree(h.base);
       cudaFree(h.baseAlt);
    }
-   cudaFree(c->fb.RP); cudaFree(c->fb.RPB); cudaFree(c->fb.MMlo); cudaFree(c->fb.MMhi); cudaFree(c->fb.touched); cudaFree(c->segInnerDev);
-   cudaFree(c->fb.nmovers); cudaFree(c->fb.movers);
+   cudaFree(c->fb.RP); cudaFree(c->fb.RPB); cudaFree(c->fb.MMlo); cudaFree(c->fb.MMhi); cudaFree(c->segInnerDev);
+   cudaFree(c->mig); cudaFree(c->fb.movers);
+   if (c->migHost) cudaFreeHost(c->migHost);
+   if (c->migEvent) cudaEventDestroy(c->migEvent);
    for (auto& h : c->inj) { cudaFree(h.cells); cudaFree(h.rates); cudaFree(h.list); }
    cudaFree(c->injCnt);
-   cudaFree(c->finc); cudaFree(c->fover); cudaFree(c->ffill); cudaFree(c->fmaxInc);
+   cudaFree(c->finc); cudaFree(c->fover); cudaFree(c->fmaxInc);
    cudaFree(c->mkey); cudaFree(c->mval); cudaFree(c->mbkt);
    cudaFree(c->sortTmp); cudaFree(c->fcap); cudaFree(c->ffirst); cudaFree(c->ftmp64); cudaFree(c->ftmpCellStart);
    cudaFree(c->ftmpInc64); cudaFree(c->foffInc); cudaFree(c->fsort); cudaFree(c->fsortSlots); cudaFree(c->flxTmp);
@@ -737,6 +743,7 @@ int rhgpu_push(rhgpu_ctx* c) {
    if (!c) return fail(RHGPU_ERR_ARG, "null context");
    RH_CUDA(cudaSetDevice(c->device));
    int rc = phasePush(c);
+   if (!rc) rc = migFinish(c);
    if (rc) return rc;
    return checkDeviceError(c);
 }
@@ -777,6 +784,9 @@ int rhgpu_step(rhgpu_ctx* c, int32_t nsteps) {
       if (!rc && c->dnOn) rc = dnApplyCtx(c);
       if (!rc) rc = phaseBoundaries(c);
       if (!rc) rc = fieldsAll(c);
+      // the movers' placement touches the particle storage only: the host looks
+      // at it once the gather and the field update are on the stream
+      if (!rc) rc = migFinish(c);
       if (rc) return rc;
    }
    return checkDeviceError(c);

@@ -71,7 +71,6 @@ int f32Init(rhgpu_ctx* c) {
    RH_CUDA(cudaMemset(c->f32b.RPB, 0, sizeof(float) * 16 * c->fg.nrows * c->fg.nseg));
    c->f32b.MMlo = c->fb.MMlo;
    c->f32b.MMhi = c->fb.MMhi;
-   c->f32b.touched = c->fb.touched;
    c->f32b.segInner = c->fb.segInner;
    c->f32b.nmovers = c->fb.nmovers;
    RH_CUDA(cudaDeviceSynchronize());   // the clears above run on the default stream
@@ -340,14 +339,14 @@ int f32RelayoutNext(rhgpu_ctx* c, unsigned mask) {
 
 int f32Push(rhgpu_ctx* c) {
    int rc = f32Init(c);
+   if (!rc) rc = migFinish(c);
    // a relayout of the last step may have grown the particle storage
    if (!rc) rc = f32MoverBuffers(c);
    if (rc) return rc;
    c->timestep += 1;
    if (c->P.initial_flow_through_period < c->t && c->useIFT) c->useIFT = 0;
-   const long long N = c->g.N, NS = c->fg.NS;
-   RH_CUDA(cudaMemsetAsync(c->fb.touched, 0, (size_t)N + 16, c->stream));
-   RH_CUDA(cudaMemsetAsync(c->fb.nmovers, 0, sizeof(unsigned long long), c->stream));
+   const long long NS = c->fg.NS;
+   if ((rc = migBegin(c)) != RHGPU_OK) return rc;
    {
       RH_TIME(c, "f32_push_deposit");
       const F32Set FS = f32Set(c);
@@ -371,43 +370,14 @@ int f32Push(rhgpu_ctx* c) {
       const int rc = injectAll(c, c->f32b.movers, c->f32b.moverCap);
       if (rc) return rc;
    }
-   unsigned long long nm = 0;
-   RH_CUDA(cudaMemcpyAsync(&nm, c->fb.nmovers, sizeof nm, cudaMemcpyDeviceToHost, c->stream));
-   RH_CUDA(cudaStreamSynchronize(c->stream));
-   if ((long long)nm > c->f32b.moverCap) return fail(RHGPU_ERR_CAPACITY, "mover list overflow");
-   if (nm > 0) {
-      {
-         RH_TIME(c, "f32_mover_deposit");
-         k_f32_mover_deposit<<<blocks1d(nm, 128), 128, 0, c->stream>>>(c->g, c->fg, f32Set(c), c->f32b, nm);
-         RH_LAUNCHED(c);
-      }
-      const long long nb = (long long)c->ns * NS;
-      int over = 0;
-      {
-         RH_TIME(c, "f32_migrate");
-         unsigned *order = nullptr, *bkt = nullptr;
-         int rc = migSort(c, c->f32b.movers, (long long)nm, f32Set(c), &order, &bkt, &over);
-         if (rc) return rc;
-         if (over) {
-            // some segments lack room for their arrivals: relayout with room for them
-            rc = f32RelayoutNext(c, (unsigned)over);
-            if (rc) return rc;
-            RH_CUDA(cudaMemsetAsync(c->fover, 0, sizeof(int), c->stream));
-            k_mig_check<<<blocks1d(nb, 256), 256, 0, c->stream>>>(f32Set(c), NS, c->finc, c->fover);
-            RH_LAUNCHED(c);
-            RH_CUDA(cudaMemcpyAsync(&over, c->fover, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            RH_CUDA(cudaStreamSynchronize(c->stream));
-            if (over) return fail(RHGPU_ERR_CAPACITY, "segment relayout did not make room");
-         }
-         k_f32_mig_place<<<blocks1d(nm, 256), 256, 0, c->stream>>>(f32Set(c), NS, nb, c->f32b.movers, order, bkt, c->foffInc,
-                                                                 (long long)nm);
-         RH_LAUNCHED(c);
-         k_mig_counts<<<blocks1d(nb, 256), 256, 0, c->stream>>>(f32Set(c), NS, c->finc);
-         RH_LAUNCHED(c);
-      }
+   {
+      RH_TIME(c, "f32_mover_deposit");
+      rc = moverPass(c, c->f32b.movers, c->f32b.moverCap, f32Set(c), MOVER_DEPOSIT, ~0u, c->f32b.MMlo, c->f32b.MMhi,
+                     c->f32b.scaleR, c->f32b.scaleJ, true);
+      if (rc) return rc;
    }
-   for (int s = 0; s < c->ns; ++s) c->f32[s].cur ^= 1;
-   return RHGPU_OK;
+   RH_TIME(c, "f32_migrate");
+   return migLaunch(c, c->f32b.movers, c->f32b.moverCap, f32Set(c));
 }
 
 int f32Gather(rhgpu_ctx* c) {
@@ -418,13 +388,13 @@ int f32Gather(rhgpu_ctx* c) {
    const double hiJ = std::ldexp(1.0, 64 - c->kJ), loJ = std::ldexp(1.0, -c->kJ);
    const double scale = f32WqRef(c) / c->g.dV;
    if (c->f.gc)
-      k_f32_gather<true><<<cellGrid(c->g), cellBlock(), 0, c->stream>>>(c->g, c->f, c->fg, c->f32b, hiR, loR, hiJ, loJ,
+      k_f32_gather<true><<<gatherGrid(c->g), 2 * GA_CELLS, 0, c->stream>>>(c->g, c->f, c->fg, c->f32b, hiR, loR, hiJ, loJ,
                                                                        scale, c->P.min_ion_charge_density, c->cntU);
    else
-      k_f32_gather<false><<<cellGrid(c->g), cellBlock(), 0, c->stream>>>(c->g, c->f, c->fg, c->f32b, hiR, loR, hiJ,
+      k_f32_gather<false><<<gatherGrid(c->g), 2 * GA_CELLS, 0, c->stream>>>(c->g, c->f, c->fg, c->f32b, hiR, loR, hiJ,
                                                                         loJ, scale, c->P.min_ion_charge_density, c->cntU);
    RH_LAUNCHED(c);
-   return RHGPU_OK;
+   return fixedClear(c, c->f32b.MMlo, c->f32b.MMhi);
 }
 
 }  // namespace rhh

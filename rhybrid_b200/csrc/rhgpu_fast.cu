@@ -161,80 +161,142 @@ int bitsFor(long long x) {
    return b;
 }
 
-// the arrivals of the nm movers: per destination (species, segment) bucket the
-// count (c->finc) and first position (c->foffInc), the movers sorted by bucket
-// and within it by key (*order, *bucket; bucket ns*NS = not placed), and
-// whether some bucket lacks room (*over). Buckets of at most MIG_SMALL arrivals
-// (the usual case) are ordered one thread per bucket, those of up to
-// MIG_LARGE one block per bucket; past that two stable radix sorts over all
-// movers (by key, then by bucket) give the same order.
+// blocks of `per` movers each for a pass over the step's movers: their number is
+// only known on the device, so the launch is sized by the last step's (the
+// kernels stride over the rest), up to a few resident waves
+unsigned moverBlocks(const rhgpu_ctx* c, int per) {
+   const long long most = 148 * 16;
+   if (c->migLast < 0) return (unsigned)most;
+   return (unsigned)std::min((c->migLast + c->migLast / 8 + 1024 + per - 1) / per, most);
+}
+
+// the migration state cleared for a push
+int migBegin(rhgpu_ctx* c) {
+   RH_CUDA(cudaMemsetAsync(c->mig, 0, sizeof(MigCtl), c->stream));
+   if (c->migDirty) RH_CUDA(cudaMemsetAsync(c->finc, 0, sizeof(int) * c->ns * c->fg.NS, c->stream));
+   c->migDirty = true;
+   return RHGPU_OK;
+}
+
+// k_mover_pass over a mover list; count: the arrivals per destination too
 template <class MV, class SET>
-int migSort(rhgpu_ctx* c, const MV* mv, long long nm, const SET& FS, unsigned** order, unsigned** bucket, int* over) {
-   const long long NS = c->fg.NS, nb = (long long)c->ns * NS;
-   if (nm > c->mcap) return fail(RHGPU_ERR_CAPACITY, "mover list larger than its sort buffers");
-   RH_CUDA(cudaMemsetAsync(c->finc, 0, sizeof(int) * nb, c->stream));
-   RH_CUDA(cudaMemsetAsync(c->fover, 0, sizeof(int), c->stream));
-   k_fast_mig_count<<<blocks1d(nm, 256), 256, 0, c->stream>>>(mv, nm, NS, c->finc);
+int moverPass(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS, int need, unsigned smask, unsigned long long* lo,
+              unsigned long long* hi, double scaleR, double scaleJ, bool count) {
+   k_mover_pass<<<moverBlocks(c, MP_THREADS / 8), MP_THREADS, 0, c->stream>>>(
+       c->g, c->fg, FS, mv, c->mig, cap, need, smask, lo, hi, scaleR, scaleJ, count ? c->finc : nullptr, c->mbkt);
    RH_LAUNCHED(c);
-   k_int_to64<<<blocks1d(nb + 1, 256), 256, 0, c->stream>>>(c->finc, nb, c->ftmpInc64);
+   return RHGPU_OK;
+}
+
+template <class MV, class SET>
+int migPlace(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS, int force) {
+   const int NS = (int)c->fg.NS;
+   k_mig_place<<<moverBlocks(c, 256), 256, 0, c->stream>>>(FS, mv, c->mig, cap, force, NS, c->finc, c->foffInc, c->mkey,
+                                                           c->mval);
    RH_LAUNCHED(c);
-   if (int rc_ = scanExclusive64(c, c->ftmpInc64, c->foffInc, nb + 1)) return rc_;
-   unsigned long long *kA = c->mkey, *kB = c->mkey + c->mcap;
-   unsigned *vA = c->mval, *vB = c->mval + c->mcap, *bA = c->mbkt, *bB = c->mbkt + c->mcap;
-   RH_CUDA(cudaMemsetAsync(c->fmaxInc, 0, sizeof(int), c->stream));
-   k_max_int<<<(unsigned)std::min<long long>(blocks1d(nb, 256), 4 * 148), 256, 0, c->stream>>>(c->finc, nb, c->fmaxInc);
+   k_mig_counts<<<blocks1d((long long)c->ns * NS, 256), 256, 0, c->stream>>>(FS, c->mig, cap, force, NS, c->finc);
    RH_LAUNCHED(c);
-   int rc = RHGPU_OK;
-   int maxInc = 0;
-   RH_CUDA(cudaMemcpyAsync(&maxInc, c->fmaxInc, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-   RH_CUDA(cudaStreamSynchronize(c->stream));
-   if (maxInc <= MIG_LARGE) {
-      // buckets past the placed movers stay at nb (not placed)
-      RH_CUDA(cudaMemsetAsync(c->ffill, 0, sizeof(int) * nb, c->stream));
-      k_fill_u32<<<blocks1d(nm, 256), 256, 0, c->stream>>>(bA, nm, (unsigned)nb);
-      k_mig_bucket<<<blocks1d(nm, 256), 256, 0, c->stream>>>(mv, nm, NS, c->foffInc, c->ffill, vA);
+   return RHGPU_OK;
+}
+
+// the placement of the counted movers as far as the device can take it, and its
+// state on the way to the host
+template <class MV, class SET>
+int migLaunch(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS) {
+   const int NS = (int)c->fg.NS;
+   k_mig_buckets<<<blocks1d((long long)c->ns * NS, 256), 256, 0, c->stream>>>(FS, NS, c->finc, c->foffInc, c->mig);
+   RH_LAUNCHED(c);
+   k_mig_list<<<moverBlocks(c, 256), 256, 0, c->stream>>>(mv, c->mig, cap, 0, NS, c->foffInc, c->mbkt, c->mkey, c->mval);
+   RH_LAUNCHED(c);
+   if (const int rc = migPlace(c, mv, cap, FS, 0)) return rc;
+   RH_CUDA(cudaMemcpyAsync(c->migHost, c->mig, sizeof(MigCtl), cudaMemcpyDeviceToHost, c->stream));
+   RH_CUDA(cudaEventRecord(c->migEvent, c->stream));
+   c->migPending = true;
+   return RHGPU_OK;
+}
+
+FastSpecies setOf(rhgpu_ctx* c, const Mover*) { return fastSpecies(c); }
+F32Set setOf(rhgpu_ctx* c, const Mover32*) { return f32Set(c); }
+int relayoutNext(rhgpu_ctx* c, unsigned mask, const Mover*);
+int relayoutNext(rhgpu_ctx* c, unsigned mask, const Mover32*) { return f32RelayoutNext(c, mask); }
+
+// placement that the device left to the host: segments without room relaid out,
+// buckets above MIG_RANK arrivals ordered by a block each, or, past MIG_LARGE,
+// all movers by two stable radix sorts (by key, then by bucket)
+template <class MV>
+int migResolve(rhgpu_ctx* c, const MV* mv, long long cap) {
+   const int NS = (int)c->fg.NS;
+   const long long nb = (long long)c->ns * NS, nm = (long long)c->migHost->nm;
+   if (c->migHost->over) {
+      if (const int rc = relayoutNext(c, c->migHost->over, mv)) return rc;
+      RH_CUDA(cudaMemsetAsync(&c->mig->over, 0, sizeof(unsigned), c->stream));
+      k_mig_check<<<blocks1d(nb, 256), 256, 0, c->stream>>>(setOf(c, mv), NS, c->finc, c->mig);
       RH_LAUNCHED(c);
-      k_mig_order_small<<<blocks1d(nb, 256), 256, 0, c->stream>>>(mv, nb, c->finc, c->foffInc, vA, bA);
+      unsigned over = 0;
+      RH_CUDA(cudaMemcpyAsync(&over, &c->mig->over, sizeof over, cudaMemcpyDeviceToHost, c->stream));
+      RH_CUDA(cudaStreamSynchronize(c->stream));
+      if (over) return fail(RHGPU_ERR_CAPACITY, "segment relayout did not make room");
+   }
+   const auto FS = setOf(c, mv);
+   if (c->migHost->maxInc <= MIG_LARGE) {
+      k_mig_list<<<moverBlocks(c, 256), 256, 0, c->stream>>>(mv, c->mig, cap, 1, NS, c->foffInc, c->mbkt, c->mkey, c->mval);
       RH_LAUNCHED(c);
-      if (maxInc > MIG_SMALL) {
-         // the large buckets (each holds more than MIG_SMALL movers, so fewer
-         // than nm / MIG_SMALL of them) listed in bB, their count in fmaxInc
+      if (c->migHost->maxInc > MIG_RANK) {
+         // each large bucket holds more than MIG_RANK movers, so fewer than nm / MIG_RANK of them
+         unsigned* const large = c->mval + c->mcap;
          RH_CUDA(cudaMemsetAsync(c->fmaxInc, 0, sizeof(int), c->stream));
-         k_mig_large_list<<<blocks1d(nb, 256), 256, 0, c->stream>>>(c->finc, nb, bB, c->fmaxInc);
+         k_mig_large_list<<<blocks1d(nb, 256), 256, 0, c->stream>>>(c->finc, nb, large, c->fmaxInc);
          RH_LAUNCHED(c);
-         const unsigned grid = (unsigned)std::min<long long>(nm / MIG_SMALL + 1, 4 * 148);
-         k_mig_order_large<<<grid, MIG_LARGE_THREADS, 0, c->stream>>>(mv, c->finc, c->foffInc, vA, bA, bB, c->fmaxInc);
+         const unsigned grid = (unsigned)std::min<long long>(nm / MIG_RANK + 1, 4 * 148);
+         k_mig_order_large<<<grid, MIG_LARGE_THREADS, 0, c->stream>>>(c->finc, c->foffInc, c->mkey, c->mval, large, c->fmaxInc);
          RH_LAUNCHED(c);
       }
-      k_mig_check<<<blocks1d(nb, 256), 256, 0, c->stream>>>(FS, NS, c->finc, c->fover);
-      RH_LAUNCHED(c);
-      RH_CUDA(cudaMemcpyAsync(over, c->fover, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-      RH_CUDA(cudaStreamSynchronize(c->stream));
-      *order = vA;
-      *bucket = bA;
-      return RHGPU_OK;
+      return migPlace(c, mv, cap, FS, 1);
    }
-   RH_TIME(c, "mig_radix_order");   // the fallback: a bucket with more than MIG_SMALL arrivals
+   RH_TIME(c, "mig_radix_order");
+   k_int_to64<<<blocks1d(nb + 1, 256), 256, 0, c->stream>>>(c->finc, nb, c->ftmpInc64);
+   RH_LAUNCHED(c);
+   if (int rc = scanExclusive64(c, c->ftmpInc64, c->foffInc, nb + 1)) return rc;
+   unsigned long long *kA = c->mkey, *kB = c->mkey + c->mcap;
+   unsigned *vA = c->mval, *vB = c->mval + c->mcap, *bA = c->mbkt, *bB = c->mbkt + c->mcap;
    k_mig_sort_keys<<<blocks1d(nm, 256), 256, 0, c->stream>>>(mv, nm, NS, nb, kA, vA, bA);
    RH_LAUNCHED(c);
-   const int kbits = 32 + bitsFor(std::max(NS > 1 ? NS - 1 : 1, c->injKeyMax)), bbits = bitsFor(nb);
+   const int kbits = 32 + bitsFor(std::max<long long>(NS > 1 ? NS - 1 : 1, c->injKeyMax)), bbits = bitsFor(nb);
    size_t s1 = 0, s2 = 0;
    cub::DeviceRadixSort::SortPairs(nullptr, s1, kA, kB, vA, vB, (int)nm, 0, kbits, c->stream);
    cub::DeviceRadixSort::SortPairs(nullptr, s2, bB, bA, vB, vA, (int)nm, 0, bbits, c->stream);
-   rc = ensureSortTmp(c, std::max(s1, s2));
-   if (rc) return rc;
+   if (int rc = ensureSortTmp(c, std::max(s1, s2))) return rc;
    size_t sb = c->sortTmpBytes;
    RH_CUDA(cub::DeviceRadixSort::SortPairs(c->sortTmp, sb, kA, kB, vA, vB, (int)nm, 0, kbits, c->stream));
    k_gather_u32<<<blocks1d(nm, 256), 256, 0, c->stream>>>(bA, vB, nm, bB);
    RH_LAUNCHED(c);
    sb = c->sortTmpBytes;
    RH_CUDA(cub::DeviceRadixSort::SortPairs(c->sortTmp, sb, bB, bA, vB, vA, (int)nm, 0, bbits, c->stream));
-   k_mig_check<<<blocks1d(nb, 256), 256, 0, c->stream>>>(FS, NS, c->finc, c->fover);
+   k_mig_place_order<<<blocks1d(nm, 256), 256, 0, c->stream>>>(FS, NS, nb, mv, vA, bA, c->foffInc, nm);
    RH_LAUNCHED(c);
-   RH_CUDA(cudaMemcpyAsync(over, c->fover, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-   RH_CUDA(cudaStreamSynchronize(c->stream));
-   *order = vA;
-   *bucket = bA;
+   k_mig_counts<<<blocks1d(nb, 256), 256, 0, c->stream>>>(FS, c->mig, cap, 1, NS, c->finc);
+   RH_LAUNCHED(c);
+   return RHGPU_OK;
+}
+
+// the pending push's movers placed; its "next" buffers become the current ones
+int migFinish(rhgpu_ctx* c) {
+   if (!c->migPending) return RHGPU_OK;
+   RH_CUDA(cudaEventSynchronize(c->migEvent));
+   c->migPending = false;
+   const bool f32 = c->path == RHGPU_PATH_FP32;
+   const long long cap = f32 ? c->f32b.moverCap : c->fb.moverCap, nm = (long long)c->migHost->nm;
+   if (nm > cap) return fail(RHGPU_ERR_CAPACITY, "mover list overflow");
+   c->migLast = nm;
+   if (c->migHost->over || c->migHost->maxInc > MIG_RANK) {
+      const int rc = f32 ? migResolve(c, c->f32b.movers, cap) : migResolve(c, c->fb.movers, cap);
+      if (rc) return rc;
+   }
+   c->migDirty = false;
+   for (int s = 0; s < c->ns; ++s) {
+      if (f32) c->f32[s].cur ^= 1;
+      else c->seg[s].cur ^= 1;
+   }
    return RHGPU_OK;
 }
 
@@ -274,6 +336,8 @@ int fastRelayoutNext(rhgpu_ctx* c, unsigned mask) {
    RH_CUDA(cudaStreamSynchronize(c->stream));
    return RHGPU_OK;
 }
+
+int relayoutNext(rhgpu_ctx* c, unsigned mask, const Mover*) { return fastRelayoutNext(c, mask); }
 
 int fastUpload(rhgpu_ctx* c, int s, const uint32_t* counts, const double* particles, long long n) {
    const long long N = c->g.N, NS = c->fg.NS;
@@ -417,7 +481,7 @@ int injectAll(rhgpu_ctx* c, MV* movers, long long moverCap) {
 // its averages: the stayers (the next buffer before the arrivals are placed)
 // by segment, then every deposited mover (left its segment, or deposited in it
 // and removed by a boundary)
-int fastAverages(rhgpu_ctx* c, long long nm) {
+int fastAverages(rhgpu_ctx* c) {
    const long long N = c->g.N;
    FastBufs& A = c->avgFB;
    if (!A.RP) {
@@ -452,13 +516,13 @@ int fastAverages(rhgpu_ctx* c, long long nm) {
 #undef RH_FAST_AVG
       }
       RH_LAUNCHED(c);
-      if (nm > 0) {
-         k_fast_avg_movers<<<blocks1d(nm, 128), 128, 0, c->stream>>>(c->g, c->fg, FS, c->fb.movers, nm, mask, A);
-         RH_LAUNCHED(c);
-      }
-      k_fast_avg_gather<<<cellGrid(c->g), cellBlock(), 0, c->stream>>>(c->g, c->fg, A, hiR, loR, hiJ, loJ,
+      if (const int rc = moverPass(c, c->fb.movers, c->fb.moverCap, FS, MOVER_DEPOSIT | MOVER_AVG, mask, A.MMlo, A.MMhi,
+                                   A.scaleR, A.scaleJ, false))
+         return rc;
+      k_fast_avg_gather<<<gatherGrid(c->g), 2 * GA_CELLS, 0, c->stream>>>(c->g, c->fg, A, hiR, loR, hiJ, loJ,
                                                                       c->avgN + (long long)grp * N, c->avgV + 3LL * grp * N);
       RH_LAUNCHED(c);
+      if (const int rc = fixedClear(c, A.MMlo, A.MMhi)) return rc;
    }
    return RHGPU_OK;
 }
@@ -482,6 +546,7 @@ int launchPushDeposit(rhgpu_ctx* c, const FastSpecies& FS, const PushParams& pp)
 }
 
 int fastPush(rhgpu_ctx* c) {
+   if (const int rc = migFinish(c)) return rc;
    // a relayout of the last step may have grown the particle storage
    if (const int rc = fastMoverBuffers(c)) return rc;
    c->timestep += 1;
@@ -493,9 +558,7 @@ int fastPush(rhgpu_ctx* c) {
    pp.GMdt = c->P.GMdt;
    pp.maxVi2 = c->P.max_ion_speed2;
    pp.avgList = c->avgGroups > 0;
-   const long long N = c->g.N, NS = c->fg.NS;
-   RH_CUDA(cudaMemsetAsync(c->fb.touched, 0, (size_t)N + 16, c->stream));
-   RH_CUDA(cudaMemsetAsync(c->fb.nmovers, 0, sizeof(unsigned long long), c->stream));
+   if (const int rc = migBegin(c)) return rc;
    {
       RH_TIME(c, "fast_push_deposit");
       const FastSpecies FS = fastSpecies(c);
@@ -518,68 +581,45 @@ int fastPush(rhgpu_ctx* c) {
       const int rc = injectAll(c, c->fb.movers, c->fb.moverCap);
       if (rc) return rc;
    }
-   unsigned long long nm = 0;
-   RH_CUDA(cudaMemcpyAsync(&nm, c->fb.nmovers, sizeof nm, cudaMemcpyDeviceToHost, c->stream));
-   RH_CUDA(cudaStreamSynchronize(c->stream));
-   if ((long long)nm > c->fb.moverCap) return fail(RHGPU_ERR_CAPACITY, "mover list overflow");
-   if (nm > 0) {
+   {
       RH_TIME(c, "fast_mover_deposit");
-      k_fast_mover_deposit<<<blocks1d(nm, 128), 128, 0, c->stream>>>(c->g, c->fg, fastSpecies(c), c->fb, nm);
-      RH_LAUNCHED(c);
-   }
-   if (c->avgGroups) {
-      const int rc = fastAverages(c, (long long)nm);
+      const int rc = moverPass(c, c->fb.movers, c->fb.moverCap, fastSpecies(c), MOVER_DEPOSIT, ~0u, c->fb.MMlo, c->fb.MMhi,
+                               c->fb.scaleR, c->fb.scaleJ, true);
       if (rc) return rc;
    }
-   if (nm > 0) {
-      const long long nb = (long long)c->ns * NS;
-      int over = 0;
-      {
-         RH_TIME(c, "fast_migrate");
-         unsigned *order = nullptr, *bkt = nullptr;
-         int rc = migSort(c, c->fb.movers, (long long)nm, fastSpecies(c), &order, &bkt, &over);
-         if (rc) return rc;
-         if (over) {
-            // some segments lack room for their arrivals: relayout with room for them
-            rc = fastRelayoutNext(c, (unsigned)over);
-            if (rc) return rc;
-            RH_CUDA(cudaMemsetAsync(c->fover, 0, sizeof(int), c->stream));
-            k_mig_check<<<blocks1d(nb, 256), 256, 0, c->stream>>>(fastSpecies(c), NS, c->finc, c->fover);
-            RH_LAUNCHED(c);
-            RH_CUDA(cudaMemcpyAsync(&over, c->fover, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            RH_CUDA(cudaStreamSynchronize(c->stream));
-            if (over) return fail(RHGPU_ERR_CAPACITY, "segment relayout did not make room");
-         }
-         k_fast_mig_place<<<blocks1d(nm, 256), 256, 0, c->stream>>>(fastSpecies(c), NS, nb, c->fb.movers, order, bkt, c->foffInc,
-                                                                 (long long)nm);
-         RH_LAUNCHED(c);
-         k_mig_counts<<<blocks1d(nb, 256), 256, 0, c->stream>>>(fastSpecies(c), NS, c->finc);
-         RH_LAUNCHED(c);
-      }
+   if (c->avgGroups) {
+      const int rc = fastAverages(c);
+      if (rc) return rc;
    }
-   for (int s = 0; s < c->ns; ++s) c->seg[s].cur ^= 1;
+   RH_TIME(c, "fast_migrate");
+   return migLaunch(c, c->fb.movers, c->fb.moverCap, fastSpecies(c));
+}
+
+// the movers' fixed-point sums cleared for the next step
+int fixedClear(rhgpu_ctx* c, unsigned long long* lo, unsigned long long* hi) {
+   const size_t bytes = sizeof(unsigned long long) * 4 * (size_t)c->g.N;
+   RH_CUDA(cudaMemsetAsync(lo, 0, bytes, c->stream));
+   RH_CUDA(cudaMemsetAsync(hi, 0, bytes, c->stream));
    return RHGPU_OK;
 }
 
 int fastGather(rhgpu_ctx* c) {
    RH_TIME(c, "fast_gather");
-   k_fast_fold_boundary<<<blocks1d(16 * c->fg.nrows * c->fg.nseg, 256), 256, 0, c->stream>>>(c->g, c->fg, c->fb);
-   RH_LAUNCHED(c);
    const double hiR = std::ldexp(1.0, 64 - c->kR), loR = std::ldexp(1.0, -c->kR);
    const double hiJ = std::ldexp(1.0, 64 - c->kJ), loJ = std::ldexp(1.0, -c->kJ);
    if (c->f.gc)
-      k_fast_gather<true><<<cellGrid(c->g), cellBlock(), 0, c->stream>>>(c->g, c->f, c->fg, c->fb, hiR, loR, hiJ, loJ,
+      k_fast_gather<true><<<gatherGrid(c->g), 2 * GA_CELLS, 0, c->stream>>>(c->g, c->f, c->fg, c->fb, hiR, loR, hiJ, loJ,
                                                                         c->P.min_ion_charge_density, c->cntU);
    else
-      k_fast_gather<false><<<cellGrid(c->g), cellBlock(), 0, c->stream>>>(c->g, c->f, c->fg, c->fb, hiR, loR, hiJ, loJ,
+      k_fast_gather<false><<<gatherGrid(c->g), 2 * GA_CELLS, 0, c->stream>>>(c->g, c->f, c->fg, c->fb, hiR, loR, hiJ, loJ,
                                                                          c->P.min_ion_charge_density, c->cntU);
    RH_LAUNCHED(c);
-   return RHGPU_OK;
+   return fixedClear(c, c->fb.MMlo, c->fb.MMhi);
 }
 
-template int migSort<Mover, FastSpecies>(rhgpu_ctx*, const Mover*, long long, const FastSpecies&, unsigned**, unsigned**,
-                                         int*);
-template int migSort<Mover32, F32Set>(rhgpu_ctx*, const Mover32*, long long, const F32Set&, unsigned**, unsigned**, int*);
+template int moverPass<Mover32, F32Set>(rhgpu_ctx*, const Mover32*, long long, const F32Set&, int, unsigned,
+                                        unsigned long long*, unsigned long long*, double, double, bool);
+template int migLaunch<Mover32, F32Set>(rhgpu_ctx*, const Mover32*, long long, const F32Set&);
 template int injectAll<Mover>(rhgpu_ctx*, Mover*, long long);
 template int injectAll<Mover32>(rhgpu_ctx*, Mover32*, long long);
 

@@ -153,9 +153,14 @@ struct rhgpu_ctx {
    unsigned* mval = nullptr;            // 2 x mcap mover indices
    unsigned* mbkt = nullptr;            // 2 x mcap destination buckets
    long long mcap = 0;
-   int* ffill = nullptr;                // ns*NS fill counters of the small-bucket placement
-   int* fmaxInc = nullptr;              // largest arrivals of a bucket
+   int* fmaxInc = nullptr;              // count of the buckets above MIG_RANK arrivals
    int* fover = nullptr;                // 16 bytes
+   MigCtl* mig = nullptr;               // the step's migration state (fb.nmovers is its nm)
+   MigCtl* migHost = nullptr;           // pinned copy, valid after migEvent
+   cudaEvent_t migEvent = nullptr;
+   bool migPending = false;             // a push's movers wait for migFinish
+   bool migDirty = false;               // finc may hold counts of a step that did not finish
+   long long migLast = -1;              // movers of the last step (-1: none yet): the next one's launch sizes
    int kR = 0, kJ = 0;
    void* sortTmp = nullptr;
    size_t sortTmpBytes = 0;
@@ -312,6 +317,7 @@ int fastNumParticles(rhgpu_ctx* c, int s, long long* n);
 int fastDownload(rhgpu_ctx* c, int s, uint32_t* counts, double* particles, long long capacity, long long* n_out);
 int fastPush(rhgpu_ctx* c);
 int fastGather(rhgpu_ctx* c);
+int fixedClear(rhgpu_ctx* c, unsigned long long* lo, unsigned long long* hi);
 
 // ---- FP32 form (rhgpu_f32.cu)
 F32Buf f32View(const F32Host& h, int which);
@@ -331,11 +337,22 @@ int f32Gather(rhgpu_ctx* c);
 int dnApplyCtx(rhgpu_ctx* c);
 void freeInjector(InjHost& h);
 
-// the movers' placement order (rhgpu_fast.cu; instantiated for the fast path's
-// and the FP32 form's movers) and the particle sources of a step appended to
-// a mover list
+// the movers' deposit and placement (rhgpu_fast.cu; instantiated for the fast
+// path's and the FP32 form's movers) and the particle sources of a step
+// appended to a mover list. migBegin clears the step's migration state,
+// moverPass and migLaunch put the whole step on the stream, migFinish waits for
+// migLaunch's state and does what the device could not.
+int migBegin(rhgpu_ctx* c);
 template <class MV, class SET>
-int migSort(rhgpu_ctx* c, const MV* mv, long long nm, const SET& FS, unsigned** order, unsigned** bucket, int* over);
+int moverPass(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS, int need, unsigned smask, unsigned long long* lo,
+              unsigned long long* hi, double scaleR, double scaleJ, bool count);
+template <class MV, class SET>
+int migLaunch(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS);
+template <class MV>
+int migResolve(rhgpu_ctx* c, const MV* mv, long long cap);
+int migFinish(rhgpu_ctx* c);
+F32Set f32Set(rhgpu_ctx* c);
+int f32RelayoutNext(rhgpu_ctx* c, unsigned mask);
 template <class MV>
 int injectAll(rhgpu_ctx* c, MV* movers, long long moverCap);
 
