@@ -131,7 +131,10 @@ k_fast_avg_deposit(GridInfo gIn, FastGeom fg, FastSpecies FS, unsigned mask, Fas
       // the next chunk's first barrier orders these reads before its record writes
    }
    __syncthreads();
-   segPartialsOut(g, fg, fb, s_rec, row, gseg, u0, u1, a0, a1, a2, a3);
+   double* const q = s_rec + myDual * 32 + myCorner * 4;
+   q[0] = a0; q[1] = a1; q[2] = a2; q[3] = a3;
+   __syncthreads();
+   segPartialsOut<FT>(g, fg, fb.RP, fb.RPB, s_rec, row, gseg, u0, u1);
 }
 
 // fast path: row partials + fixed-point part added to the population's sums;

@@ -86,24 +86,34 @@ __device__ inline int halfSf(float o) { return o < 0.5f ? 0 : 1; }
 using SegFields32 = SegFieldsT<float>;
 
 // Boris-Buneman push in FP32 (boris.h:64-194 in cell units); o: offsets, v: velocity
-__device__ inline bool pushF32(const GridInfo& g, const SegFields32& F, const F32Set& FS, int s, const F32Params& pp,
-                               int i, int j, int k, int lc, int ly, int lz, float o[3], float v[3]) {
+__device__ __forceinline__ bool pushF32(const GridInfo& g, const SegFields32& F, float qm, bool accelerate,
+                                        const F32Params& pp, int i, int j, int k, int lc, int ly, int lz, float o[3],
+                                        float v[3]) {
    bool clamp = false;
-   const bool accelerate = FS.accelerate[s] && !pp.useIFT && allNb(g, i, j, k);
    float vx = v[0], vy = v[1], vz = v[2];
    if (accelerate) {
       float B[3], Ue[3], E[3];
       const float xs = o[0], ys = o[1], zs = o[2];
+      constexpr int SX = SEG + 2;
+      const int at = (2 * lz + ly) * SX + lc;      // bx, bz, ue, ep
+      const float* const bx = &F.bx[0][0][0] + at;
+      const float* const by = &F.by[0][0][0] + at + lz * SX;
+      const float* const bz = &F.bz[0][0][0] + at;
+      const float* const ue = &F.ue[0][0][0][0] + at;
       // (fused multiply-adds: the FP32 form is not held to the FP64 operation order)
-      B[0] = fmaf(xs, F.bx[lz][ly][lc + 1], (1.0f - xs) * F.bx[lz][ly][lc]);
-      B[1] = fmaf(ys, F.by[lz][ly + 1][lc], (1.0f - ys) * F.by[lz][ly][lc]);
-      B[2] = fmaf(zs, F.bz[lz + 1][ly][lc], (1.0f - zs) * F.bz[lz][ly][lc]);
-      for (int l = 0; l < 3; ++l) Ue[l] = F.ue[l][lz][ly][lc];
+      B[0] = fmaf(xs, bx[1], (1.0f - xs) * bx[0]);
+      B[1] = fmaf(ys, by[SX], (1.0f - ys) * by[0]);
+      B[2] = fmaf(zs, bz[2 * SX], (1.0f - zs) * bz[0]);
+#pragma unroll
+      for (int l = 0; l < 3; ++l) Ue[l] = ue[4 * SX * l];
       E[0] = fmaf(B[1], Ue[2], -(B[2] * Ue[1]));
       E[1] = fmaf(B[2], Ue[0], -(B[0] * Ue[2]));
       E[2] = fmaf(B[0], Ue[1], -(B[1] * Ue[0]));
-      if (pp.use_ep) for (int l = 0; l < 3; ++l) E[l] += F.ep[l][lz][ly][lc];
-      const float qm = FS.qm[s];
+      if (pp.use_ep) {
+         const float* const ep = &F.ep[0][0][0][0] + at;
+#pragma unroll
+         for (int l = 0; l < 3; ++l) E[l] += ep[4 * SX * l];
+      }
       const float dvx = qm * E[0], dvy = qm * E[1], dvz = qm * E[2];
       const float tx = qm * B[0], ty = qm * B[1], tz = qm * B[2];
       const float t2 = fmaf(tx, tx, fmaf(ty, ty, tz * tz));
@@ -174,30 +184,33 @@ __device__ inline void cicWeightsF(const float o[3], float wq, float w8[8]) {
    w8[7] = wx * wy * wz * wq;
 }
 
-constexpr int REC32 = 11;   // floats per deposit record: w8[8], v[3]
+constexpr int REC32 = 12;   // floats per deposit record: w8[8], then 1, v[3] (48 bytes apart: any eight on different banks)
 
+// resident blocks per SM: the kernel waits on its barriers and shared-memory
+// round trips, so warps count for more than the few registers that 36 a thread
+// spill (Mars run, 9.25e7 ions: 4 blocks 3.63 ms, 5 3.31, 6 3.09, 7 and 8 3.05)
+constexpr int F32_BLOCKS = 7;
 // shared memory of k_f32_push_deposit
 constexpr int F32_PTRS = 14;   // one species' arrays offset to the segment: current cell, o, v (0-6), next (7-13)
 struct F32PushShared {
-   float rec[FT * REC32];                   // deposit records of a chunk; at the end acc[SEG][32]
-   float pf[7][FT];                         // the next chunk's particles: cell (int bits), o[3], v[3]
+   alignas(16) float rec[PD_T * REC32];     // deposit records of a chunk; at the end acc[SEG][32]
+   float pf[7][PD_T];                       // the next chunk's particles: cell (int bits), o[3], v[3]
    SegFields32 f;                           // field stencil of the segment
    void* ptr[FAST_MAX_SPECIES][F32_PTRS];
    StencilRow rows[SF_MAX_ROWS];
-   alignas(8) unsigned char wd[SEG][FW];    // records per (dual cell, warp)
-   int rank[FT];                            // stayers of the chunk before each chunk position
-   int wcnt[FW];                            // stayers per warp
-   int prefix[FAST_MAX_SPECIES + 1];        // first particle of each species in the segment
-   int stay[FAST_MAX_SPECIES];              // stayers of each species so far
+   alignas(8) unsigned char wd[SEG][PD_VW];   // records per (dual cell, group)
+   int wcnt[PD_VW];                         // stayers per group
+   int first[FAST_MAX_SPECIES + 1];         // first group of each species in the segment
+   int cnt[FAST_MAX_SPECIES];               // particles of each species in the segment
+   int stay[FAST_MAX_SPECIES];              // stayers of each species up to and with the chunk
 };
 
-// chunk position tid of the chunk starting at c0 requested into pf (cp.async)
-__device__ __forceinline__ void f32Prefetch(F32PushShared& sh, int i, int total, int ns, int s0) {
-   const int tid = threadIdx.x;
-   if (i < total) {
-      int s = s0;
-      while (s + 1 < ns && i >= sh.prefix[s + 1]) ++s;
-      const int p = i - sh.prefix[s];
+// this thread's particle of the chunk that starts at group V0 requested into pf (cp.async)
+__device__ __forceinline__ void f32Prefetch(F32PushShared& sh, int V0, int ns) {
+   const int tid = threadIdx.x, V = V0 + (tid >> 5);
+   const int s = pdSpecies(sh, V, ns);
+   const int p = (V - sh.first[s]) * 32 + (tid & 31);
+   if (p < sh.cnt[s]) {
 #pragma unroll
       for (int a = 0; a < 7; ++a) cpAsync4(&sh.pf[a][tid], (const float*)sh.ptr[s][a] + p);
    }
@@ -208,14 +221,14 @@ __device__ __forceinline__ void f32Prefetch(F32PushShared& sh, int i, int total,
 // launches the instantiation that matches the grid
 // GC: the variant that also counts the per-cell maxVi constraint (grid counters on)
 //
-// One block per segment, one thread per particle, chunks of FT particles in
-// storage order (species after species), as k_fast_push_deposit: the next
-// chunk's particles are copied to shared memory (cp.async) while the current
-// one is processed, two barriers per chunk, per-warp record counts packed in
-// bytes, a leaving particle's mover slot reserved before the second barrier
-// and written after the deposit sums.
+// One block per segment, as k_fast_push_deposit: chunks of PD_T particles,
+// every species starting at a group of 32, one particle per thread, the next
+// chunk copied to shared memory (cp.async) while the current one is processed,
+// two barriers per chunk, per-group record counts packed in bytes, a leaving
+// particle's mover slot reserved before the second barrier and written after
+// the deposit sums.
 template <int PER, bool GC>
-__global__ void __launch_bounds__(FT, 4)
+__global__ void __launch_bounds__(PD_T, F32_BLOCKS)
 k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp, F32Bufs fb, double* cntd,
                    unsigned long long* cntu, unsigned* err) {
    GridInfo g = gIn;
@@ -225,26 +238,31 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
    __shared__ F32PushShared sh;
    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
    const unsigned below = (1u << lane) - 1u;
-   const long long S = blockIdx.x;
-   const long long row = S / fg.nseg;
-   const int gseg = (int)(S % fg.nseg);
-   const int uy = (int)(row % fg.nd[1]), uz = (int)(row / fg.nd[1]);
-   const int ndx = fg.nd[0];
-   const int u0 = gseg * SEG, u1 = min(u0 + SEG, ndx);
+   const int S = (int)blockIdx.x;
+   const int nseg = fg.nseg;
+   const int row = S / nseg, gseg = S - row * nseg;
+   const int uz = row / fg.nd[1], uy = row - uz * fg.nd[1];
+   const int u0 = gseg * SEG, u1 = min(u0 + SEG, fg.nd[0]);
    const int ns = FS.ns;
-   // set-up: species prefix (warp 0), segment pointers (warps 1-4)
+   const int xs0 = dualB(u0, g.per[0]), ys0 = dualB(uy, g.per[1]), zs0 = dualB(uz, g.per[2]);
+   const bool segInner = fb.segInner[S] != 0;   // an obstacle cell within one step of the segment
+   // every cell a particle of the segment can be in or reach has its neighbours in y and z
+   const bool yzIn = ((PER & 2) || (ys0 >= 2 && ys0 + 2 <= g.ny - 2)) && ((PER & 4) || (zs0 >= 2 && zs0 + 2 <= g.nz - 2));
+   // set-up: species (warp 0), segment pointers
    if (warp == 0) {
       const int cnt = lane < ns ? FS.st[lane].cur.cnt[S] : 0;
-      int x = cnt;
+      const int groups = (cnt + 31) >> 5;
+      int x = groups;
 #pragma unroll
       for (int o = 1; o < 16; o <<= 1) {
          const int y = __shfl_up_sync(0xffffffffu, x, o);
          if (lane >= o) x += y;
       }
-      if (lane <= ns) sh.prefix[lane] = x - cnt;
-      if (lane < FAST_MAX_SPECIES) sh.stay[lane] = 0;
-   } else if (tid < 32 + F32_PTRS * ns) {
-      const int q = tid - 32, s = q / F32_PTRS, k = q - s * F32_PTRS;
+      if (lane <= ns) sh.first[lane] = x - groups;
+      if (lane < FAST_MAX_SPECIES) { sh.cnt[lane] = cnt; sh.stay[lane] = 0; }
+   }
+   for (int q = tid; q < F32_PTRS * ns; q += PD_T) {
+      const int s = q / F32_PTRS, k = q - s * F32_PTRS;
       const F32Species& SS = FS.st[s];
       const long long b = SS.base[S];
       const F32Buf& B = k < 7 ? SS.cur : SS.nxt;
@@ -255,222 +273,205 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
       else v = B.v[kk - 4] + b;
       sh.ptr[s][k] = v;
    }
-   const int by0 = dualB(uy, g.per[1]), bz0 = dualB(uz, g.per[2]);
-   const bool segInner = fb.segInner[S] != 0;   // an obstacle cell within one step of the segment
-   // (stageSegRows' own barrier publishes the prefix and the pointers)
-   stageSegRows(g, f, pp.use_ep, dualB(u0, g.per[0]), by0, bz0, sh.f, sh.rows);
+   // (stageSegRows' own barrier publishes the species and the pointers)
+   stageSegRows<PD_T>(g, f, pp.use_ep, xs0, ys0, zs0, sh.f, sh.rows);
    __syncthreads();
-   const int total = sh.prefix[ns];
-   f32Prefetch(sh, tid, total, ns, 0);
-   const int myDual = tid >> 3, myCorner = tid & 7;
-   float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+   const int groups = sh.first[ns];
+   f32Prefetch(sh, 0, ns);
+   const int myDual = tid >> 3, myPair = (tid >> 1) & 3, myHalf = tid & 1;
+   float a00 = 0.0f, a01 = 0.0f, a10 = 0.0f, a11 = 0.0f;
 
-   for (int c0 = 0; c0 < total; c0 += FT) {
-      const int i = c0 + tid;
-      const bool active = i < total;
-      int s = 0;
-      if (active)
-         while (s + 1 < ns && i >= sh.prefix[s + 1]) ++s;
+   for (int V0 = 0; V0 < groups; V0 += PD_VW) {
       float o[3], v[3];
-      int cell = 0, p = 0;
-      bool stay = false, rec = false, leave = false, clamp = false;
-      int mflags = 0, vx = 0, vy = 0, vz = 0, ti = 0, tj = 0, tk = 0;
+      int cell = 0, duv = 0, dyz = 0, mflags = 0, rrank = 0;
+      bool stay = false, rec = false, clamp = false;
       cpAsyncWaitAll();   // this thread's copies of the chunk
-      if (active) {
-         p = i - sh.prefix[s];
-         cell = __float_as_int(sh.pf[0][tid]);
+      const int V = V0 + warp;
+      const int s = pdSpecies(sh, V, ns);
+      const int p = (V - sh.first[s]) * 32 + lane;
+      if (p < sh.cnt[s]) {
+         const int c = __float_as_int(sh.pf[0][tid]);
+#pragma unroll
          for (int a = 0; a < 3; ++a) { o[a] = sh.pf[1 + a][tid]; v[a] = sh.pf[4 + a][tid]; }
-         const int sx = halfSf(o[0]), sy = halfSf(o[1]), sz = halfSf(o[2]);
-         int cj = by0 + 1 - sy, ck = bz0 + 1 - sz;
-         if (cj >= g.ny) cj -= g.ny;
-         if (ck >= g.nz) ck -= g.nz;
-         const int ci = cell - g.nx * (cj + g.ny * ck);
-         const int lu = dualU(ci + sx - 1, g.nx, g.per[0]) - u0;
-         const int lc = lu + 1 - sx, ly = 1 - sy, lz = 1 - sz;
-         clamp = pushF32(g, sh.f, FS, s, pp, ci, cj, ck, lc, ly, lz, o, v);
+         const int gx = halfSf(o[0]), gy = halfSf(o[1]), gz = halfSf(o[2]);
+         const int ly = 1 - gy, lz = 1 - gz;
+         const int cj = ys0 + ly, ck = zs0 + lz;   // not wrapped (periodic axes: up to n)
+         const int wj = (PER & 2) && cj >= g.ny ? cj - g.ny : cj, wk = (PER & 4) && ck >= g.nz ? ck - g.nz : ck;
+         const int wi = c - g.nx * (wj + g.ny * wk);
+         const int lu = dualU(wi + gx - 1, g.nx, g.per[0]) - u0;
+         const int lc = lu + 1 - gx, ci = xs0 + lc;
+         bool accelerate = FS.accelerate[s] && !pp.useIFT && ((PER & 1) || (unsigned)(ci - 1) < (unsigned)(g.nx - 2));
+         if (!yzIn)
+            accelerate = accelerate && ((PER & 2) || (unsigned)(cj - 1) < (unsigned)(g.ny - 2)) &&
+                         ((PER & 4) || (unsigned)(ck - 1) < (unsigned)(g.nz - 2));
+         clamp = pushF32(g, sh.f, FS.qm[s], accelerate, pp, wi, wj, wk, lc, ly, lz, o, v);
+         if (GC) gridCountAtomic(f, GC_CELL_MAX_VI, g.N, c, clamp);
          if (isnan(o[0]) || isnan(o[1]) || isnan(o[2])) raiseError(err, RHGPU_DEVERR_NAN_PARTICLE);
          int ox, oy, oz;
          int bad = migrateAxisF(o[0], ox, pp.below1);
          bad |= migrateAxisF(o[1], oy, pp.below1);
          bad |= migrateAxisF(o[2], oz, pp.below1);
-         ti = ci + ox; tj = cj + oy; tk = ck + oz;
-         const bool inside = wrapc(ti, g.nx, g.per[0]) && wrapc(tj, g.ny, g.per[1]) && wrapc(tk, g.nz, g.per[2]);
-         const double w = FS.w[s];
-         const double ke = w * ((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]);
-         if (bad || !inside) {
-            atomicAdd(&cntd[4 * s + 0], w);
-            atomicAdd(&cntd[4 * s + 1], ke);
-         } else {
-            vx = dualU(ti + halfSf(o[0]) - 1, g.nx, g.per[0]);
-            vy = dualU(tj + halfSf(o[1]) - 1, g.ny, g.per[1]);
-            vz = dualU(tk + halfSf(o[2]) - 1, g.nz, g.per[2]);
-            const bool inSeg = vy == uy && vz == uz && vx >= u0 && vx < u1;
-            if (FS.accumulate[s]) {
-               if (inSeg) {
-                  rec = true;   // its CIC weights are formed just before the record is written
-               } else {
-                  mflags |= MOVER_DEPOSIT;
-               }
+         // target cell: inside the box, and with all its neighbours
+         int ti = ci + ox, tj = cj + oy, tk = ck + oz;
+         bool inside = !bad && ((PER & 1) || (unsigned)ti < (unsigned)g.nx);
+         bool all = (PER & 1) || (unsigned)(ti - 1) < (unsigned)(g.nx - 2);
+         if (!yzIn) {
+            inside = inside && ((PER & 2) || (unsigned)tj < (unsigned)g.ny) && ((PER & 4) || (unsigned)tk < (unsigned)g.nz);
+            all = all && ((PER & 2) || (unsigned)(tj - 1) < (unsigned)(g.ny - 2)) &&
+                  ((PER & 4) || (unsigned)(tk - 1) < (unsigned)(g.nz - 2));
+         }
+         bool removed = !inside || !all;
+         if (removed) {
+            atomicAdd(&cntd[4 * s + 0], FS.w[s]);
+            atomicAdd(&cntd[4 * s + 1], FS.w[s] * ((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]));
+         }
+         if (inside) {
+            if (PER & 1) wrapc(ti, g.nx, 1);
+            if (PER & 2) wrapc(tj, g.ny, 1);
+            if (PER & 4) wrapc(tk, g.nz, 1);
+            cell = ti + g.nx * (tj + g.ny * tk);
+            // the new dual cell relative to the segment's first, and to its row
+            int du = lu + ox + halfSf(o[0]) - gx;
+            const int dy = oy + halfSf(o[1]) - gy, dz = oz + halfSf(o[2]) - gz;
+            if ((PER & 1) && nseg == 1) {
+               if (du < 0) du += fg.nd[0];
+               else if (du >= fg.nd[0]) du -= fg.nd[0];
             }
-            bool removed = false;
-            if (!allNb(g, ti, tj, tk)) {
-               removed = true;
-               atomicAdd(&cntd[4 * s + 0], w);
-               atomicAdd(&cntd[4 * s + 1], ke);
-            } else if (segInner && (f.flags[cidx(g, ti, tj, tk)] & RHGPU_FLAG_INNER_PARTICLE)) {
+            const bool inSeg = dy == 0 && dz == 0 && (unsigned)du < (unsigned)(u1 - u0);
+            duv = du;
+            dyz = (dy + 2) | ((dz + 2) << 3);
+            if (FS.accumulate[s]) {
+               rec = inSeg;   // its CIC weights are formed just before the record is written
+               if (!inSeg) mflags = MOVER_DEPOSIT;
+            }
+            if (segInner && !removed && (f.flags[cell] & RHGPU_FLAG_INNER_PARTICLE)) {
                const float xp = (float)blockOrigin(g.x_min, ti, g.dx) + o[0] * pp.dx;
                const float yp = (float)blockOrigin(g.y_min, tj, g.dx) + o[1] * pp.dx;
                const float zp = (float)blockOrigin(g.z_min, tk, g.dx) + o[2] * pp.dx;
                if (xp * xp + yp * yp + zp * zp < FS.R2obs[s]) {
                   removed = true;
-                  atomicAdd(&cntd[4 * s + 2], w);
-                  atomicAdd(&cntd[4 * s + 3], ke);
+                  atomicAdd(&cntd[4 * s + 2], FS.w[s]);
+                  atomicAdd(&cntd[4 * s + 3],
+                            FS.w[s] * ((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]));
                }
             }
             if (!removed) {
                stay = inSeg;
                if (!inSeg) mflags |= MOVER_PLACE;
             }
-            leave = mflags != 0;
          }
       }
       if (clamp) atomicAdd(&cntu[CNT_SPECIES_MAXVI + s], 1ull);
-      if (GC) gridCountAtomic(f, GC_CELL_MAX_VI, g.N, cell, clamp);
-
-      // ---- order of the chunk's stayers and records (warp-local first) ---------------------
-      const unsigned bs = __ballot_sync(0xffffffffu, stay), br = __ballot_sync(0xffffffffu, rec);
-      if (lane == 0) sh.wcnt[warp] = __popc(bs);
+      // order of the group's stayers and records: ballots, and its records per dual cell
+      const unsigned bs = __ballot_sync(0xffffffffu, stay);
+      const unsigned br = __ballot_sync(0xffffffffu, rec);
+      if (lane == 0) {
+         const int n = __popc(bs);
+         sh.wcnt[warp] = n;
+         if (n) atomicAdd(&sh.stay[s], n);
+      }
       sh.wd[lane][warp] = 0;
       __syncwarp();
-      const int rd = rec ? vx - u0 : 0;
-      int rrank = 0;
       if (rec) {
-         const unsigned mm = __match_any_sync(br, rd);
+         const unsigned mm = __match_any_sync(br, duv);
          rrank = __popc(mm & below);
-         if (rrank == 0) sh.wd[rd][warp] = (unsigned char)__popc(mm);
+         if (rrank == 0) sh.wd[duv][warp] = (unsigned char)__popc(mm);
       }
       __syncthreads();
       // every shared-memory read of this chunk's particles is done: request the next chunk's
-      f32Prefetch(sh, i + FT, total, ns, s);
-      // every warp, per dual cell (lane): the first sorted record of the dual cell
-      // (bin) and of this warp's records for it (off)
-      int binD, offD, nrec;
+      if (V0 + PD_VW < groups) f32Prefetch(sh, V0 + PD_VW, ns);
+      // every warp, per dual cell (lane): the first sorted record of the dual cell (bin)
+      const uint2 c8 = *reinterpret_cast<const uint2*>(&sh.wd[lane][0]);
+      int binD, nrec;
       {
-         const uint2 c8 = *reinterpret_cast<const uint2*>(&sh.wd[lane][0]);
          const int t = (int)(((c8.x * 0x01010101u) >> 24) + ((c8.y * 0x01010101u) >> 24));
-         const unsigned mlo = warp >= 4 ? 0xffffffffu : (1u << (8 * warp)) - 1u;
-         const unsigned mhi = warp <= 4 ? 0u : (1u << (8 * (warp - 4))) - 1u;
-         const int before = (int)((((c8.x & mlo) * 0x01010101u) >> 24) + (((c8.y & mhi) * 0x01010101u) >> 24));
          int x = t;
          for (int q = 1; q < 32; q <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, q);
             if (lane >= q) x += y;
          }
          binD = x - t;
-         offD = binD + before;
          nrec = __shfl_sync(0xffffffffu, x, 31);
       }
-      const int recPos = __shfl_sync(0xffffffffu, offD, rd) + rrank;
       const int sumLo = __shfl_sync(0xffffffffu, binD, myDual);
       const int sumHiN = __shfl_sync(0xffffffffu, binD, (myDual + 1) & 31);
       const int sumHi = myDual == SEG - 1 ? nrec : sumHiN;
-      // stayers of the chunk before this position (and in all), and this species' count so far
-      const int wc = lane < FW ? sh.wcnt[lane] : 0;
-      const int myRank = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < warp ? wc : 0)) + __popc(bs & below);
-      const int chunkStay = (int)__reduce_add_sync(0xffffffffu, (unsigned)wc);
-      sh.rank[tid] = myRank;
-      const int stayBase = stay ? sh.stay[s] : 0;
+      const int wc = lane < PD_VW ? sh.wcnt[lane] : 0;
+      // this group's records start after those of the groups before it, per dual cell
+      const unsigned mlo = warp >= 4 ? 0xffffffffu : (1u << (8 * warp)) - 1u;
+      const unsigned mhi = warp <= 4 ? 0u : (1u << (8 * (warp - 4))) - 1u;
+      const int before = (int)((((c8.x & mlo) * 0x01010101u) >> 24) + (((c8.y & mhi) * 0x01010101u) >> 24));
+      const int recPos = __shfl_sync(0xffffffffu, binD + before, rec ? duv : 0) + rrank;
+      // next slot of a stayer: the species' stayers up to and with the chunk less those from this group on
+      const int vEnd = sh.first[s + 1] - V0;
+      const int from = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane >= warp && lane < vEnd ? wc : 0));
+      const int slot = sh.stay[s] - from + __popc(bs & below);
       // mover slots reserved now, written after the sums
-      const unsigned lm = __ballot_sync(0xffffffffu, leave);
-      const int leader = lm ? __ffs(lm) - 1 : 0;
+      const unsigned lm = __ballot_sync(0xffffffffu, mflags != 0);
       unsigned long long mb = 0;
-      if (lm && lane == leader) mb = atomicAdd(fb.nmovers, (unsigned long long)__popc(lm));
+      if (lm && lane == __ffs(lm) - 1) mb = atomicAdd(fb.nmovers, (unsigned long long)__popc(lm));
       if (rec) {
          float w8[8];
          cicWeightsF(o, FS.wqRel[s], w8);
-         float* r = sh.rec + recPos * REC32;
-         for (int q = 0; q < 8; ++q) r[q] = w8[q];
-         r[8] = v[0]; r[9] = v[1]; r[10] = v[2];
+         float4* const r = reinterpret_cast<float4*>(sh.rec + recPos * REC32);
+         r[0] = make_float4(w8[0], w8[1], w8[2], w8[3]);
+         r[1] = make_float4(w8[4], w8[5], w8[6], w8[7]);
+         r[2] = make_float4(1.0f, v[0], v[1], v[2]);
       }
       __syncthreads();
       if (stay) {
-         const int p0 = sh.prefix[s] - c0;   // chunk position of the species' first particle
-         const int q = stayBase + myRank - (p0 > 0 ? sh.rank[p0] : 0);
-         ((int*)sh.ptr[s][7])[q] = (int)cidx(g, ti, tj, tk);
+         void* const* nx = &sh.ptr[s][7];
+         ((int*)nx[0])[slot] = cell;
+#pragma unroll
          for (int a = 0; a < 3; ++a) {
-            ((float*)sh.ptr[s][8 + a])[q] = o[a];
-            ((float*)sh.ptr[s][11 + a])[q] = v[a];
+            ((float*)nx[1 + a])[slot] = o[a];
+            ((float*)nx[4 + a])[slot] = v[a];
          }
       }
-      // running stayer count of each species
-      if (tid < ns) {
-         const int lo = min(max(sh.prefix[tid] - c0, 0), FT), hi = min(max(sh.prefix[tid + 1] - c0, 0), FT);
-         const int rlo = lo < FT ? sh.rank[lo] : chunkStay, rhi = hi < FT ? sh.rank[hi] : chunkStay;
-         sh.stay[tid] += rhi - rlo;
-      }
-      // ---- sums of this thread's (dual cell, corner), records in list order ----------------
+      // ---- this thread's sums, records in list order ----------------------------------------
 #pragma unroll 2
       for (int r = sumLo; r < sumHi; ++r) {
-         const float* rr = sh.rec + r * REC32;
-         const float w = rr[myCorner];
-         a0 += w;
-         a1 = fmaf(w, rr[8], a1);
-         a2 = fmaf(w, rr[9], a2);
-         a3 = fmaf(w, rr[10], a3);
+         const float2* const rr = reinterpret_cast<const float2*>(sh.rec + r * REC32);
+         const float2 w = rr[myPair], u = rr[4 + myHalf];
+         a00 = fmaf(w.x, u.x, a00);
+         a01 = fmaf(w.x, u.y, a01);
+         a10 = fmaf(w.y, u.x, a10);
+         a11 = fmaf(w.y, u.y, a11);
       }
       // ---- particles that left the segment -----------------------------------------------
-      if (lm) {
-         mb = __shfl_sync(0xffffffffu, mb, leader);
-         if (leave) {
-            const unsigned long long m = mb + __popc(lm & below);
-            if ((long long)m < fb.moverCap) {
-               Mover32& M = fb.movers[m];
-               for (int a = 0; a < 3; ++a) { M.o[a] = o[a]; M.v[a] = v[a]; }
-               M.cell = (int)cidx(g, ti, tj, tk);
-               M.species = s;
-               M.key = ((unsigned long long)S << 32) | (unsigned long long)p;
-               const int gd = vx / SEG;
-               M.dest = ((long long)vy + (long long)fg.nd[1] * vz) * fg.nseg + gd;
-               M.lx = (vx - gd * SEG) | mflags;
-            } else {
-               raiseError(err, RHGPU_DEVERR_CAPACITY);
-            }
-         }
+      if (!lm) continue;
+      const unsigned long long m0 = __shfl_sync(0xffffffffu, mb, __ffs(lm) - 1);
+      if (!mflags) continue;
+      const unsigned long long m = m0 + __popc(lm & below);
+      if ((long long)m >= fb.moverCap) {
+         raiseError(err, RHGPU_DEVERR_CAPACITY);
+         continue;
       }
-      // no barrier here: the next chunk's first barrier orders the reads of rec,
-      // rank and stay before their next writes
+      int vx = u0 + duv, vy = uy + (dyz & 7) - 2, vz = uz + (dyz >> 3) - 2;
+      if (PER & 1) wrapc(vx, fg.nd[0], 1);
+      if (PER & 2) wrapc(vy, fg.nd[1], 1);
+      if (PER & 4) wrapc(vz, fg.nd[2], 1);
+      Mover32& M = fb.movers[m];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) { M.o[a] = o[a]; M.v[a] = v[a]; }
+      M.cell = cell;
+      M.species = s;
+      M.key = ((unsigned long long)S << 32) | (unsigned long long)p;
+      const int gd = vx / SEG;
+      M.dest = ((long long)vy + (long long)fg.nd[1] * vz) * nseg + gd;
+      M.lx = (vx - gd * SEG) | mflags;
+      // no barrier here: the next chunk's first barrier orders the reads of rec
+      // and wd before their next writes
    }
 
    __syncthreads();
    if (tid < ns) FS.st[tid].nxt.cnt[S] = sh.stay[tid];
    {
-      float* q = sh.rec + myDual * 32 + myCorner * 4;
-      q[0] = a0; q[1] = a1; q[2] = a2; q[3] = a3;
+      float* const q = sh.rec + myDual * 32 + myPair * 8 + myHalf * 2;
+      q[0] = a00; q[1] = a01; q[4] = a10; q[5] = a11;
    }
    __syncthreads();
-   const int nx = g.nx;
-   const long long nrows = fg.nrows;
-   for (int e = tid; e < SEG * 16; e += FT) {
-      const int dl = e >> 4, qq = (e >> 2) & 3, m = e & 3;
-      const int lo = u0 + dl;
-      if (lo >= u1) continue;
-      int x, hi;
-      if (g.per[0]) {
-         x = lo + 1 == nx ? 0 : lo + 1;
-         hi = lo + 1 < u1 ? dl + 1 : (fg.nseg == 1 ? 0 : -1);
-      } else {
-         x = lo;
-         if (x >= nx) continue;
-         hi = lo + 1 < u1 ? dl + 1 : -1;
-      }
-      float val = sh.rec[dl * 32 + ((1 + 2 * qq) << 2) + m];
-      if (hi >= 0) val = val + sh.rec[hi * 32 + ((2 * qq) << 2) + m];
-      fb.RP[(((long long)qq * nrows + row) * nx + x) * 4 + m] = val;
-   }
-   if (tid < 16 && (g.per[0] ? fg.nseg > 1 : gseg >= 1)) {
-      const int qq = tid >> 2, m = tid & 3;
-      fb.RPB[(((long long)qq * nrows + row) * fg.nseg + gseg) * 4 + m] = sh.rec[((2 * qq) << 2) + m];
-   }
+   segPartialsOut<PD_T>(g, fg, fb.RP, fb.RPB, sh.rec, row, gseg, u0, u1);
 }
 
 // corner o's four deposits of one mover (k_mover_pass): cicWeightsF's products, in its order

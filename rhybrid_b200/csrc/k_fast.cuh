@@ -25,9 +25,9 @@
 //                        next buffer in order; their deposit records go to
 //                        shared memory counting-sorted by target dual cell
 //                        (stable) and are summed sequentially per (dual cell,
-//                        corner, moment) in FP64, one thread per (dual cell,
-//                        corner). Particles that leave the segment go to the
-//                        mover list.
+//                        corner, moment) in FP64, one thread per two corners
+//                        and two moments. Particles that leave the segment go
+//                        to the mover list.
 //   k_mover_pass         the movers' CIC contributions as exact 128-bit
 //                        fixed-point sums (order-independent), and their count
 //                        per destination
@@ -46,10 +46,10 @@ namespace rh {
 
 constexpr int FAST_MAX_SPECIES = 8;
 constexpr int SEG = RHGPU_FAST_SEGMENT;   // dual cells per segment
-constexpr int FT = 256;                   // threads of k_fast_push_deposit (one chunk of particles)
+constexpr int FT = 256;                   // threads of k_fast_avg_deposit (one chunk of particles)
 constexpr int FW = FT / 32;
-constexpr int REC = 11;                   // doubles per deposit record: w8[8], v[3]
-static_assert(SEG == 32 && SEG * 8 == FT, "the deposit sums map (dual cell, corner) to one thread");
+constexpr int REC = 11;                   // its doubles per deposit record: w8[8], v[3]
+static_assert(SEG == 32 && SEG * 8 == FT, "its deposit sums map (dual cell, corner) to one thread");
 
 struct SegBuf {
    double* a[7];        // x, y, z (cell-local), vx, vy, vz, weight
@@ -164,28 +164,17 @@ __device__ inline void cicWeightsLocal(double x, double y, double z, double wq, 
    w8[7] = w_x * w_y * w_z * wq;
 }
 
-// stayers of a chunk in the chunk positions [p0, p1), from the warps' stayer ballots
-__device__ inline int stayersIn(const unsigned* bs, int p0, int p1) {
-   int n = 0;
-   for (int w = 0; w < FW; ++w) {
-      const int lo = max(p0 - 32 * w, 0), hi = min(p1 - 32 * w, 32);
-      if (lo >= hi) continue;
-      const unsigned m = (hi == 32 ? ~0u : ((1u << hi) - 1u)) & (~0u << lo);
-      n += __popc(bs[w] & m);
-   }
-   return n;
-}
-
 // the field stencil of one segment's cells in shared memory: local cell
 // (lc, ly, lz) = global (xs0 + lc, ys0 + ly, zs0 + lz), lc in [0, SEG],
 // ly, lz in {0, 1}; faceB also holds the -x / -y / -z neighbour faces
+// (every x-row has the same length, so that one offset serves all but by)
 template <class T>
 struct SegFieldsT {
    T bx[2][2][SEG + 2];    // [lz][ly][lc + 1]
-   T by[2][3][SEG + 1];    // [lz][ly + 1][lc]
-   T bz[3][2][SEG + 1];    // [lz + 1][ly][lc]
-   T ue[3][2][2][SEG + 1]; // [l][lz][ly][lc]
-   T ep[3][2][2][SEG + 1];
+   T by[2][3][SEG + 2];    // [lz][ly + 1][lc]
+   T bz[3][2][SEG + 2];    // [lz + 1][ly][lc]
+   T ue[3][2][2][SEG + 2]; // [l][lz][ly][lc]
+   T ep[3][2][2][SEG + 2];
 };
 using SegFields = SegFieldsT<double>;
 constexpr int SF_ROWS_B = 4 + 6 + 6;    // x-rows of faceB components in the stencil
@@ -229,7 +218,6 @@ __device__ inline T* stencilRow(SegFieldsT<T>& F, const Fields& f, int r, int& l
 // loads of a thread are issued before its shared-memory stores
 constexpr int SF_ROW_W = SEG + 2;                               // slots per row (bx rows use all)
 constexpr int SF_MAX_ROWS = SF_ROWS_B + 2 * SF_ROWS_C;
-constexpr int SF_PER_THREAD = (SF_MAX_ROWS * SF_ROW_W + FT - 1) / FT;
 struct StencilRow {
    const double* src;   // global x = 0 of the row, or nullptr (zeros)
    int dst;             // element offset of the row in the stencil
@@ -237,7 +225,7 @@ struct StencilRow {
    int len;             // elements of the row
 };
 
-template <class T>
+template <int NT, class T>
 __device__ inline void stageSegRows(const GridInfo& g, const Fields& f, bool useEp, int xs0, int ys0, int zs0,
                                     SegFieldsT<T>& F, StencilRow* rows) {
    const int nrows = SF_ROWS_B + SF_ROWS_C * (useEp ? 2 : 1);
@@ -259,11 +247,12 @@ __device__ inline void stageSegRows(const GridInfo& g, const Fields& f, bool use
       rows[tid] = r;
    }
    __syncthreads();
+   constexpr int SF_PER_THREAD = (SF_MAX_ROWS * SF_ROW_W + NT - 1) / NT;
    double v[SF_PER_THREAD];
    int d[SF_PER_THREAD];
 #pragma unroll
    for (int k = 0; k < SF_PER_THREAD; ++k) {
-      const int e = tid + FT * k;
+      const int e = tid + NT * k;
       const int ri = e / SF_ROW_W, c = e - ri * SF_ROW_W;
       v[k] = 0.0;
       d[k] = -1;
@@ -281,26 +270,52 @@ __device__ inline void stageSegRows(const GridInfo& g, const Fields& f, bool use
       if (d[k] >= 0) base[d[k]] = (T)v[k];
 }
 
-// pushOne with the fields from the segment's staged stencil and divDx; the
-// same arithmetic in the same order
-__device__ inline bool pushStaged(const GridInfo& g, const SegFields& F, const SpeciesDev& sp, const PushParams& pp,
-                                  int i, int j, int k, int lc, int ly, int lz, double st[7]) {
+// x, y, z in [0, dx) over dx, as divDx: the three quotients' range is tested at
+// once, by exponent (2^-500 to 2^500; zeros, negative and non-finite values fail it)
+__device__ __forceinline__ void divDx3(double x, double y, double z, const GridInfo& g, double q[3]) {
+   q[0] = x * g.rdx; q[1] = y * g.rdx; q[2] = z * g.rdx;
+   constexpr unsigned LO = (1023u - 500u) << 20, RANGE = 1000u << 20;
+   const unsigned e = max(max((unsigned)__double2hiint(q[0]) - LO, (unsigned)__double2hiint(q[1]) - LO),
+                          (unsigned)__double2hiint(q[2]) - LO);
+   if (e < RANGE) {
+      q[0] = fma(fma(-q[0], g.dx, x), g.rdx, q[0]);
+      q[1] = fma(fma(-q[1], g.dx, y), g.rdx, q[1]);
+      q[2] = fma(fma(-q[2], g.dx, z), g.rdx, q[2]);
+   } else {
+      q[0] = x / g.dx; q[1] = y / g.dx; q[2] = z / g.dx;
+   }
+}
+
+// push of one particle with the fields of cell (lc, ly, lz) of the segment's
+// staged stencil, the arithmetic and order of the exact path's k_push with its
+// divisions by dx as divDx; true if its speed was clamped. (i, j, k) is the
+// cell, used by gravity only.
+__device__ __forceinline__ bool pushStaged(const GridInfo& g, const SegFields& F, double qm, bool accelerate,
+                                           const PushParams& pp, int i, int j, int k, int lc, int ly, int lz, double st[7]) {
    bool clamp = false;
-   const bool accelerate = sp.accelerate && !pp.useIFT && allNb(g, i, j, k);
    double vx = st[3], vy = st[4], vz = st[5];
    if (accelerate) {
-      const double dx = g.dx;
-      double B[3], Ue[3], E[3];
-      const double xs = divDx(st[0], g), ys = divDx(st[1], g), zs = divDx(st[2], g);
-      B[0] = (xs - 0.0) * F.bx[lz][ly][lc + 1] + (1.0 - xs) * F.bx[lz][ly][lc];
-      B[1] = (ys - 0.0) * F.by[lz][ly + 1][lc] + (1.0 - ys) * F.by[lz][ly][lc];
-      B[2] = (zs - 0.0) * F.bz[lz + 1][ly][lc] + (1.0 - zs) * F.bz[lz][ly][lc];
-      for (int l = 0; l < 3; ++l) Ue[l] = F.ue[l][lz][ly][lc];
+      constexpr int SX = SEG + 2;
+      const int o = (2 * lz + ly) * SX + lc;      // bx, bz, ue, ep
+      const double* const bx = &F.bx[0][0][0] + o;
+      const double* const by = &F.by[0][0][0] + o + lz * SX;
+      const double* const bz = &F.bz[0][0][0] + o;
+      const double* const ue = &F.ue[0][0][0][0] + o;
+      double B[3], Ue[3], E[3], q[3];
+      divDx3(st[0], st[1], st[2], g, q);
+      B[0] = q[0] * bx[1] + (1.0 - q[0]) * bx[0];
+      B[1] = q[1] * by[SX] + (1.0 - q[1]) * by[0];
+      B[2] = q[2] * bz[2 * SX] + (1.0 - q[2]) * bz[0];
+#pragma unroll
+      for (int l = 0; l < 3; ++l) Ue[l] = ue[4 * SX * l];
       E[0] = B[1] * Ue[2] - B[2] * Ue[1];
       E[1] = B[2] * Ue[0] - B[0] * Ue[2];
       E[2] = B[0] * Ue[1] - B[1] * Ue[0];
-      if (pp.use_ep) for (int l = 0; l < 3; ++l) E[l] += F.ep[l][lz][ly][lc];
-      const double qm = sp.qmideltT2;
+      if (pp.use_ep) {
+         const double* const ep = &F.ep[0][0][0][0] + o;
+#pragma unroll
+         for (int l = 0; l < 3; ++l) E[l] += ep[4 * SX * l];
+      }
       const double dvx = qm * E[0], dvy = qm * E[1], dvz = qm * E[2];
       const double tx = qm * B[0], ty = qm * B[1], tz = qm * B[2];
       const double t2 = tx * tx + ty * ty + tz * tz;
@@ -315,8 +330,8 @@ __device__ inline bool pushStaged(const GridInfo& g, const SegFields& F, const S
       const double vpz = vmz + v0x * sy - v0y * sx;
       vx = vpx + dvx; vy = vpy + dvy; vz = vpz + dvz;
       if (pp.use_gravity) {
-         const double xg = st[0] + blockOrigin(g.x_min, i, dx), yg = st[1] + blockOrigin(g.y_min, j, dx),
-                      zg = st[2] + blockOrigin(g.z_min, k, dx);
+         const double xg = st[0] + blockOrigin(g.x_min, i, g.dx), yg = st[1] + blockOrigin(g.y_min, j, g.dx),
+                      zg = st[2] + blockOrigin(g.z_min, k, g.dx);
          const double rr = sqrt(sq(xg) + sq(yg) + sq(zg));
          const double r3 = rr * rr * rr;
          if (r3 > 0) {
@@ -338,81 +353,18 @@ __device__ inline bool pushStaged(const GridInfo& g, const SegFields& F, const S
    return clamp;
 }
 
-// push of one particle at local position st[0..2] in cell (i,j,k); returns true if clamped
-__device__ inline bool pushOne(const GridInfo& g, const Fields& f, const SpeciesDev& sp, const PushParams& pp,
-                               int i, int j, int k, double st[7]) {
-   const long long N = g.N;
-   const long long c = cidx(g, i, j, k);
-   bool clamp = false;
-   const bool accelerate = sp.accelerate && !pp.useIFT && allNb(g, i, j, k);
-   double vx = st[3], vy = st[4], vz = st[5];
-   if (accelerate) {
-      const double dx = g.dx;
-      double B[3], Ue[3], E[3];
-      const double xs = st[0] / dx, ys = st[1] / dx, zs = st[2] / dx;
-      B[0] = (xs - 0.0) * f.faceB[0 * N + c] + (1.0 - xs) * f.faceB[0 * N + nbr(g, i, j, k, -1, 0, 0)];
-      B[1] = (ys - 0.0) * f.faceB[1 * N + c] + (1.0 - ys) * f.faceB[1 * N + nbr(g, i, j, k, 0, -1, 0)];
-      B[2] = (zs - 0.0) * f.faceB[2 * N + c] + (1.0 - zs) * f.faceB[2 * N + nbr(g, i, j, k, 0, 0, -1)];
-      for (int l = 0; l < 3; ++l) Ue[l] = f.cellUe[l * N + c];
-      E[0] = B[1] * Ue[2] - B[2] * Ue[1];
-      E[1] = B[2] * Ue[0] - B[0] * Ue[2];
-      E[2] = B[0] * Ue[1] - B[1] * Ue[0];
-      if (pp.use_ep) for (int l = 0; l < 3; ++l) E[l] += f.cellEp[l * N + c];
-      const double qm = sp.qmideltT2;
-      const double dvx = qm * E[0], dvy = qm * E[1], dvz = qm * E[2];
-      const double tx = qm * B[0], ty = qm * B[1], tz = qm * B[2];
-      const double t2 = tx * tx + ty * ty + tz * tz;
-      const double b2 = 2. / (1. + t2);
-      const double sx = b2 * tx, sy = b2 * ty, sz = b2 * tz;
-      const double vmx = vx + dvx, vmy = vy + dvy, vmz = vz + dvz;
-      const double v0x = vmx + vmy * tz - vmz * ty;
-      const double v0y = vmy + vmz * tx - vmx * tz;
-      const double v0z = vmz + vmx * ty - vmy * tx;
-      const double vpx = vmx + v0y * sz - v0z * sy;
-      const double vpy = vmy + v0z * sx - v0x * sz;
-      const double vpz = vmz + v0x * sy - v0y * sx;
-      vx = vpx + dvx; vy = vpy + dvy; vz = vpz + dvz;
-      if (pp.use_gravity) {
-         const double xg = st[0] + blockOrigin(g.x_min, i, dx), yg = st[1] + blockOrigin(g.y_min, j, dx),
-                      zg = st[2] + blockOrigin(g.z_min, k, dx);
-         const double rr = sqrt(sq(xg) + sq(yg) + sq(zg));
-         const double r3 = rr * rr * rr;
-         if (r3 > 0) {
-            const double s = -pp.GMdt / r3;
-            vx += s * xg; vy += s * yg; vz += s * zg;
-         }
-      }
-      const double v2 = sq(vx) + sq(vy) + sq(vz);
-      if (v2 > pp.maxVi2) {
-         const double norm = sqrt(pp.maxVi2 / v2);
-         vx *= norm; vy *= norm; vz *= norm;
-         clamp = true;
-      }
-   }
-   st[3] = vx; st[4] = vy; st[5] = vz;
-   st[0] += g.dt * vx;
-   st[1] += g.dt * vy;
-   st[2] += g.dt * vz;
-   return clamp;
-}
-
-// PER: the periodic axes (bit a = axis a), fixed at compile time; the host
-// launches the instantiation that matches the grid
-// the block's sums per (dual cell, corner) -> the segment's row partials (corner
-// ox = 1 of each dual cell plus ox = 0 of the next) and, where the first dual
-// cell's partner is in another segment, its boundary partial. s_rec is free.
-__device__ __forceinline__ void segPartialsOut(const GridInfo& g, const FastGeom& fg, const FastBufs& fb, double* s_rec,
-                                               long long row, int gseg, int u0, int u1, double a0, double a1,
-                                               double a2, double a3) {
-   const int tid = threadIdx.x, myDual = tid >> 3, myCorner = tid & 7;
-   {
-      double* q = s_rec + myDual * 32 + myCorner * 4;
-      q[0] = a0; q[1] = a1; q[2] = a2; q[3] = a3;
-   }
-   __syncthreads();
+// the block's sums per (dual cell, corner, moment), in acc[dual * 32 + corner *
+// 4 + moment] -> the segment's row partials (corner ox = 1 of each dual cell
+// plus ox = 0 of the next) and, where the first dual cell's partner is in
+// another segment, its boundary partial. NT threads.
+template <int NT, class T>
+__device__ __forceinline__ void segPartialsOut(const GridInfo& g, const FastGeom& fg, T* RP, T* RPB, const T* acc,
+                                               long long row, int gseg, int u0, int u1) {
+   const int tid = threadIdx.x;
    const int nx = g.nx;
    const long long nrows = fg.nrows;
-   for (int e = tid; e < SEG * 16; e += FT) {
+#pragma unroll
+   for (int e = tid; e < SEG * 16; e += NT) {
       const int dl = e >> 4, qq = (e >> 2) & 3, m = e & 3;
       const int lo = u0 + dl;   // the dual cell giving corner ox = 1 to cell x
       if (lo >= u1) continue;
@@ -425,14 +377,14 @@ __device__ __forceinline__ void segPartialsOut(const GridInfo& g, const FastGeom
          if (x >= nx) continue;
          hi = lo + 1 < u1 ? dl + 1 : -1;
       }
-      double v = s_rec[dl * 32 + ((1 + 2 * qq) << 2) + m];
-      if (hi >= 0) v = v + s_rec[hi * 32 + ((2 * qq) << 2) + m];
-      fb.RP[(((long long)qq * nrows + row) * nx + x) * 4 + m] = v;
+      T v = acc[dl * 32 + ((1 + 2 * qq) << 2) + m];
+      if (hi >= 0) v = v + acc[hi * 32 + ((2 * qq) << 2) + m];
+      RP[(((long long)qq * nrows + row) * nx + x) * 4 + m] = v;
    }
    // corner ox = 0 of the first dual cell, when the cell's other dual cell is in another segment
    if (tid < 16 && (g.per[0] ? fg.nseg > 1 : gseg >= 1)) {
       const int qq = tid >> 2, m = tid & 3;
-      fb.RPB[(((long long)qq * nrows + row) * fg.nseg + gseg) * 4 + m] = s_rec[((2 * qq) << 2) + m];
+      RPB[(((long long)qq * nrows + row) * fg.nseg + gseg) * 4 + m] = acc[((2 * qq) << 2) + m];
    }
 }
 
@@ -440,39 +392,39 @@ __device__ __forceinline__ void segPartialsOut(const GridInfo& g, const FastGeom
 // x..w (7-13), current lx (14), next lx (15)
 constexpr int SEG_PTRS = 16;
 
+// k_fast_push_deposit: one thread per particle of a chunk, a warp's 32 particles
+// a group of one species
+constexpr int PD_T = 256, PD_VW = PD_T / 32;
+static_assert(PD_VW == 8, "a dual cell's record counts per group are the bytes of a 64-bit word");
+static_assert(SEG * 8 == PD_T, "the deposit sums map (dual cell, corner pair, moment pair) to one thread");
+// a deposit record: w8[8], then 1, vx, vy, vz, so that the charge is one more
+// product of the same sum; 14 doubles apart, so that the 16-byte accesses of
+// eight lanes at any records fall on different banks
+constexpr int PD_REC = 14;
+
 // shared memory of k_fast_push_deposit (dynamic: more than the 48 KB static limit)
 struct PushDepositShared {
-   double rec[FT * REC];                  // deposit records of a chunk; at the end acc[SEG][32]
-   double pf[7][FT];                      // the next chunk's particles, one plane per component
+   double rec[PD_T * PD_REC];            // deposit records of a chunk; at the end acc[SEG][32]
+   double pf[7][PD_T];                // the next chunk's particles, one plane per component
    SegFields f;                           // field stencil of the segment
    void* ptr[FAST_MAX_SPECIES][SEG_PTRS];
    StencilRow rows[SF_MAX_ROWS];
-   alignas(8) unsigned char wd[SEG][FW];  // records per (dual cell, warp)
-   int rank[FT];                          // stayers of the chunk before each chunk position
-   int wcnt[FW];                          // stayers per warp
-   int prefix[FAST_MAX_SPECIES + 1];      // first particle of each species in the segment
-   int stay[FAST_MAX_SPECIES];            // stayers of each species so far
+   alignas(8) unsigned char wd[SEG][PD_VW];   // records per (dual cell, group)
+   int wcnt[PD_VW];                       // stayers per group
+   int first[FAST_MAX_SPECIES + 1];       // first group of each species in the segment
+   int cnt[FAST_MAX_SPECIES];             // particles of each species in the segment
+   int stay[FAST_MAX_SPECIES];            // stayers of each species up to and with the chunk
 };
 constexpr size_t PUSH_DEPOSIT_SMEM = sizeof(PushDepositShared);
+static_assert(PD_T * PD_REC >= SEG * 32, "the final sums reuse the records");
 
-// the segment's first chunk and the field stencil requested with cp.async: the
-// stencil rows (see stageSegRows) with zeros outside a non-periodic box, the
-// particles of chunk positions tid into pf
+// the field stencil requested with cp.async: the stencil rows (see
+// stageSegRows) with zeros outside a non-periodic box
 template <int PER>
-__device__ __forceinline__ void pdStage(const GridInfo& g, const Fields& f, bool useEp, PushDepositShared& sh,
-                                        int total, int ns, int& lxNext) {
-   const int tid = threadIdx.x;
-   if (tid < total) {
-      int s = 0;
-      while (s + 1 < ns && tid >= sh.prefix[s + 1]) ++s;
-      const int p = tid - sh.prefix[s];
-#pragma unroll
-      for (int a = 0; a < 7; ++a) cpAsync8(&sh.pf[a][tid], (const double*)sh.ptr[s][a] + p, 8);
-      lxNext = ((const unsigned char*)sh.ptr[s][14])[p];
-   }
+__device__ __forceinline__ void pdStage(const GridInfo& g, const Fields& f, bool useEp, PushDepositShared& sh) {
    const int nrows = SF_ROWS_B + SF_ROWS_C * (useEp ? 2 : 1);
    double* const base = (double*)&sh.f;
-   for (int e = tid; e < nrows * SF_ROW_W; e += FT) {
+   for (int e = threadIdx.x; e < nrows * SF_ROW_W; e += PD_T) {
       const int ri = e / SF_ROW_W, c = e - ri * SF_ROW_W;
       const StencilRow r = sh.rows[ri];
       if (c >= r.len) continue;
@@ -481,15 +433,41 @@ __device__ __forceinline__ void pdStage(const GridInfo& g, const Fields& f, bool
       const bool ok = r.src != nullptr && x >= 0 && x < g.nx;
       cpAsync8(base + r.dst + c, ok ? r.src + x : f.faceB, ok ? 8 : 0);
    }
+}
+
+// species of group V of the segment (groups past the last one: the last species)
+template <class SH>
+__device__ __forceinline__ int pdSpecies(const SH& sh, int V, int ns) {
+   int s = 0;
+   while (s + 1 < ns && V >= sh.first[s + 1]) ++s;
+   return s;
+}
+
+// this thread's particle of the chunk that starts at group V0 requested into pf
+__device__ __forceinline__ void pdPrefetch(PushDepositShared& sh, int V0, int ns, int& lx) {
+   const int tid = threadIdx.x, V = V0 + (tid >> 5);
+   const int s = pdSpecies(sh, V, ns);
+   const int p = (V - sh.first[s]) * 32 + (tid & 31);
+   if (p < sh.cnt[s]) {
+#pragma unroll
+      for (int a = 0; a < 7; ++a) cpAsync8(&sh.pf[a][tid], (const double*)sh.ptr[s][a] + p, 8);
+      lx = ((const unsigned char*)sh.ptr[s][14])[p];
+   }
    cpAsyncCommit();
 }
 
-// cicWeightsLocal with the dual cell's lower centre (i - 1 + 0.5) dx = -dx/2 or
-// +dx/2 selected (both exact), the same weights bit for bit
-__device__ __forceinline__ void cicWeightsHalf(double x, double y, double z, double wq, const GridInfo& g, double hdx,
-                                               double w8[8]) {
-   const double x0 = x < hdx ? -hdx : hdx, y0 = y < hdx ? -hdx : hdx, z0 = z < hdx ? -hdx : hdx;
-   const double w_x = divDx(x - x0, g), w_y = divDx(y - y0, g), w_z = divDx(z - z0, g);
+// the CIC weights of a position in its cell, as cicWeightsLocal, bit for bit.
+// The quotients need no range test: the numerators are 0 or at least an ulp of
+// dx / 2, at most dx.
+__device__ __forceinline__ void cicWeightsHalf(double x, double y, double z, bool hx, bool hy, bool hz, double wq,
+                                               const GridInfo& g, double hdx, double w8[8]) {
+   const double rx = hx ? x - hdx : x + hdx, ry = hy ? y - hdx : y + hdx, rz = hz ? z - hdx : z + hdx;
+   double q = rx * g.rdx;
+   const double w_x = fma(fma(-q, g.dx, rx), g.rdx, q);
+   q = ry * g.rdx;
+   const double w_y = fma(fma(-q, g.dx, ry), g.rdx, q);
+   q = rz * g.rdx;
+   const double w_z = fma(fma(-q, g.dx, rz), g.rdx, q);
    w8[0] = (1 - w_x) * (1 - w_y) * (1 - w_z) * wq;
    w8[1] = w_x * (1 - w_y) * (1 - w_z) * wq;
    w8[2] = (1 - w_x) * w_y * (1 - w_z) * wq;
@@ -500,19 +478,38 @@ __device__ __forceinline__ void cicWeightsHalf(double x, double y, double z, dou
    w8[7] = w_x * w_y * w_z * wq;
 }
 
+// migration of one axis (migrateAxis); a coordinate inside [0, dx) is told by
+// one unsigned comparison of its bits (negative values and NaN compare above)
+__device__ __forceinline__ int migrateAxisBits(double& x, int& off, const GridInfo& g, bool& nan) {
+   off = 0;
+   if ((unsigned long long)__double_as_longlong(x) < (unsigned long long)__double_as_longlong(g.dx)) return 0;
+   nan |= isnan(x);
+   return migrateAxis(x, off, g.dx, g.dx_below);
+}
+
 // EXTRA: the variant with the optional outputs (the removed in-segment deposits
 // listed for the population averages, the per-cell maxVi constraint counter);
 // the default instantiation carries neither.
+// PER: the periodic axes (bit a = axis a), fixed at compile time; the host
+// launches the instantiation that matches the grid.
 //
-// One block per segment, one thread per particle, chunks of FT particles in
-// storage order (species after species). The particles of chunk k+1 are copied
-// to shared memory (cp.async, each thread its own position) while chunk k is
-// processed; per chunk two barriers order the records and the stayers. A
-// particle leaving the segment reserves its mover slot before the second
-// barrier and is written after the deposit sums, so the reservation's round
-// trip overlaps the chunk's remaining work.
+// One block per segment; chunks of PD_T particles in storage order, species
+// after species, every species starting at a group of 32 so that a warp's
+// species is uniform. The particles of chunk k+1 are copied to shared memory
+// (cp.async, each thread its own position) while chunk k is processed; per chunk
+// two barriers order the records and the stayers. A particle leaving the segment reserves its mover
+// slot before the second barrier and is written after the deposit sums, so the
+// reservation's round trip overlaps the chunk's remaining work.
+//
+// It is bound by issue slots and the waits between them at the 32 warps per SM
+// that 64 registers and 57 KB of shared memory leave (62 % of cycles issue, 67 %
+// of the shared-memory wavefronts), not by memory.
+// Mars run, 9.25e7 ions, 120 x 160 x 160 cells: 4.33 ms per step = 2300 GB/s of
+// its 104 bytes per ion and cell; 4.62 ms with species packed within a chunk,
+// eleven 8-byte accesses per record and one corner x four moments per thread;
+// 5.35 ms with two particles per thread at 16 warps per SM.
 template <int PER, bool EXTRA>
-__global__ void __launch_bounds__(FT, 4)
+__global__ void __launch_bounds__(PD_T, 4)
 k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushParams pp, FastBufs fb,
                     double* cntd, unsigned long long* cntu, unsigned* err) {
    extern __shared__ __align__(16) unsigned char pdSmem[];
@@ -526,27 +523,31 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
    const int S = (int)blockIdx.x;
    const int nseg = fg.nseg;
    const int row = S / nseg, gseg = S - row * nseg;
-   const int uy = row % fg.nd[1], uz = row / fg.nd[1];
+   const int uz = row / fg.nd[1], uy = row - uz * fg.nd[1];
    const int u0 = gseg * SEG, u1 = min(u0 + SEG, fg.nd[0]);
    const int ns = FS.ns;
    const double dx = g.dx, hdx = 0.5 * dx;
    const int xs0 = dualB(u0, g.per[0]), ys0 = dualB(uy, g.per[1]), zs0 = dualB(uz, g.per[2]);
    // no obstacle cell within one step of the segment: the obstacle test is skipped
    const bool segInner = fb.segInner[S] != 0;
+   // every cell a particle of the segment can be in or reach has its neighbours in y and z
+   const bool yzIn = ((PER & 2) || (ys0 >= 2 && ys0 + 2 <= g.ny - 2)) && ((PER & 4) || (zs0 >= 2 && zs0 + 2 <= g.nz - 2));
 
-   // ---- set-up: species prefix (warp 0), segment pointers (warps 1-4), stencil rows (warps 5-6)
+   // ---- set-up: species (warp 0), segment pointers, stencil rows
    if (warp == 0) {
       const int cnt = lane < ns ? FS.st[lane].cur.cnt[S] : 0;
-      int x = cnt;
+      const int groups = (cnt + 31) >> 5;
+      int x = groups;
 #pragma unroll
       for (int o = 1; o < 16; o <<= 1) {
          const int y = __shfl_up_sync(0xffffffffu, x, o);
          if (lane >= o) x += y;
       }
-      if (lane <= ns) sh.prefix[lane] = x - cnt;
-      if (lane < FAST_MAX_SPECIES) sh.stay[lane] = 0;
-   } else if (tid < 32 + SEG_PTRS * ns) {
-      const int q = tid - 32, s = q / SEG_PTRS, k = q - s * SEG_PTRS;
+      if (lane <= ns) sh.first[lane] = x - groups;
+      if (lane < FAST_MAX_SPECIES) { sh.cnt[lane] = cnt; sh.stay[lane] = 0; }
+   }
+   for (int q = tid; q < SEG_PTRS * ns; q += PD_T) {
+      const int s = q / SEG_PTRS, k = q - s * SEG_PTRS;
       const SegSpecies& SS = FS.st[s];
       const long long b = SS.base[S];
       void* v;
@@ -555,8 +556,8 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
       else if (k == 14) v = SS.cur.lx + b;
       else v = SS.nxt.lx + b;
       sh.ptr[s][k] = v;
-   } else if (tid >= 160 && tid < 160 + SF_ROWS_B + SF_ROWS_C * (pp.use_ep ? 2 : 1)) {
-      const int r = tid - 160;
+   }
+   if (const int r = PD_T - 1 - tid; r < SF_ROWS_B + SF_ROWS_C * (pp.use_ep ? 2 : 1)) {
       int len, dxs, l, dy, dz;
       const double* arr;
       double* dst = stencilRow(sh.f, f, r, len, dxs, arr, l, dy, dz);
@@ -573,78 +574,85 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
       sh.rows[r] = sr;
    }
    __syncthreads();
-   const int total = sh.prefix[ns];
-   int lxNext = 0;
-   pdStage<PER>(g, f, pp.use_ep, sh, total, ns, lxNext);
+   const int groups = sh.first[ns];
+   int lxn = 0;
+   pdPrefetch(sh, 0, ns, lxn);
+   pdStage<PER>(g, f, pp.use_ep, sh);
+   cpAsyncCommit();
    cpAsyncWaitAll();
    __syncthreads();
 
-   const int myDual = tid >> 3, myCorner = tid & 7;   // this thread's sums: (dual cell, corner) x 4 moments
-   double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+   // this thread's sums: two corners of one dual cell, two moments (charge and Jx, or Jy and Jz)
+   const int myDual = tid >> 3, myPair = (tid >> 1) & 3, myHalf = tid & 1;
+   double a00 = 0.0, a01 = 0.0, a10 = 0.0, a11 = 0.0;
 
-   for (int c0 = 0; c0 < total; c0 += FT) {
-      const int i = c0 + tid;
-      const bool active = i < total;
-      int s = 0;
-      if (active)
-         while (s + 1 < ns && i >= sh.prefix[s + 1]) ++s;
+   for (int V0 = 0; V0 < groups; V0 += PD_VW) {
       double st[7];
-      bool stay = false, rec = false, leave = false, clamp = false;
-      int mflags = 0;
-      int vx = 0, vy = 0, vz = 0;
-      int p = 0;
-      const int lu = lxNext;
-      if (c0 > 0) cpAsyncWaitAll();   // this thread's copies of the chunk
-      if (active) {
-         p = i - sh.prefix[s];
+      int duv = 0, dyz = 0, mflags = 0, rrank = 0;
+      bool stay = false, rec = false, hx = false, hy = false, hz = false, clamp = false;
+      if (V0 > 0) cpAsyncWaitAll();   // this thread's copies of the chunk
+      const int V = V0 + warp;
+      const int s = pdSpecies(sh, V, ns);
+      const int p = (V - sh.first[s]) * 32 + lane;
+      if (p < sh.cnt[s]) {
 #pragma unroll
          for (int a = 0; a < 7; ++a) st[a] = sh.pf[a][tid];
-         const int hx = halfS(st[0], dx), hy = halfS(st[1], dx), hz = halfS(st[2], dx);
-         const int lc = lu + 1 - hx, ly = 1 - hy, lz = 1 - hz;
-         int ci = xs0 + lu + 1 - hx;
-         int cj = ys0 + ly;
-         int ck = zs0 + lz;
-         if (ci >= g.nx) ci -= g.nx;   // periodic axes: dual cell 0 holds the upper half of the last cell
-         if (cj >= g.ny) cj -= g.ny;
-         if (ck >= g.nz) ck -= g.nz;
-         clamp = pushStaged(g, sh.f, FS.sp[s], pp, ci, cj, ck, lc, ly, lz, st);
-         if (EXTRA) gridCountAtomic(f, GC_CELL_MAX_VI, g.N, cidx(g, ci, cj, ck), clamp);
-         if (isnan(st[0]) || isnan(st[1]) || isnan(st[2])) raiseError(err, RHGPU_DEVERR_NAN_PARTICLE);
+         const int lu = lxn;
+         const int gx = st[0] < hdx ? 0 : 1, gy = st[1] < hdx ? 0 : 1, gz = st[2] < hdx ? 0 : 1;
+         const int lc = lu + 1 - gx, ly = 1 - gy, lz = 1 - gz;
+         const int ci = xs0 + lc, cj = ys0 + ly, ck = zs0 + lz;   // not wrapped (periodic axes: up to n)
+         bool accelerate = FS.sp[s].accelerate && !pp.useIFT && ((PER & 1) || (unsigned)(ci - 1) < (unsigned)(g.nx - 2));
+         if (!yzIn)
+            accelerate = accelerate && ((PER & 2) || (unsigned)(cj - 1) < (unsigned)(g.ny - 2)) &&
+                         ((PER & 4) || (unsigned)(ck - 1) < (unsigned)(g.nz - 2));
+         const int wi = (PER & 1) && ci >= g.nx ? ci - g.nx : ci, wj = (PER & 2) && cj >= g.ny ? cj - g.ny : cj,
+                   wk = (PER & 4) && ck >= g.nz ? ck - g.nz : ck;
+         clamp = pushStaged(g, sh.f, FS.sp[s].qmideltT2, accelerate, pp, wi, wj, wk, lc, ly, lz, st);
+         if (EXTRA) gridCountAtomic(f, GC_CELL_MAX_VI, g.N, cidx(g, wi, wj, wk), clamp);
          int ox, oy, oz;
-         int bad = migrateAxis(st[0], ox, dx, g.dx_below);
-         bad |= migrateAxis(st[1], oy, dx, g.dx_below);
-         bad |= migrateAxis(st[2], oz, dx, g.dx_below);
-         int ti = ci + ox, tj = cj + oy, tk = ck + oz;
-         const bool inside = wrapc(ti, g.nx, g.per[0]) && wrapc(tj, g.ny, g.per[1]) && wrapc(tk, g.nz, g.per[2]);
-         if (bad || !inside) {
+         bool nan = false;
+         int bad = migrateAxisBits(st[0], ox, g, nan);
+         bad |= migrateAxisBits(st[1], oy, g, nan);
+         bad |= migrateAxisBits(st[2], oz, g, nan);
+         if (nan) raiseError(err, RHGPU_DEVERR_NAN_PARTICLE);
+         // target cell: inside the box, and with all its neighbours
+         const int ti = ci + ox, tj = cj + oy, tk = ck + oz;
+         bool inside = !bad && ((PER & 1) || (unsigned)ti < (unsigned)g.nx);
+         bool all = (PER & 1) || (unsigned)(ti - 1) < (unsigned)(g.nx - 2);
+         if (!yzIn) {
+            inside = inside && ((PER & 2) || (unsigned)tj < (unsigned)g.ny) && ((PER & 4) || (unsigned)tk < (unsigned)g.nz);
+            all = all && ((PER & 2) || (unsigned)(tj - 1) < (unsigned)(g.ny - 2)) &&
+                  ((PER & 4) || (unsigned)(tk - 1) < (unsigned)(g.nz - 2));
+         }
+         bool removed = !inside || !all;
+         if (removed) {
             const double ke = st[6] * (sq(st[3]) + sq(st[4]) + sq(st[5]));
             atomicAdd(&cntd[4 * s + 0], st[6]);
             atomicAdd(&cntd[4 * s + 1], ke);
-         } else {
-            vx = dualU(ti + halfS(st[0], dx) - 1, g.nx, g.per[0]);
-            vy = dualU(tj + halfS(st[1], dx) - 1, g.ny, g.per[1]);
-            vz = dualU(tk + halfS(st[2], dx) - 1, g.nz, g.per[2]);
-            const bool inSeg = vy == uy && vz == uz && vx >= u0 && vx < u1;
-            if (FS.sp[s].accumulate) {
-               if (inSeg) {
-                  rec = true;   // its CIC weights are formed just before the record is written
-               } else {
-                  mflags |= MOVER_DEPOSIT;   // deposited by k_fast_mover_deposit
-               }
+         }
+         if (inside) {
+            // the new dual cell relative to the segment's first, and to its row
+            hx = !(st[0] < hdx); hy = !(st[1] < hdx); hz = !(st[2] < hdx);
+            int du = lu + ox + (hx ? 1 : 0) - gx;
+            const int dy = oy + (hy ? 1 : 0) - gy, dz = oz + (hz ? 1 : 0) - gz;
+            if ((PER & 1) && nseg == 1) {
+               if (du < 0) du += fg.nd[0];
+               else if (du >= fg.nd[0]) du -= fg.nd[0];
             }
-            // boundary conditions of the step
-            bool removed = false;
-            if (!allNb(g, ti, tj, tk)) {
-               removed = true;
-               const double ke = st[6] * (sq(st[3]) + sq(st[4]) + sq(st[5]));
-               atomicAdd(&cntd[4 * s + 0], st[6]);
-               atomicAdd(&cntd[4 * s + 1], ke);
-            } else {
-               const unsigned cn = (unsigned)ti + (unsigned)g.nx * ((unsigned)tj + (unsigned)g.ny * (unsigned)tk);
-               if (segInner && (f.flags[cn] & RHGPU_FLAG_INNER_PARTICLE)) {
-                  const double xp = blockOrigin(g.x_min, ti, dx) + st[0];
-                  const double yp = blockOrigin(g.y_min, tj, dx) + st[1];
-                  const double zp = blockOrigin(g.z_min, tk, dx) + st[2];
+            const bool inSeg = dy == 0 && dz == 0 && (unsigned)du < (unsigned)(u1 - u0);
+            duv = du;
+            dyz = (dy + 2) | ((dz + 2) << 3);
+            if (FS.sp[s].accumulate) {
+               rec = inSeg;   // its CIC weights are formed just before the record is written
+               if (!inSeg) mflags = MOVER_DEPOSIT;   // deposited by k_mover_pass
+            }
+            if (segInner && !removed) {
+               int xi = ti, xj = tj, xk = tk;
+               wrapc(xi, g.nx, g.per[0]); wrapc(xj, g.ny, g.per[1]); wrapc(xk, g.nz, g.per[2]);
+               if (f.flags[cidx(g, xi, xj, xk)] & RHGPU_FLAG_INNER_PARTICLE) {
+                  const double xp = blockOrigin(g.x_min, xi, dx) + st[0];
+                  const double yp = blockOrigin(g.y_min, xj, dx) + st[1];
+                  const double zp = blockOrigin(g.z_min, xk, dx) + st[2];
                   if (sq(xp) + sq(yp) + sq(zp) < FS.sp[s].R2obs) {
                      removed = true;
                      const double ke = st[6] * (sq(st[3]) + sq(st[4]) + sq(st[5]));
@@ -659,133 +667,119 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
             } else if (EXTRA && rec && pp.avgList) {
                mflags |= MOVER_AVG;   // population averages: its in-segment deposit is listed
             }
-            leave = mflags != 0;
          }
       }
       if (clamp) atomicAdd(&cntu[CNT_SPECIES_MAXVI + s], 1ull);
-
-      // ---- order of the chunk's stayers and records --------------------------------------
-      // warp-local first: stayer/record ballots and the records per (warp, dual cell)
-      const unsigned bs = __ballot_sync(0xffffffffu, stay), br = __ballot_sync(0xffffffffu, rec);
-      if (lane == 0) sh.wcnt[warp] = __popc(bs);
+      // order of the group's stayers and records: ballots, and its records per dual cell
+      const unsigned bs = __ballot_sync(0xffffffffu, stay);
+      const unsigned br = __ballot_sync(0xffffffffu, rec);
+      if (lane == 0) {
+         const int n = __popc(bs);
+         sh.wcnt[warp] = n;
+         if (n) atomicAdd(&sh.stay[s], n);
+      }
       sh.wd[lane][warp] = 0;
       __syncwarp();
-      const int rd = rec ? vx - u0 : 0;
-      int rrank = 0;
       if (rec) {
-         const unsigned mm = __match_any_sync(br, rd);
+         const unsigned mm = __match_any_sync(br, duv);
          rrank = __popc(mm & below);
-         if (rrank == 0) sh.wd[rd][warp] = (unsigned char)__popc(mm);
+         if (rrank == 0) sh.wd[duv][warp] = (unsigned char)__popc(mm);
       }
       __syncthreads();
       // every shared-memory read of this chunk's particles is done: request the next chunk's
-      {
-         const int i2 = i + FT;
-         if (i2 < total) {
-            int s2 = s;
-            while (s2 + 1 < ns && i2 >= sh.prefix[s2 + 1]) ++s2;
-            const int p2 = i2 - sh.prefix[s2];
-#pragma unroll
-            for (int a = 0; a < 7; ++a) cpAsync8(&sh.pf[a][tid], (const double*)sh.ptr[s2][a] + p2, 8);
-            lxNext = ((const unsigned char*)sh.ptr[s2][14])[p2];
-         }
-         cpAsyncCommit();
-      }
+      if (V0 + PD_VW < groups) pdPrefetch(sh, V0 + PD_VW, ns, lxn);
       // every warp, per dual cell (lane): the first sorted record of the dual cell
-      // (bin) and of this warp's records for it (off)
-      int binD, offD, nrec;
+      // (bin); the group counts of dual cell `lane` are bytes (each at most 32),
+      // byte sums by one multiply per 32-bit half
+      const uint2 c8 = *reinterpret_cast<const uint2*>(&sh.wd[lane][0]);
+      int binD, nrec;
       {
-         // the eight per-warp counts of dual cell `lane` are bytes (each at most 32):
-         // byte sums by one multiply per 32-bit half
-         const uint2 c8 = *reinterpret_cast<const uint2*>(&sh.wd[lane][0]);
          const int t = (int)(((c8.x * 0x01010101u) >> 24) + ((c8.y * 0x01010101u) >> 24));
-         const unsigned mlo = warp >= 4 ? 0xffffffffu : (1u << (8 * warp)) - 1u;
-         const unsigned mhi = warp <= 4 ? 0u : (1u << (8 * (warp - 4))) - 1u;
-         const int before = (int)((((c8.x & mlo) * 0x01010101u) >> 24) + (((c8.y & mhi) * 0x01010101u) >> 24));
          int x = t;
          for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
          }
          binD = x - t;
-         offD = binD + before;
          nrec = __shfl_sync(0xffffffffu, x, 31);
       }
-      const int recPos = __shfl_sync(0xffffffffu, offD, rd) + rrank;
       const int sumLo = __shfl_sync(0xffffffffu, binD, myDual);
       const int sumHiN = __shfl_sync(0xffffffffu, binD, (myDual + 1) & 31);
       const int sumHi = myDual == SEG - 1 ? nrec : sumHiN;
-      // stayers of the chunk before this position (and in all), and this species' count so far
-      const int wc = lane < FW ? sh.wcnt[lane] : 0;
-      const int myRank = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < warp ? wc : 0)) + __popc(bs & below);
-      const int chunkStay = (int)__reduce_add_sync(0xffffffffu, (unsigned)wc);
-      sh.rank[tid] = myRank;
-      const int stayBase = stay ? sh.stay[s] : 0;
+      const int wc = lane < PD_VW ? sh.wcnt[lane] : 0;
+      // this group's records start after those of the groups before it, per dual cell
+      const unsigned mlo = warp >= 4 ? 0xffffffffu : (1u << (8 * warp)) - 1u;
+      const unsigned mhi = warp <= 4 ? 0u : (1u << (8 * (warp - 4))) - 1u;
+      const int before = (int)((((c8.x & mlo) * 0x01010101u) >> 24) + (((c8.y & mhi) * 0x01010101u) >> 24));
+      const int recPos = __shfl_sync(0xffffffffu, binD + before, rec ? duv : 0) + rrank;
+      // next slot of a stayer: the species' stayers up to and with the chunk less those from this group on
+      const int vEnd = sh.first[s + 1] - V0;
+      const int from = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane >= warp && lane < vEnd ? wc : 0));
+      const int slot = sh.stay[s] - from + __popc(bs & below);
       // mover slots reserved now, written after the sums
-      const unsigned lm = __ballot_sync(0xffffffffu, leave);
-      const int leader = lm ? __ffs(lm) - 1 : 0;
+      const unsigned lm = __ballot_sync(0xffffffffu, mflags != 0);
       unsigned long long mb = 0;
-      if (lm && lane == leader) mb = atomicAdd(fb.nmovers, (unsigned long long)__popc(lm));
+      if (lm && lane == __ffs(lm) - 1) mb = atomicAdd(fb.nmovers, (unsigned long long)__popc(lm));
       if (rec) {
          double w8[8];
-         cicWeightsHalf(st[0], st[1], st[2], st[6] * FS.sp[s].q, g, hdx, w8);
-         double* r = sh.rec + recPos * REC;
+         cicWeightsHalf(st[0], st[1], st[2], hx, hy, hz, st[6] * FS.sp[s].q, g, hdx, w8);
+         double2* const r = reinterpret_cast<double2*>(sh.rec + recPos * PD_REC);
 #pragma unroll
-         for (int o = 0; o < 8; ++o) r[o] = w8[o];
-         r[8] = st[3]; r[9] = st[4]; r[10] = st[5];
+         for (int o = 0; o < 4; ++o) r[o] = make_double2(w8[2 * o], w8[2 * o + 1]);
+         r[4] = make_double2(1.0, st[3]);
+         r[5] = make_double2(st[4], st[5]);
       }
       __syncthreads();
       if (stay) {
-         const int p0 = sh.prefix[s] - c0;   // chunk position of the species' first particle
-         const int q = stayBase + myRank - (p0 > 0 ? sh.rank[p0] : 0);
          double* const* nx = (double* const*)&sh.ptr[s][7];
 #pragma unroll
-         for (int a = 0; a < 7; ++a) nx[a][q] = st[a];
-         ((unsigned char*)sh.ptr[s][15])[q] = (unsigned char)(vx - u0);
+         for (int a = 0; a < 7; ++a) nx[a][slot] = st[a];
+         ((unsigned char*)sh.ptr[s][15])[slot] = (unsigned char)duv;
       }
-      // running stayer count of each species
-      if (tid < ns) {
-         const int lo = min(max(sh.prefix[tid] - c0, 0), FT), hi = min(max(sh.prefix[tid + 1] - c0, 0), FT);
-         const int rlo = lo < FT ? sh.rank[lo] : chunkStay, rhi = hi < FT ? sh.rank[hi] : chunkStay;
-         sh.stay[tid] += rhi - rlo;
-      }
-      // ---- sums of this thread's (dual cell, corner), records in list order ----------------
+      // ---- this thread's sums, records in list order ----------------------------------------
 #pragma unroll 2
       for (int r = sumLo; r < sumHi; ++r) {
-         const double* rr = sh.rec + r * REC;
-         const double w = rr[myCorner];
-         a0 += w;
-         a1 += w * rr[8];
-         a2 += w * rr[9];
-         a3 += w * rr[10];
+         const double2* const rr = reinterpret_cast<const double2*>(sh.rec + r * PD_REC);
+         const double2 w = rr[myPair], u = rr[4 + myHalf];
+         a00 += w.x * u.x;
+         a01 += w.x * u.y;
+         a10 += w.y * u.x;
+         a11 += w.y * u.y;
       }
       // ---- particles that left the segment -----------------------------------------------
-      if (lm) {
-         mb = __shfl_sync(0xffffffffu, mb, leader);
-         if (leave) {
-            const unsigned long long m = mb + __popc(lm & below);
-            if ((long long)m < fb.moverCap) {
-               Mover& M = fb.movers[m];
-#pragma unroll
-               for (int a = 0; a < 7; ++a) M.s[a] = st[a];
-               M.key = ((unsigned long long)S << 32) | (unsigned long long)p;
-               const int gd = vx / SEG;
-               M.dest = ((long long)vy + (long long)fg.nd[1] * vz) * nseg + gd;
-               M.species = s;
-               M.lx = (vx - gd * SEG) | mflags;
-            } else {
-               raiseError(err, RHGPU_DEVERR_CAPACITY);
-            }
-         }
+      if (!lm) continue;
+      const unsigned long long m0 = __shfl_sync(0xffffffffu, mb, __ffs(lm) - 1);
+      if (!mflags) continue;
+      const unsigned long long m = m0 + __popc(lm & below);
+      if ((long long)m >= fb.moverCap) {
+         raiseError(err, RHGPU_DEVERR_CAPACITY);
+         continue;
       }
-      // no barrier here: the next chunk's first barrier orders the reads of rec,
-      // rank and stay before their next writes
+      int vx = u0 + duv, vy = uy + (dyz & 7) - 2, vz = uz + (dyz >> 3) - 2;
+      if (PER & 1) wrapc(vx, fg.nd[0], 1);
+      if (PER & 2) wrapc(vy, fg.nd[1], 1);
+      if (PER & 4) wrapc(vz, fg.nd[2], 1);
+      Mover& M = fb.movers[m];
+#pragma unroll
+      for (int a = 0; a < 7; ++a) M.s[a] = st[a];
+      M.key = ((unsigned long long)S << 32) | (unsigned long long)p;
+      const int gd = vx / SEG;
+      M.dest = ((long long)vy + (long long)fg.nd[1] * vz) * nseg + gd;
+      M.species = s;
+      M.lx = (vx - gd * SEG) | mflags;
+      // no barrier here: the next chunk's first barrier orders the reads of rec
+      // and wd before their next writes
    }
 
    // ---- outputs: stayer counts, row partials, segment-boundary partial ---------------------
    __syncthreads();
    if (tid < ns) FS.st[tid].nxt.cnt[S] = sh.stay[tid];
-   segPartialsOut(g, fg, fb, sh.rec, row, gseg, u0, u1, a0, a1, a2, a3);
+   {
+      double* const q = sh.rec + myDual * 32 + myPair * 8 + myHalf * 2;
+      q[0] = a00; q[1] = a01; q[4] = a10; q[5] = a11;
+   }
+   __syncthreads();
+   segPartialsOut<PD_T>(g, fg, fb.RP, fb.RPB, sh.rec, row, gseg, u0, u1);
 }
 
 // corner o's four deposits (charge, current) of one mover: the weight products

@@ -355,10 +355,10 @@ int f32Push(rhgpu_ctx* c) {
 #define RH_F32_PD(M)                                                                                            \
    case M:                                                                                                        \
       if (c->f.gc)                                                                                                \
-         k_f32_push_deposit<M, true><<<(unsigned)NS, FT, 0, c->stream>>>(c->g, c->f, c->fg, FS, FP, c->f32b, c->cntD,  \
+         k_f32_push_deposit<M, true><<<(unsigned)NS, PD_T, 0, c->stream>>>(c->g, c->f, c->fg, FS, FP, c->f32b, c->cntD,  \
                                                                          c->cntU, c->err);                         \
       else                                                                                                        \
-         k_f32_push_deposit<M, false><<<(unsigned)NS, FT, 0, c->stream>>>(c->g, c->f, c->fg, FS, FP, c->f32b,          \
+         k_f32_push_deposit<M, false><<<(unsigned)NS, PD_T, 0, c->stream>>>(c->g, c->f, c->fg, FS, FP, c->f32b,          \
                                                                           c->cntD, c->cntU, c->err);               \
       break;
          RH_F32_PD(0) RH_F32_PD(1) RH_F32_PD(2) RH_F32_PD(3) RH_F32_PD(4) RH_F32_PD(5) RH_F32_PD(6) RH_F32_PD(7)

@@ -540,7 +540,7 @@ int launchPushDeposit(rhgpu_ctx* c, const FastSpecies& FS, const PushParams& pp)
                                    (int)PUSH_DEPOSIT_SMEM));
       raised[dev] = true;
    }
-   k_fast_push_deposit<PER, EXTRA><<<(unsigned)c->fg.NS, FT, PUSH_DEPOSIT_SMEM, c->stream>>>(
+   k_fast_push_deposit<PER, EXTRA><<<(unsigned)c->fg.NS, PD_T, PUSH_DEPOSIT_SMEM, c->stream>>>(
        c->g, c->f, c->fg, FS, pp, c->fb, c->cntD, c->cntU, c->err);
    return RHGPU_OK;
 }
