@@ -4,9 +4,12 @@
 
 namespace rh {
 
-__global__ void k_dn_bimage(const float* W, __nv_bfloat16* img, int transposed) {
+__global__ void k_dn_bimage(const float* params, __nv_bfloat16* images) {
    const int e = blockIdx.x * blockDim.x + threadIdx.x;   // (q, n, k)
    if (e >= 9 * TC_NB * DN_C) return;
+   const int layer = blockIdx.y % 3, transposed = blockIdx.y / 3;
+   const float* const W = params + (size_t)layer * DN_LAYER;
+   __nv_bfloat16* const img = images + (size_t)blockIdx.y * (TC_BIMG / 2);
    const int k = e % DN_C, n = (e / DN_C) % TC_NB, q = e / (DN_C * TC_NB);
    const int b = n / DN_C, c = n % DN_C;
    const int sx = q % 3 - 1, sy = q / 3 - 1;
@@ -16,74 +19,125 @@ __global__ void k_dn_bimage(const float* W, __nv_bfloat16* img, int transposed) 
    img[q * (TC_QIMG / 2) + (k / 8) * (TC_NB * 8) + (n / 8) * 64 + (n % 8) * 8 + (k % 8)] = __float2bfloat16_rn(w);
 }
 
-__global__ void __launch_bounds__(32 * DN_WARPS)
-k_dn_wgrad(DnGrid g, const unsigned* X, const unsigned* dY, float* part) {
-   __shared__ float sacc[DN_WARPS][DN_C * DN_C];
-   const unsigned short* x16 = reinterpret_cast<const unsigned short*>(X);
-   const unsigned short* y16 = reinterpret_cast<const unsigned short*>(dY);
-   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   const int gq = lane >> 2, q = lane & 3;
-   const int t = blockIdx.y;
-   float c[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-   const long long vw = (long long)blockIdx.x * DN_WGRAD_VOX + warp * (DN_WGRAD_VOX / DN_WARPS);
-   auto yv = [&](long long v, int ch) -> unsigned { return (v < g.N) ? (unsigned)y16[v * DN_C + ch] : 0u; };
-   for (int ks = 0; ks < DN_WGRAD_VOX / DN_WARPS; ks += 16) {
-      const long long vk = vw + ks;
-      if (vk >= g.N) break;
-      // the input voxels (at tap t) of this thread's four k indices
-      const int n0 = dnNb(g, dnDecode(g, vk + 2 * q), t, 1), n1 = dnNb(g, dnDecode(g, vk + 2 * q + 1), t, 1);
-      const int n8 = dnNb(g, dnDecode(g, vk + 2 * q + 8), t, 1), n9 = dnNb(g, dnDecode(g, vk + 2 * q + 9), t, 1);
-      auto xv = [&](int n, int ch) -> unsigned { return n >= 0 ? (unsigned)x16[(long long)n * DN_C + ch] : 0u; };
-      unsigned a[4];
-      a[0] = xv(n0, gq) | (xv(n1, gq) << 16);
-      a[1] = xv(n0, gq + 8) | (xv(n1, gq + 8) << 16);
-      a[2] = xv(n8, gq) | (xv(n9, gq) << 16);
-      a[3] = xv(n8, gq + 8) | (xv(n9, gq + 8) << 16);
-      for (int nt = 0; nt < 2; ++nt) {
-         const int co = nt * 8 + gq;
-         const unsigned b0 = yv(vk + 2 * q, co) | (yv(vk + 2 * q + 1, co) << 16);
-         const unsigned b1 = yv(vk + 2 * q + 8, co) | (yv(vk + 2 * q + 9, co) << 16);
-         mma16816(c[nt], a, b0, b1);
-      }
-   }
-   // c[nt][0,1]: ci = gq, co = nt*8 + 2q, +1; c[nt][2,3]: ci = gq + 8
-   for (int nt = 0; nt < 2; ++nt) {
-      const int co = nt * 8 + 2 * q;
-      sacc[warp][gq * DN_C + co] = c[nt][0];
-      sacc[warp][gq * DN_C + co + 1] = c[nt][1];
-      sacc[warp][(gq + 8) * DN_C + co] = c[nt][2];
-      sacc[warp][(gq + 8) * DN_C + co + 1] = c[nt][3];
-   }
-   __syncthreads();
-   for (int e = threadIdx.x; e < DN_C * DN_C; e += blockDim.x) {
-      float a = 0.f;
-      for (int w = 0; w < DN_WARPS; ++w) a += sacc[w][e];
-      part[((long long)blockIdx.x * DN_TAPS + t) * DN_C * DN_C + e] = a;
-   }
+// four 8 x 8 BF16 matrices transposed out of shared memory
+__device__ __forceinline__ void ldmatrixT(unsigned r[4], unsigned addr) {
+   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                : "r"(addr)
+                : "memory");
 }
 
-__global__ void k_dn_bgrad(DnGrid g, const unsigned* dY, float* part) {
-   __shared__ float s[256][DN_C];
-   const unsigned short* y16 = reinterpret_cast<const unsigned short*>(dY);
-   float a[DN_C];
-   for (int c = 0; c < DN_C; ++c) a[c] = 0.f;
-   for (long long v = (long long)blockIdx.x * DN_WGRAD_VOX + threadIdx.x;
-        v < min(g.N, (long long)(blockIdx.x + 1) * DN_WGRAD_VOX); v += blockDim.x)
-      for (int c = 0; c < DN_C; ++c) a[c] += __bfloat162float(__ushort_as_bfloat16(y16[v * DN_C + c]));
-   for (int c = 0; c < DN_C; ++c) s[threadIdx.x][c] = a[c];
-   __syncthreads();
-   if (threadIdx.x < DN_C) {
-      float t = 0.f;
-      for (int r = 0; r < (int)blockDim.x; ++r) t += s[r][threadIdx.x];
-      part[(long long)blockIdx.x * DN_C + threadIdx.x] = t;
+__global__ void __launch_bounds__(32 * DN_WARPS)
+k_dn_wgrad(DnGrid g, const unsigned* X, const unsigned* dY, float* part) {
+   constexpr int ROW = 48;   // bytes of a staged voxel (32 used): eight rows on different banks
+   __shared__ alignas(16) unsigned char tile[DN_WARPS][4][16 * ROW];   // per warp: dY and X at three taps, 16 voxels
+   __shared__ float sacc[DN_WARPS][DN_C * DN_C];
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+   float* const out = part + (long long)blockIdx.x * DN_LAYER;
+   if (blockIdx.y == DN_WGRAD_ROWS) {   // bias: sums of dY over the block's voxels, 256 strided partial sums added in order
+      __shared__ float s[256][DN_C];
+      for (int r = threadIdx.x; r < 256; r += 32 * DN_WARPS) {
+         float a[DN_C];
+         for (int c = 0; c < DN_C; ++c) a[c] = 0.f;
+         for (long long v = (long long)blockIdx.x * DN_WGRAD_VOX + r;
+              v < min(g.N, (long long)(blockIdx.x + 1) * DN_WGRAD_VOX); v += 256) {
+            const uint4* const y = reinterpret_cast<const uint4*>(dY) + 2 * v;
+            const uint4 y0 = y[0], y1 = y[1];
+            const unsigned w[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+#pragma unroll
+            for (int c = 0; c < 8; ++c) { a[2 * c] += bf16lo(w[c]); a[2 * c + 1] += bf16hi(w[c]); }
+         }
+         for (int c = 0; c < DN_C; ++c) s[r][c] = a[c];
+      }
+      __syncthreads();
+      if (threadIdx.x < DN_C) {
+         float t = 0.f;
+#pragma unroll 16
+         for (int r = 0; r < 256; ++r) t += s[r][threadIdx.x];
+         out[DN_TAPS * DN_C * DN_C + threadIdx.x] = t;
+      }
+      return;
+   }
+   const int dy = (int)blockIdx.y % 3 - 1, dz = (int)blockIdx.y / 3 - 1;
+   float c[3][2][4] = {};
+   const long long vw = (long long)blockIdx.x * DN_WGRAD_VOX + warp * (DN_WGRAD_VOX / DN_WARPS);
+   // a lane stages half a voxel (16 bytes) of dY and of X at the three taps of the row
+   const int sv = lane >> 1, sh = lane & 1;
+   const uint4* const X4 = reinterpret_cast<const uint4*>(X);
+   const uint4* const Y4 = reinterpret_cast<const uint4*>(dY);
+   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+   auto fetch = [&](long long vk, uint4 r[4]) {
+      const long long v = vk + sv;
+      r[0] = r[1] = r[2] = r[3] = zero;
+      if (v >= g.N) return;
+      r[0] = Y4[2 * v + sh];
+      const DnPos p = dnDecode(g, v);
+      const int j = dnWrap(p.j + dy, g.ny, g.per[1]), k = dnWrap(p.k + dz, g.nz, g.per[2]);
+      if (j < 0 || k < 0) return;
+      const long long row = (long long)g.nx * (j + (long long)g.ny * k);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+         const int i = dnWrap(p.i + t - 1, g.nx, g.per[0]);
+         if (i >= 0) r[1 + t] = X4[2 * (row + i) + sh];
+      }
+   };
+   const unsigned base = (unsigned)__cvta_generic_to_shared(&tile[warp][0][0]);
+   // ldmatrix rows: matrix lane / 8 holds voxels 8 (m / 2) .. + 7, channels 8 (m % 2) .. + 7
+   const unsigned mrow = base + (unsigned)(((lane >> 4) * 8 + (lane & 7)) * ROW + ((lane >> 3) & 1) * 16);
+   uint4 r[4];
+   fetch(vw, r);
+   for (int ks = 0; ks < DN_WGRAD_VOX / DN_WARPS; ks += 16) {
+      if (vw + ks >= g.N) break;
+      __syncwarp();
+#pragma unroll
+      for (int m = 0; m < 4; ++m) *reinterpret_cast<uint4*>(&tile[warp][m][sv * ROW + sh * 16]) = r[m];
+      __syncwarp();
+      if (ks + 16 < DN_WGRAD_VOX / DN_WARPS) fetch(vw + ks + 16, r);
+      unsigned b[4];
+      ldmatrixT(b, mrow);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+         unsigned a[4];
+         ldmatrixT(a, mrow + (unsigned)((1 + t) * 16 * ROW));
+         mma16816(c[t][0], a, b[0], b[2]);
+         mma16816(c[t][1], a, b[1], b[3]);
+      }
+   }
+   // c[t][nt][0,1]: ci = gq, co = nt*8 + 2q, +1; c[t][nt][2,3]: ci = gq + 8
+   const int gq = lane >> 2, q = lane & 3;
+#pragma unroll
+   for (int t = 0; t < 3; ++t) {
+      __syncthreads();
+      for (int nt = 0; nt < 2; ++nt) {
+         const int co = nt * 8 + 2 * q;
+         sacc[warp][gq * DN_C + co] = c[t][nt][0];
+         sacc[warp][gq * DN_C + co + 1] = c[t][nt][1];
+         sacc[warp][(gq + 8) * DN_C + co] = c[t][nt][2];
+         sacc[warp][(gq + 8) * DN_C + co + 1] = c[t][nt][3];
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < DN_C * DN_C; e += blockDim.x) {
+         float a = 0.f;
+         for (int w = 0; w < DN_WARPS; ++w) a += sacc[w][e];
+         out[(3 * blockIdx.y + t) * DN_C * DN_C + e] = a;
+      }
    }
 }
 
 __global__ void k_dn_reduce_rows(const float* part, long long rows, int n, float* out) {
    const int e = blockIdx.x * blockDim.x + threadIdx.x;
    if (e >= n) return;
+   constexpr int B = 16;   // rows in flight
    float a = 0.f;
-   for (long long r = 0; r < rows; ++r) a += part[r * n + e];
+   long long r = 0;
+   for (; r + B <= rows; r += B) {
+      float v[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) v[u] = part[(r + u) * n + e];
+#pragma unroll
+      for (int u = 0; u < B; ++u) a += v[u];
+   }
+   for (; r < rows; ++r) a += part[r * n + e];
    out[e] = a;
 }
 
@@ -129,7 +183,16 @@ __global__ void k_dn_norm(long long N, const double* rho, const double* J, doubl
    if (v >= N) return;
    const double fj = dnJFactor(vel, rsj, rho[v]);
    out[v * 4] = (float)(rho[v] * rsr);
-   for (int l = 0; l < 3; ++l) out[v * 4 + 1 + l] = (float)(J[l * N + v] * fj);
+   for (int l = 0; l < 3; ++l) out[v * 4 + 1 + l] = (float)(J[3 * v + l] * fj);
+}
+
+__global__ void k_dn_planar(long long N, const double* in, double* out, int back) {
+   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+   if (t >= 3 * N) return;
+   const long long n = t / 3;
+   const long long p = (t - 3 * n) * N + n;
+   if (back) out[t] = in[p];
+   else out[p] = in[t];
 }
 
 __global__ void k_dn_res_to_act(long long N, const float* res, unsigned* act) {

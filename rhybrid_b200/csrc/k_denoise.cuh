@@ -178,7 +178,8 @@ static_assert(TC_PLANE % 16 == 0 && TC_QIMG % 16 == 0, "descriptor strides are m
 // input slice z' to output slice z' - 1 + b: forward the tap (sx, sy, 1 - b)
 // with B(n, k) = W[t][k][n % 16]; the data gradient the tap (-sx, -sy, b - 1)
 // with B(n, k) = W[t][n % 16][k]. Tap t = (dx + 1) + 3 (dy + 1) + 9 (dz + 1).
-__global__ void k_dn_bimage(const float* W, __nv_bfloat16* img, int transposed);
+// blockIdx.y: the layer, + 3 for the transposed image; images one after another.
+__global__ void k_dn_bimage(const float* params, __nv_bfloat16* images);
 
 __device__ __forceinline__ unsigned long long umma_desc(unsigned addr, unsigned lbo, unsigned sbo) {
    // start >> 4 [0,14), LBO >> 4 [16,30), SBO >> 4 [32,46), version 1 [46,48), no swizzle
@@ -464,15 +465,21 @@ k_dn_conv_tc(DnGrid g, const unsigned* in, const __nv_bfloat16* bimg, const floa
    }
 }
 
-// Weight gradient of one layer: dW[t][ci][co] = sum_v X[nb(v,t)][ci] dY[v][co].
-// Block (blockIdx.x, tap blockIdx.y) covers DN_WGRAD_VOX voxels, each warp a
-// quarter in k-steps of 16 voxels: C[ci][co] += A[ci][vox] B[vox][co] (mma),
-// then the 4 warps are added in order and the block's partial row written.
+// Weight and bias gradients of one layer: dW[t][ci][co] = sum_v X[nb(v,t)][ci]
+// dY[v][co], db[co] = sum_v dY[v][co]. Block blockIdx.x covers DN_WGRAD_VOX
+// voxels, blockIdx.y the three taps of one (dy, dz) (or, last, the bias), each
+// warp a quarter of the voxels in k-steps of 16: C[ci][co] += A[ci][vox]
+// B[vox][co] (mma), then the 4 warps are added in order and the block's part of
+// its partial row (DN_LAYER values) written. A warp stages a k-step's voxels as
+// 16-byte halves in shared memory, where ldmatrix transposes them into operands;
+// the next k-step's are loaded meanwhile. 52 us for 64^3 voxels; bound by the
+// L2 reads of X, three times per row of taps. A training iteration at 64^3, with
+// one tap per block, 2-byte operand loads, the partial rows added one load after
+// another, 21 launches and a read-back: 0.98 ms; with this, rows added 16 loads at
+// a time, 14 launches and the losses read every 64 iterations: 0.40 ms.
+constexpr int DN_WGRAD_ROWS = 9;   // (dy, dz) pairs
 __global__ void __launch_bounds__(32 * DN_WARPS)
 k_dn_wgrad(DnGrid g, const unsigned* X, const unsigned* dY, float* part);
-
-// bias gradient partials: sum over the block's voxels of dY[v][co]
-__global__ void k_dn_bgrad(DnGrid g, const unsigned* dY, float* part);
 
 // sum of the block partials in block order -> grad (n values per row)
 __global__ void k_dn_reduce_rows(const float* part, long long rows, int n, float* out);
@@ -488,10 +495,13 @@ __global__ void k_dn_loss(DnGrid g, const float* pred, const float* target, doub
 __global__ void k_dn_adam(float* p, const float* gr, float* m, float* v, const unsigned char* mask, int n, float lr,
                           float b1, float b2, float eps, float c1, float c2);
 
-// normalized FP32 copy (N x 4) of planar FP64 moments: rho / sr and J / sj as
+// normalized FP32 copy (N x 4) of FP64 moments, J interleaved (3 per cell): rho / sr and J / sj as
 // products with the reciprocals rsr = 1 / sr, rsj = 1 / sj (velocity form:
 // J / (sj rho), dnJFactor)
 __global__ void k_dn_norm(long long N, const double* rho, const double* J, double rsr, double rsj, int vel, float* out);
+
+// a 3-vector per cell from interleaved to planes, or (back) from planes to interleaved
+__global__ void k_dn_planar(long long N, const double* in, double* out, int back);
 
 // FP32 normalized moments (N x 4) -> BF16 network input (16 channels)
 __global__ void k_dn_res_to_act(long long N, const float* res, unsigned* act);

@@ -6,13 +6,11 @@
 namespace rhh {
 
 const int DN_LOSS_BLOCKS = 296;
+const int DN_LOSS_RING = 64;   // training iterations whose loss partials wait on the device
 
 // the UMMA B images of every layer (forward and transposed) from the FP32 parameters
 int dnRebuildImages(rhgpu_dn* d) {
-   for (int l = 0; l < 3; ++l)
-      for (int tr = 0; tr < 2; ++tr)
-         k_dn_bimage<<<(DN_TAPS * DN_C * DN_C + 255) / 256, 256, 0, d->stream>>>(
-             d->params + (size_t)l * DN_LAYER, d->bimg + (size_t)(3 * tr + l) * (TC_BIMG / 2), tr);
+   k_dn_bimage<<<dim3((DN_TAPS * DN_C * DN_C + 255) / 256, 6), 256, 0, d->stream>>>(d->params, d->bimg);
    RH_CUDA(cudaGetLastError());
    return RHGPU_OK;
 }
@@ -51,61 +49,58 @@ int dnCheckError(rhgpu_dn* d) {
    return RHGPU_OK;
 }
 
-// forward of the network on d->res (normalized FP32 input) into d->out32
-int dnForward(rhgpu_dn* d) {
+// forward of the network on res (normalized FP32 input) into d->out32
+int dnForward(rhgpu_dn* d, const float* res) {
    const long long N = d->g.N;
-   k_dn_res_to_act<<<blocks1d(N, 256), 256, 0, d->stream>>>(N, d->res, d->act[0]);
+   k_dn_res_to_act<<<blocks1d(N, 256), 256, 0, d->stream>>>(N, res, d->act[0]);
    const float* b0 = d->params + DN_TAPS * DN_C * DN_C;
    const float* b1 = d->params + DN_LAYER + DN_TAPS * DN_C * DN_C;
    const float* b2 = d->params + 2 * DN_LAYER + DN_TAPS * DN_C * DN_C;
    int rc = dnConv(d, d->stream, false, 0, d->act[0], b0, 0, d->act[1], nullptr, nullptr, nullptr, DnMoments{}, d->err);
    if (!rc) rc = dnConv(d, d->stream, false, 1, d->act[1], b1, 0, d->act[2], nullptr, nullptr, nullptr, DnMoments{}, d->err);
-   if (!rc) rc = dnConv(d, d->stream, false, 2, d->act[2], b2, 3, nullptr, nullptr, d->out32, d->res, DnMoments{}, d->err);
+   if (!rc) rc = dnConv(d, d->stream, false, 2, d->act[2], b2, 3, nullptr, nullptr, d->out32, res, DnMoments{}, d->err);
    return rc;
 }
 
-// loss against target (normalized FP32, N x 4) and the gradient of all parameters into d->grad
-int dnBackward(rhgpu_dn* d, const float* target, double* loss) {
-   const long long N = d->g.N;
-   // voxels in the loss: all but the masked border of the non-periodic faces
+// voxels in the loss: all but the masked border of the non-periodic faces
+long long dnLossVoxels(const rhgpu_dn* d) {
    long long in = 1;
    const int nn[3] = {d->g.nx, d->g.ny, d->g.nz};
    for (int a = 0; a < 3; ++a) in *= d->g.per[a] ? nn[a] : std::max(0, nn[a] - 2 * d->border);
+   return in;
+}
+
+// the loss from the partial sums of k_dn_loss, added in block order
+double dnLossOf(const rhgpu_dn* d, const double* part) {
+   double a = 0.0;
+   for (int b = 0; b < DN_LOSS_BLOCKS; ++b) a += part[b];
+   return a / (4.0 * (double)dnLossVoxels(d));
+}
+
+// loss partials against target (normalized FP32, N x 4) into lossPart and the gradient of all parameters into d->grad
+int dnBackward(rhgpu_dn* d, const float* target, double* lossPart) {
+   const long long in = dnLossVoxels(d);
    if (in < 1) return fail(RHGPU_ERR_STATE, "dn_train: the loss border leaves no voxel");
-   k_dn_loss<<<DN_LOSS_BLOCKS, 256, 0, d->stream>>>(d->g, d->out32, target, 1.0 / (4.0 * (double)in), d->dY[2], d->lossPart,
+   k_dn_loss<<<DN_LOSS_BLOCKS, 256, 0, d->stream>>>(d->g, d->out32, target, 1.0 / (4.0 * (double)in), d->dY[2], lossPart,
                                                    d->border);
-   const unsigned wb = (unsigned)((N + DN_WGRAD_VOX - 1) / DN_WGRAD_VOX);
+   const unsigned wb = (unsigned)d->partRows;
    for (int l = 2; l >= 0; --l) {
-      k_dn_wgrad<<<dim3(wb, DN_TAPS), 32 * DN_WARPS, 0, d->stream>>>(d->g, d->act[l], d->dY[l], d->part);
-      k_dn_reduce_rows<<<(DN_TAPS * DN_C * DN_C + 255) / 256, 256, 0, d->stream>>>(d->part, wb, DN_TAPS * DN_C * DN_C,
-                                                                                  d->grad + (size_t)l * DN_LAYER);
-      k_dn_bgrad<<<wb, 256, 0, d->stream>>>(d->g, d->dY[l], d->part);
-      k_dn_reduce_rows<<<1, DN_C, 0, d->stream>>>(d->part, wb, DN_C, d->grad + (size_t)l * DN_LAYER + DN_TAPS * DN_C * DN_C);
+      k_dn_wgrad<<<dim3(wb, DN_WGRAD_ROWS + 1), 32 * DN_WARPS, 0, d->stream>>>(d->g, d->act[l], d->dY[l], d->part);
+      k_dn_reduce_rows<<<(DN_LAYER + 63) / 64, 64, 0, d->stream>>>(d->part, wb, DN_LAYER, d->grad + (size_t)l * DN_LAYER);
       if (l > 0)
          if (int rc = dnConv(d, d->stream, true, l, d->dY[l], nullptr, 2, d->dY[l - 1], d->act[l], nullptr, nullptr,
                              DnMoments{}, d->err))
             return rc;
    }
    RH_CUDA(cudaGetLastError());
-   std::vector<double> lp(DN_LOSS_BLOCKS);
-   RH_CUDA(cudaMemcpyAsync(lp.data(), d->lossPart, sizeof(double) * DN_LOSS_BLOCKS, cudaMemcpyDeviceToHost, d->stream));
-   RH_CUDA(cudaStreamSynchronize(d->stream));
-   double a = 0.0;
-   for (double x : lp) a += x;
-   if (loss) *loss = a / (4.0 * (double)in);
    return RHGPU_OK;
 }
 
-// host moments in the ABI layout (rho N, Ji interleaved 3N) -> device planar scratch (acc)
-int dnUploadMoments(rhgpu_dn* d, const double* rho, const double* ji, double* planar) {
+// host moments in the ABI layout (rho N, Ji interleaved 3N) -> the same on the device
+int dnUploadMoments(rhgpu_dn* d, const double* rho, const double* ji, double* dev) {
    const long long N = d->g.N;
-   std::vector<double> h(4 * (size_t)N);
-   for (long long n = 0; n < N; ++n) {
-      h[n] = rho[n];
-      for (int l = 0; l < 3; ++l) h[(1 + l) * N + n] = ji[3 * n + l];
-   }
-   RH_CUDA(cudaMemcpyAsync(planar, h.data(), sizeof(double) * 4 * N, cudaMemcpyHostToDevice, d->stream));
-   RH_CUDA(cudaStreamSynchronize(d->stream));
+   RH_CUDA(cudaMemcpyAsync(dev, rho, sizeof(double) * N, cudaMemcpyHostToDevice, d->stream));
+   RH_CUDA(cudaMemcpyAsync(dev + N, ji, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, d->stream));
    return RHGPU_OK;
 }
 
@@ -166,9 +161,9 @@ int rhgpu_dn_create(int32_t nx, int32_t ny, int32_t nz, const int32_t* periodic,
    }
    alloc((void**)&d->res, sizeof(float) * 4 * N);
    alloc((void**)&d->out32, sizeof(float) * 4 * N);
-   alloc((void**)&d->part, sizeof(float) * d->partRows * DN_TAPS * DN_C * DN_C);
-   alloc((void**)&d->lossPart, sizeof(double) * DN_LOSS_BLOCKS);
-   alloc((void**)&d->acc, sizeof(double) * std::max(4 * N, 4LL * 64));   // also k_dn_err's 64 x 4 partials
+   alloc((void**)&d->part, sizeof(float) * d->partRows * DN_LAYER);
+   alloc((void**)&d->lossPart, sizeof(double) * DN_LOSS_BLOCKS * DN_LOSS_RING);
+   alloc((void**)&d->acc, sizeof(double) * std::max(8 * N, 4LL * 64));   // also k_dn_err's 64 x 4 partials
    if (pair_capacity > 0) {
       alloc((void**)&d->pairIn, sizeof(float) * 4 * N * pair_capacity);
       alloc((void**)&d->pairOut, sizeof(float) * 4 * N * pair_capacity);
@@ -265,18 +260,20 @@ int rhgpu_dn_apply(rhgpu_dn* d, const double* rho_in, const double* ji_in, doubl
    if (!d || !rho_in || !ji_in || !rho_out || !ji_out) return fail(RHGPU_ERR_ARG, "dn_apply: bad arguments");
    RH_CUDA(cudaSetDevice(d->device));
    const long long N = d->g.N;
-   int rc = dnUploadMoments(d, rho_in, ji_in, d->acc);
-   if (rc) return rc;
-   rc = dnApplyMoments(d, d->stream, d->acc, d->acc + N, min_rho, d->err);
+   // acc: rho and J in planes (the network's form), then J interleaved as the caller has it
+   double* const J = d->acc + N;
+   double* const Jin = d->acc + 4 * N;
+   RH_CUDA(cudaMemcpyAsync(d->acc, rho_in, sizeof(double) * N, cudaMemcpyHostToDevice, d->stream));
+   RH_CUDA(cudaMemcpyAsync(Jin, ji_in, sizeof(double) * 3 * N, cudaMemcpyHostToDevice, d->stream));
+   k_dn_planar<<<blocks1d(3 * N, 256), 256, 0, d->stream>>>(N, Jin, J, 0);
+   int rc = dnApplyMoments(d, d->stream, d->acc, J, min_rho, d->err);
    if (!rc) rc = dnCheckError(d);
    if (rc) return rc;
-   std::vector<double> h(4 * (size_t)N);
-   RH_CUDA(cudaMemcpyAsync(h.data(), d->acc, sizeof(double) * 4 * N, cudaMemcpyDeviceToHost, d->stream));
+   k_dn_planar<<<blocks1d(3 * N, 256), 256, 0, d->stream>>>(N, J, Jin, 1);
+   RH_CUDA(cudaGetLastError());
+   RH_CUDA(cudaMemcpyAsync(rho_out, d->acc, sizeof(double) * N, cudaMemcpyDeviceToHost, d->stream));
+   RH_CUDA(cudaMemcpyAsync(ji_out, Jin, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, d->stream));
    RH_CUDA(cudaStreamSynchronize(d->stream));
-   for (long long v = 0; v < N; ++v) {
-      rho_out[v] = h[v];
-      for (int l = 0; l < 3; ++l) ji_out[3 * v + l] = h[(1 + l) * N + v];
-   }
    return RHGPU_OK;
 }
 
@@ -285,21 +282,23 @@ int rhgpu_dn_loss_grad(rhgpu_dn* d, const double* rho_in, const double* ji_in, c
    if (!d || !rho_in || !ji_in || !rho_t || !ji_t) return fail(RHGPU_ERR_ARG, "dn_loss_grad: bad arguments");
    RH_CUDA(cudaSetDevice(d->device));
    const long long N = d->g.N;
-   int rc = dnUploadMoments(d, rho_t, ji_t, d->acc);
+   // acc: the target's and the input's moments, normalized into out32's and res' form;
+   // the target waits in acc's first half, which the input's upload leaves alone
+   double* const in = d->acc + 4 * N;
+   int rc = dnUploadMoments(d, rho_t, ji_t, in);
    if (rc) return rc;
-   k_dn_norm<<<blocks1d(N, 256), 256, 0, d->stream>>>(N, d->acc, d->acc + N, 1.0 / d->sr, 1.0 / d->sj, d->vel, d->out32);
-   // target kept in dY[0]'s storage as FP32 (N x 4 floats fit in 8 u32 per voxel)
-   float* target = reinterpret_cast<float*>(d->dY[0]);
-   RH_CUDA(cudaMemcpyAsync(target, d->out32, sizeof(float) * 4 * N, cudaMemcpyDeviceToDevice, d->stream));
-   rc = dnUploadMoments(d, rho_in, ji_in, d->acc);
+   float* const target = reinterpret_cast<float*>(d->acc);
+   k_dn_norm<<<blocks1d(N, 256), 256, 0, d->stream>>>(N, in, in + N, 1.0 / d->sr, 1.0 / d->sj, d->vel, target);
+   rc = dnUploadMoments(d, rho_in, ji_in, in);
    if (rc) return rc;
-   k_dn_norm<<<blocks1d(N, 256), 256, 0, d->stream>>>(N, d->acc, d->acc + N, 1.0 / d->sr, 1.0 / d->sj, d->vel, d->res);
-   rc = dnForward(d);
+   k_dn_norm<<<blocks1d(N, 256), 256, 0, d->stream>>>(N, in, in + N, 1.0 / d->sr, 1.0 / d->sj, d->vel, d->res);
+   rc = dnForward(d, d->res);
+   if (!rc) rc = dnBackward(d, target, d->lossPart);
    if (rc) return rc;
-   // the loss kernel reads the target before the backward overwrites dY[0]
-   float* tcopy = reinterpret_cast<float*>(d->acc);
-   RH_CUDA(cudaMemcpyAsync(tcopy, target, sizeof(float) * 4 * N, cudaMemcpyDeviceToDevice, d->stream));
-   rc = dnBackward(d, tcopy, loss);
+   double lp[DN_LOSS_BLOCKS];
+   RH_CUDA(cudaMemcpyAsync(lp, d->lossPart, sizeof lp, cudaMemcpyDeviceToHost, d->stream));
+   RH_CUDA(cudaStreamSynchronize(d->stream));
+   if (loss) *loss = dnLossOf(d, lp);
    if (!rc) rc = dnCheckError(d);
    if (rc) return rc;
    if (grad) {
@@ -405,22 +404,27 @@ int rhgpu_dn_train(rhgpu_dn* d, int32_t iterations, float lr, double* mean_loss)
    const long long N = d->g.N;
    double tot = 0.0;
    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+   std::vector<double> lp((size_t)DN_LOSS_BLOCKS * std::min(iterations, DN_LOSS_RING));
    for (int it = 0; it < iterations; ++it) {
       d->rng = d->rng * 6364136223846793005ull + 1442695040888963407ull;
       const int p = (int)((d->rng >> 33) % (unsigned long long)d->pairCount);
-      RH_CUDA(cudaMemcpyAsync(d->res, d->pairIn + (size_t)p * 4 * N, sizeof(float) * 4 * N, cudaMemcpyDeviceToDevice, d->stream));
-      int rc = dnForward(d);
+      int rc = dnForward(d, d->pairIn + (size_t)p * 4 * N);
       if (rc) return rc;
-      double l = 0.0;
-      rc = dnBackward(d, d->pairOut + (size_t)p * 4 * N, &l);
+      const int ring = it % DN_LOSS_RING;
+      rc = dnBackward(d, d->pairOut + (size_t)p * 4 * N, d->lossPart + (size_t)ring * DN_LOSS_BLOCKS);
       if (rc) return rc;
-      tot += l;
       d->adamStep += 1;
       const float c1 = 1.f - std::pow(b1, (float)d->adamStep), c2 = 1.f - std::pow(b2, (float)d->adamStep);
       k_dn_adam<<<(DN_PARAMS + 255) / 256, 256, 0, d->stream>>>(d->params, d->grad, d->m, d->v, d->mask, DN_PARAMS, lr, b1, b2,
                                                                eps, c1, c2);
       rc = dnRebuildImages(d);
       if (rc) return rc;
+      if (ring == DN_LOSS_RING - 1 || it == iterations - 1) {   // the losses of the last ring + 1 iterations
+         RH_CUDA(cudaMemcpyAsync(lp.data(), d->lossPart, sizeof(double) * DN_LOSS_BLOCKS * (ring + 1),
+                                 cudaMemcpyDeviceToHost, d->stream));
+         RH_CUDA(cudaStreamSynchronize(d->stream));
+         for (int r = 0; r <= ring; ++r) tot += dnLossOf(d, lp.data() + (size_t)r * DN_LOSS_BLOCKS);
+      }
    }
    RH_CUDA(cudaStreamSynchronize(d->stream));
    if (int rc = dnCheckError(d)) return rc;
@@ -444,8 +448,7 @@ int rhgpu_dn_pair_error(rhgpu_dn* d, int32_t pair, double* out4) {
    const long long N = d->g.N;
    const float* in = d->pairIn + (size_t)pair * 4 * N;
    const float* tg = d->pairOut + (size_t)pair * 4 * N;
-   RH_CUDA(cudaMemcpyAsync(d->res, in, sizeof(float) * 4 * N, cudaMemcpyDeviceToDevice, d->stream));
-   int rc = dnForward(d);
+   int rc = dnForward(d, in);
    if (rc) return rc;
    std::vector<double> h(4 * 64);
    double r[2][4];
