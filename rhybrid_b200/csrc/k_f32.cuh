@@ -28,7 +28,8 @@
 namespace rh {
 
 struct F32Buf {
-   int* cell;        // cell index
+   int* cell;        // cell index; the seven arrays are planes of one
+   long long plane;  // their distance in elements
    float* o[3];      // offsets in the cell, cell units
    float* v[3];      // velocity [m/s]
    int* cnt;         // particles per segment
@@ -187,16 +188,22 @@ __device__ inline void cicWeightsF(const float o[3], float wq, float w8[8]) {
 constexpr int REC32 = 12;   // floats per deposit record: w8[8], then 1, v[3] (48 bytes apart: any eight on different banks)
 
 // resident blocks per SM: the kernel waits on its barriers and shared-memory
-// round trips, so warps count for more than the few registers that 36 a thread
-// spill (Mars run, 9.25e7 ions: 4 blocks 3.63 ms, 5 3.31, 6 3.09, 7 and 8 3.05)
-constexpr int F32_BLOCKS = 7;
+// round trips, so warps count for more than the few registers that 32 a thread
+// spill (Mars run, 9.25e7 ions: 4 blocks 3.63 ms, 5 3.31, 6 3.09, 8 3.05)
+constexpr int F32_BLOCKS = 8;
 // shared memory of k_f32_push_deposit
-constexpr int F32_PTRS = 14;   // one species' arrays offset to the segment: current cell, o, v (0-6), next (7-13)
+// one species' storage at the block's segment: its current and next cell planes
+// and the other planes' distances (cell, o[3], v[3])
+struct F32At {
+   const int* cur;
+   int* nxt;
+   long long curPlane, nxtPlane;
+};
 struct F32PushShared {
    alignas(16) float rec[PD_T * REC32];     // deposit records of a chunk; at the end acc[SEG][32]
    float pf[7][PD_T];                       // the next chunk's particles: cell (int bits), o[3], v[3]
    SegFields32 f;                           // field stencil of the segment
-   void* ptr[FAST_MAX_SPECIES][F32_PTRS];
+   F32At at[FAST_MAX_SPECIES];
    StencilRow rows[SF_MAX_ROWS];
    alignas(8) unsigned char wd[SEG][PD_VW];   // records per (dual cell, group)
    int wcnt[PD_VW];                         // stayers per group
@@ -205,14 +212,19 @@ struct F32PushShared {
    int stay[FAST_MAX_SPECIES];              // stayers of each species up to and with the chunk
 };
 
-// this thread's particle of the chunk that starts at group V0 requested into pf (cp.async)
-__device__ __forceinline__ void f32Prefetch(F32PushShared& sh, int V0, int ns) {
+// this thread's particle of the chunk that starts at group V0 requested into pf
+// (cp.async): its species s and index p (p < 0: none)
+__device__ __forceinline__ void f32Prefetch(F32PushShared& sh, int V0, int ns, int& s, int& p) {
    const int tid = threadIdx.x, V = V0 + (tid >> 5);
-   const int s = pdSpecies(sh, V, ns);
-   const int p = (V - sh.first[s]) * 32 + (tid & 31);
-   if (p < sh.cnt[s]) {
+   s = pdSpecies(sh, V, ns);
+   p = (V - sh.first[s]) * 32 + (tid & 31);
+   if (p >= sh.cnt[s]) {
+      p = -1;
+   } else {
+      const int* q = sh.at[s].cur + p;
+      const long long plane = sh.at[s].curPlane;
 #pragma unroll
-      for (int a = 0; a < 7; ++a) cpAsync4(&sh.pf[a][tid], (const float*)sh.ptr[s][a] + p);
+      for (int a = 0; a < 7; ++a, q += plane) cpAsync4(&sh.pf[a][tid], q);
    }
    cpAsyncCommit();
 }
@@ -261,23 +273,21 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
       if (lane <= ns) sh.first[lane] = x - groups;
       if (lane < FAST_MAX_SPECIES) { sh.cnt[lane] = cnt; sh.stay[lane] = 0; }
    }
-   for (int q = tid; q < F32_PTRS * ns; q += PD_T) {
-      const int s = q / F32_PTRS, k = q - s * F32_PTRS;
-      const F32Species& SS = FS.st[s];
+   if (tid >= 32 && tid < 32 + ns) {
+      const F32Species& SS = FS.st[tid - 32];
       const long long b = SS.base[S];
-      const F32Buf& B = k < 7 ? SS.cur : SS.nxt;
-      const int kk = k < 7 ? k : k - 7;
-      void* v;
-      if (kk == 0) v = B.cell + b;
-      else if (kk < 4) v = B.o[kk - 1] + b;
-      else v = B.v[kk - 4] + b;
-      sh.ptr[s][k] = v;
+      F32At& A = sh.at[tid - 32];
+      A.cur = SS.cur.cell + b;
+      A.nxt = SS.nxt.cell + b;
+      A.curPlane = SS.cur.plane;
+      A.nxtPlane = SS.nxt.plane;
    }
    // (stageSegRows' own barrier publishes the species and the pointers)
    stageSegRows<PD_T>(g, f, pp.use_ep, xs0, ys0, zs0, sh.f, sh.rows);
    __syncthreads();
    const int groups = sh.first[ns];
-   f32Prefetch(sh, 0, ns);
+   int sn = 0, pn = -1;   // the prefetched particle's species and index
+   f32Prefetch(sh, 0, ns, sn, pn);
    const int myDual = tid >> 3, myPair = (tid >> 1) & 3, myHalf = tid & 1;
    float a00 = 0.0f, a01 = 0.0f, a10 = 0.0f, a11 = 0.0f;
 
@@ -286,10 +296,8 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
       int cell = 0, duv = 0, dyz = 0, mflags = 0, rrank = 0;
       bool stay = false, rec = false, clamp = false;
       cpAsyncWaitAll();   // this thread's copies of the chunk
-      const int V = V0 + warp;
-      const int s = pdSpecies(sh, V, ns);
-      const int p = (V - sh.first[s]) * 32 + lane;
-      if (p < sh.cnt[s]) {
+      const int s = sn, p = pn;
+      if (p >= 0) {
          const int c = __float_as_int(sh.pf[0][tid]);
 #pragma unroll
          for (int a = 0; a < 3; ++a) { o[a] = sh.pf[1 + a][tid]; v[a] = sh.pf[4 + a][tid]; }
@@ -379,7 +387,7 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
       }
       __syncthreads();
       // every shared-memory read of this chunk's particles is done: request the next chunk's
-      if (V0 + PD_VW < groups) f32Prefetch(sh, V0 + PD_VW, ns);
+      if (V0 + PD_VW < groups) f32Prefetch(sh, V0 + PD_VW, ns, sn, pn);
       // every warp, per dual cell (lane): the first sorted record of the dual cell (bin)
       const uint2 c8 = *reinterpret_cast<const uint2*>(&sh.wd[lane][0]);
       int binD, nrec;
@@ -420,13 +428,13 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
       }
       __syncthreads();
       if (stay) {
-         void* const* nx = &sh.ptr[s][7];
-         ((int*)nx[0])[slot] = cell;
+         int* q = sh.at[s].nxt + slot;
+         const long long plane = sh.at[s].nxtPlane;
+         *q = cell;
 #pragma unroll
-         for (int a = 0; a < 3; ++a) {
-            ((float*)nx[1 + a])[slot] = o[a];
-            ((float*)nx[4 + a])[slot] = v[a];
-         }
+         for (int a = 0; a < 3; ++a) { q += plane; *q = __float_as_int(o[a]); }
+#pragma unroll
+         for (int a = 0; a < 3; ++a) { q += plane; *q = __float_as_int(v[a]); }
       }
       // ---- this thread's sums, records in list order ----------------------------------------
 #pragma unroll 2

@@ -52,7 +52,8 @@ constexpr int REC = 11;                   // its doubles per deposit record: w8[
 static_assert(SEG == 32 && SEG * 8 == FT, "its deposit sums map (dual cell, corner) to one thread");
 
 struct SegBuf {
-   double* a[7];        // x, y, z (cell-local), vx, vy, vz, weight
+   double* a[7];        // x, y, z (cell-local), vx, vy, vz, weight: planes of one array
+   long long plane;     // their distance in elements
    unsigned char* lx;   // dual x index within the segment
    int* cnt;            // particles per segment
 };
@@ -388,9 +389,15 @@ __device__ __forceinline__ void segPartialsOut(const GridInfo& g, const FastGeom
    }
 }
 
-// one species' arrays offset to the block's segment: current x..w (0-6), next
-// x..w (7-13), current lx (14), next lx (15)
-constexpr int SEG_PTRS = 16;
+// one species' storage at the block's segment: its current and next x planes,
+// the other planes' distances, and the dual x indices
+struct SegAt {
+   const double* cur;
+   double* nxt;
+   long long curPlane, nxtPlane;
+   const unsigned char* curLx;
+   unsigned char* nxtLx;
+};
 
 // k_fast_push_deposit: one thread per particle of a chunk, a warp's 32 particles
 // a group of one species
@@ -407,7 +414,7 @@ struct PushDepositShared {
    double rec[PD_T * PD_REC];            // deposit records of a chunk; at the end acc[SEG][32]
    double pf[7][PD_T];                // the next chunk's particles, one plane per component
    SegFields f;                           // field stencil of the segment
-   void* ptr[FAST_MAX_SPECIES][SEG_PTRS];
+   SegAt at[FAST_MAX_SPECIES];
    StencilRow rows[SF_MAX_ROWS];
    alignas(8) unsigned char wd[SEG][PD_VW];   // records per (dual cell, group)
    int wcnt[PD_VW];                       // stayers per group
@@ -444,38 +451,30 @@ __device__ __forceinline__ int pdSpecies(const SH& sh, int V, int ns) {
 }
 
 // this thread's particle of the chunk that starts at group V0 requested into pf
-__device__ __forceinline__ void pdPrefetch(PushDepositShared& sh, int V0, int ns, int& lx) {
+// (its species s, index p and dual x lx; p < 0: none)
+__device__ __forceinline__ void pdPrefetch(PushDepositShared& sh, int V0, int ns, int& s, int& p, int& lx) {
    const int tid = threadIdx.x, V = V0 + (tid >> 5);
-   const int s = pdSpecies(sh, V, ns);
-   const int p = (V - sh.first[s]) * 32 + (tid & 31);
-   if (p < sh.cnt[s]) {
+   s = pdSpecies(sh, V, ns);
+   p = (V - sh.first[s]) * 32 + (tid & 31);
+   if (p >= sh.cnt[s]) {
+      p = -1;
+   } else {
+      const double* q = sh.at[s].cur + p;
+      const long long plane = sh.at[s].curPlane;
 #pragma unroll
-      for (int a = 0; a < 7; ++a) cpAsync8(&sh.pf[a][tid], (const double*)sh.ptr[s][a] + p, 8);
-      lx = ((const unsigned char*)sh.ptr[s][14])[p];
+      for (int a = 0; a < 7; ++a, q += plane) cpAsync8(&sh.pf[a][tid], q, 8);
+      lx = sh.at[s].curLx[p];
    }
    cpAsyncCommit();
 }
 
-// the CIC weights of a position in its cell, as cicWeightsLocal, bit for bit.
-// The quotients need no range test: the numerators are 0 or at least an ulp of
-// dx / 2, at most dx.
-__device__ __forceinline__ void cicWeightsHalf(double x, double y, double z, bool hx, bool hy, bool hz, double wq,
-                                               const GridInfo& g, double hdx, double w8[8]) {
-   const double rx = hx ? x - hdx : x + hdx, ry = hy ? y - hdx : y + hdx, rz = hz ? z - hdx : z + hdx;
-   double q = rx * g.rdx;
-   const double w_x = fma(fma(-q, g.dx, rx), g.rdx, q);
-   q = ry * g.rdx;
-   const double w_y = fma(fma(-q, g.dx, ry), g.rdx, q);
-   q = rz * g.rdx;
-   const double w_z = fma(fma(-q, g.dx, rz), g.rdx, q);
-   w8[0] = (1 - w_x) * (1 - w_y) * (1 - w_z) * wq;
-   w8[1] = w_x * (1 - w_y) * (1 - w_z) * wq;
-   w8[2] = (1 - w_x) * w_y * (1 - w_z) * wq;
-   w8[3] = w_x * w_y * (1 - w_z) * wq;
-   w8[4] = (1 - w_x) * (1 - w_y) * w_z * wq;
-   w8[5] = w_x * (1 - w_y) * w_z * wq;
-   w8[6] = (1 - w_x) * w_y * w_z * wq;
-   w8[7] = w_x * w_y * w_z * wq;
+// the CIC fraction of one axis: (x - the dual cell's lower centre) / dx, bit for
+// bit that of cicWeightsLocal. The quotient needs no range test: the numerator
+// is 0 or at least an ulp of dx / 2, at most dx.
+__device__ __forceinline__ double cicFraction(double x, const GridInfo& g, double hdx) {
+   const double r = x < hdx ? x + hdx : x - hdx;
+   const double q = r * g.rdx;
+   return fma(fma(-q, g.dx, r), g.rdx, q);
 }
 
 // migration of one axis (migrateAxis); a coordinate inside [0, dx) is told by
@@ -546,16 +545,16 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
       if (lane <= ns) sh.first[lane] = x - groups;
       if (lane < FAST_MAX_SPECIES) { sh.cnt[lane] = cnt; sh.stay[lane] = 0; }
    }
-   for (int q = tid; q < SEG_PTRS * ns; q += PD_T) {
-      const int s = q / SEG_PTRS, k = q - s * SEG_PTRS;
-      const SegSpecies& SS = FS.st[s];
+   if (tid >= 32 && tid < 32 + ns) {
+      const SegSpecies& SS = FS.st[tid - 32];
       const long long b = SS.base[S];
-      void* v;
-      if (k < 7) v = SS.cur.a[k] + b;
-      else if (k < 14) v = SS.nxt.a[k - 7] + b;
-      else if (k == 14) v = SS.cur.lx + b;
-      else v = SS.nxt.lx + b;
-      sh.ptr[s][k] = v;
+      SegAt& A = sh.at[tid - 32];
+      A.cur = SS.cur.a[0] + b;
+      A.nxt = SS.nxt.a[0] + b;
+      A.curPlane = SS.cur.plane;
+      A.nxtPlane = SS.nxt.plane;
+      A.curLx = SS.cur.lx + b;
+      A.nxtLx = SS.nxt.lx + b;
    }
    if (const int r = PD_T - 1 - tid; r < SF_ROWS_B + SF_ROWS_C * (pp.use_ep ? 2 : 1)) {
       int len, dxs, l, dy, dz;
@@ -575,8 +574,8 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
    }
    __syncthreads();
    const int groups = sh.first[ns];
-   int lxn = 0;
-   pdPrefetch(sh, 0, ns, lxn);
+   int sn = 0, pn = -1, lxn = 0;   // the prefetched particle's species, index and dual x
+   pdPrefetch(sh, 0, ns, sn, pn, lxn);
    pdStage<PER>(g, f, pp.use_ep, sh);
    cpAsyncCommit();
    cpAsyncWaitAll();
@@ -589,12 +588,10 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
    for (int V0 = 0; V0 < groups; V0 += PD_VW) {
       double st[7];
       int duv = 0, dyz = 0, mflags = 0, rrank = 0;
-      bool stay = false, rec = false, hx = false, hy = false, hz = false, clamp = false;
+      bool stay = false, rec = false, clamp = false;
       if (V0 > 0) cpAsyncWaitAll();   // this thread's copies of the chunk
-      const int V = V0 + warp;
-      const int s = pdSpecies(sh, V, ns);
-      const int p = (V - sh.first[s]) * 32 + lane;
-      if (p < sh.cnt[s]) {
+      const int s = sn, p = pn;
+      if (p >= 0) {
 #pragma unroll
          for (int a = 0; a < 7; ++a) st[a] = sh.pf[a][tid];
          const int lu = lxn;
@@ -632,9 +629,8 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
          }
          if (inside) {
             // the new dual cell relative to the segment's first, and to its row
-            hx = !(st[0] < hdx); hy = !(st[1] < hdx); hz = !(st[2] < hdx);
-            int du = lu + ox + (hx ? 1 : 0) - gx;
-            const int dy = oy + (hy ? 1 : 0) - gy, dz = oz + (hz ? 1 : 0) - gz;
+            int du = lu + ox + (st[0] < hdx ? 0 : 1) - gx;
+            const int dy = oy + (st[1] < hdx ? 0 : 1) - gy, dz = oz + (st[2] < hdx ? 0 : 1) - gz;
             if ((PER & 1) && nseg == 1) {
                if (du < 0) du += fg.nd[0];
                else if (du >= fg.nd[0]) du -= fg.nd[0];
@@ -687,7 +683,9 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
       }
       __syncthreads();
       // every shared-memory read of this chunk's particles is done: request the next chunk's
-      if (V0 + PD_VW < groups) pdPrefetch(sh, V0 + PD_VW, ns, lxn);
+      if (V0 + PD_VW < groups) pdPrefetch(sh, V0 + PD_VW, ns, sn, pn, lxn);
+      // (unconditional: the arithmetic fills the waits of the scan below)
+      const double w_x = cicFraction(st[0], g, hdx), w_y = cicFraction(st[1], g, hdx), w_z = cicFraction(st[2], g, hdx);
       // every warp, per dual cell (lane): the first sorted record of the dual cell
       // (bin); the group counts of dual cell `lane` are bytes (each at most 32),
       // byte sums by one multiply per 32-bit half
@@ -721,20 +719,22 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
       unsigned long long mb = 0;
       if (lm && lane == __ffs(lm) - 1) mb = atomicAdd(fb.nmovers, (unsigned long long)__popc(lm));
       if (rec) {
-         double w8[8];
-         cicWeightsHalf(st[0], st[1], st[2], hx, hy, hz, st[6] * FS.sp[s].q, g, hdx, w8);
          double2* const r = reinterpret_cast<double2*>(sh.rec + recPos * PD_REC);
-#pragma unroll
-         for (int o = 0; o < 4; ++o) r[o] = make_double2(w8[2 * o], w8[2 * o + 1]);
+         const double wq = st[6] * FS.sp[s].q;
+         r[0] = make_double2((1 - w_x) * (1 - w_y) * (1 - w_z) * wq, w_x * (1 - w_y) * (1 - w_z) * wq);
+         r[1] = make_double2((1 - w_x) * w_y * (1 - w_z) * wq, w_x * w_y * (1 - w_z) * wq);
+         r[2] = make_double2((1 - w_x) * (1 - w_y) * w_z * wq, w_x * (1 - w_y) * w_z * wq);
+         r[3] = make_double2((1 - w_x) * w_y * w_z * wq, w_x * w_y * w_z * wq);
          r[4] = make_double2(1.0, st[3]);
          r[5] = make_double2(st[4], st[5]);
       }
       __syncthreads();
       if (stay) {
-         double* const* nx = (double* const*)&sh.ptr[s][7];
+         double* q = sh.at[s].nxt + slot;
+         const long long plane = sh.at[s].nxtPlane;
 #pragma unroll
-         for (int a = 0; a < 7; ++a) nx[a][slot] = st[a];
-         ((unsigned char*)sh.ptr[s][15])[slot] = (unsigned char)duv;
+         for (int a = 0; a < 7; ++a, q += plane) *q = st[a];
+         sh.at[s].nxtLx[slot] = (unsigned char)duv;
       }
       // ---- this thread's sums, records in list order ----------------------------------------
 #pragma unroll 2

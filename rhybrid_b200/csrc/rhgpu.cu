@@ -417,7 +417,7 @@ int rhgpu_destroy(rhgpu_ctx* c) {
    for (int s = 0; s < c->ns; ++s) {
       SegHost& h = c->seg[s];
       for (int b = 0; b < 2; ++b) {
-         for (int a = 0; a < 7; ++a) cudaFree(h.a[b][a]);
+         cudaFree(h.a[b][0]);   // the planes are one allocation
          cudaFree(h.lx[b]);
          cudaFree(h.cnt[b]);
       }
@@ -444,8 +444,7 @@ int rhgpu_destroy(rhgpu_ctx* c) {
    for (int s = 0; s < c->ns; ++s) {
       F32Host& h = c->f32[s];
       for (int b = 0; b < 2; ++b) {
-         cudaFree(h.cell[b]);
-         for (int a = 0; a < 3; ++a) { cudaFree(h.o[b][a]); cudaFree(h.v[b][a]); }
+         cudaFree(h.cell[b]);   // the seven arrays are one allocation
          cudaFree(h.cnt[b]);
       }
       cudaFree(h.base);

@@ -10,6 +10,7 @@ namespace rhh {
 F32Buf f32View(const F32Host& h, int which) {
    F32Buf b;
    b.cell = h.cell[which];
+   b.plane = h.capOf[which];
    for (int a = 0; a < 3; ++a) { b.o[a] = h.o[which][a]; b.v[a] = h.v[which][a]; }
    b.cnt = h.cnt[which];
    return b;
@@ -19,20 +20,17 @@ int f32Reserve(F32Host& h, int which, long long slots) {
    if (slots <= h.capOf[which] && h.cell[which]) return RHGPU_OK;
    const long long had = h.capOf[which];
    auto release = [&]() {
-      cudaFree(h.cell[which]);
+      cudaFree(h.cell[which]);   // the seven arrays are one allocation
       h.cell[which] = nullptr;
-      for (int a = 0; a < 3; ++a) {
-         cudaFree(h.o[which][a]); cudaFree(h.v[which][a]);
-         h.o[which][a] = nullptr; h.v[which][a] = nullptr;
-      }
+      for (int a = 0; a < 3; ++a) { h.o[which][a] = nullptr; h.v[which][a] = nullptr; }
       h.capOf[which] = 0;
    };
    auto alloc = [&](long long n) {
-      cudaError_t e = cudaMalloc(&h.cell[which], sizeof(int) * n);
-      for (int a = 0; a < 3 && e == cudaSuccess; ++a) {
-         e = cudaMalloc(&h.o[which][a], sizeof(float) * n);
-         if (e == cudaSuccess) e = cudaMalloc(&h.v[which][a], sizeof(float) * n);
-      }
+      static_assert(sizeof(int) == sizeof(float), "planes of one allocation");
+      const cudaError_t e = cudaMalloc(&h.cell[which], sizeof(int) * 7 * n);
+      if (e != cudaSuccess) return e;
+      float* const f = reinterpret_cast<float*>(h.cell[which]);
+      for (int a = 0; a < 3; ++a) { h.o[which][a] = f + (1 + a) * n; h.v[which][a] = f + (4 + a) * n; }
       return e;
    };
    release();

@@ -25,6 +25,7 @@ int ensureSortTmp(rhgpu_ctx* c, size_t bytes) {
 SegBuf segView(const SegHost& h, int which) {
    SegBuf b;
    for (int a = 0; a < 7; ++a) b.a[a] = h.a[which][a];
+   b.plane = h.capOf[which];
    b.lx = h.lx[which];
    b.cnt = h.cnt[which];
    return b;
@@ -35,16 +36,17 @@ int segReserve(SegHost& h, int which, long long slots) {
    if (slots <= h.capOf[which] && h.a[which][0]) return RHGPU_OK;
    const long long had = h.capOf[which];
    auto release = [&]() {
-      for (int a = 0; a < 7; ++a) { cudaFree(h.a[which][a]); h.a[which][a] = nullptr; }
+      cudaFree(h.a[which][0]);   // the planes are one allocation
+      for (int a = 0; a < 7; ++a) h.a[which][a] = nullptr;
       cudaFree(h.lx[which]);
       h.lx[which] = nullptr;
       h.capOf[which] = 0;
    };
    auto alloc = [&](long long n) {
-      cudaError_t e = cudaSuccess;
-      for (int a = 0; a < 7 && e == cudaSuccess; ++a) e = cudaMalloc(&h.a[which][a], sizeof(double) * n);
-      if (e == cudaSuccess) e = cudaMalloc(&h.lx[which], n);
-      return e;
+      cudaError_t e = cudaMalloc(&h.a[which][0], sizeof(double) * 7 * n);
+      if (e != cudaSuccess) return e;
+      for (int a = 1; a < 7; ++a) h.a[which][a] = h.a[which][0] + a * n;
+      return cudaMalloc(&h.lx[which], n);
    };
    release();
    long long n = growSlots(had, slots);
