@@ -195,45 +195,47 @@ __global__ void k_ext_bc(GridInfo g, Fields f, FieldParams fp, const int* ext, i
    }
 }
 
-__global__ void __launch_bounds__(128, 8) k_node_fused(GridInfo g, Fields f, FieldParams fp, unsigned long long* cnt) {
-   RH_CELL_PROLOGUE
-   for (int l = 0; l < 3; ++l) f.cellAvgB[l * N + n] += f.cellB[l * N + n];
+// one layer slot's array a at (x, y) of this thread plus (dx, dy)
+struct NodeStencil {
+   const double* L;   // cell layer k
+   const double* U;   // cell layer k + 1
+   int off;
+   __device__ __forceinline__ double at(int a, int dx, int dy, int dz) const {
+      return (dz ? U : L)[a * (ND_Y + 1) * NT_LX + off + dy * NT_LX + dx];
+   }
+   // the eight corners' mean in the reference's order
+   __device__ __forceinline__ double mean(int a) const {
+      return 0.125 * (at(a, 0, 0, 0) + at(a, 0, 0, 1) + at(a, 0, 1, 0) + at(a, 1, 0, 0) + at(a, 0, 1, 1) + at(a, 1, 1, 0) +
+                      at(a, 1, 0, 1) + at(a, 1, 1, 1));
+   }
+};
+
+__device__ __forceinline__ void nodeFromStencil(const GridInfo& g, const Fields& f, const FieldParams& fp,
+                                                unsigned long long* cnt, int i, int j, int k, long long n,
+                                                const NodeStencil& st, const double avg[3], double eta) {
+   const long long N = g.N;
+   for (int l = 0; l < 3; ++l) f.cellAvgB[l * N + n] = avg[l] + st.at(l, 0, 0, 0);
    if (!plusOk(g, i, j, k)) return;
-   const long long c000 = n, c001 = nbr(g, i, j, k, 0, 0, 1), c010 = nbr(g, i, j, k, 0, 1, 0),
-                   c100 = nbr(g, i, j, k, 1, 0, 0), c011 = nbr(g, i, j, k, 0, 1, 1),
-                   c110 = nbr(g, i, j, k, 1, 1, 0), c101 = nbr(g, i, j, k, 1, 0, 1),
-                   c111 = nbr(g, i, j, k, 1, 1, 1);
    // cell2Node
    double nodeBavg[3];
-   for (int l = 0; l < 3; ++l) {
-      const double* s = f.cellB + l * N;
-      nodeBavg[l] = 0.125 * (s[c000] + s[c001] + s[c010] + s[c100] + s[c011] + s[c110] + s[c101] + s[c111]);
-   }
-   double rho;
-   {
-      const double* s = f.cellRho;
-      rho = 0.125 * (s[c000] + s[c001] + s[c010] + s[c100] + s[c011] + s[c110] + s[c101] + s[c111]);
-   }
+#pragma unroll
+   for (int l = 0; l < 3; ++l) nodeBavg[l] = st.mean(l);
+   double rho = st.mean(3);
    double Ji[3];
 #pragma unroll
    for (int l = 0; l < 3; ++l) {
-      const double* s = f.cellJi + l * N;
-      Ji[l] = 0.125 * (s[c000] + s[c001] + s[c010] + s[c100] + s[c011] + s[c110] + s[c101] + s[c111]);
+      Ji[l] = st.mean(4 + l);
       f.nodeJi[l * N + n] = Ji[l];
    }
    // calcNodeJ (its whistler limiter reads the averaged nodeB and the unclamped nodeRhoQi)
    double Jn[3];
    {
-      const double* fb = f.faceB;
-      const long long a000 = n, a100 = c100, a010 = c010, a001 = c001, a110 = c110, a101 = c101, a011 = c011;
-#define FB(a, l) fb[(l) * N + (a)]
-      const double edgeJx1 = -FB(a000, 2) + FB(a000, 1) + FB(a010, 2) - FB(a001, 1);
-      const double edgeJx2 = -FB(a100, 2) + FB(a100, 1) + FB(a110, 2) - FB(a101, 1);
-      const double edgeJy1 = +FB(a000, 2) + FB(a001, 0) - FB(a100, 2) - FB(a000, 0);
-      const double edgeJy2 = +FB(a010, 2) + FB(a011, 0) - FB(a110, 2) - FB(a010, 0);
-      const double edgeJz1 = -FB(a000, 1) + FB(a000, 0) + FB(a100, 1) - FB(a010, 0);
-      const double edgeJz2 = -FB(a001, 1) + FB(a001, 0) + FB(a101, 1) - FB(a011, 0);
-#undef FB
+      const double edgeJx1 = -st.at(7 + 2, 0, 0, 0) + st.at(7 + 1, 0, 0, 0) + st.at(7 + 2, 0, 1, 0) - st.at(7 + 1, 0, 0, 1);
+      const double edgeJx2 = -st.at(7 + 2, 1, 0, 0) + st.at(7 + 1, 1, 0, 0) + st.at(7 + 2, 1, 1, 0) - st.at(7 + 1, 1, 0, 1);
+      const double edgeJy1 = +st.at(7 + 2, 0, 0, 0) + st.at(7 + 0, 0, 0, 1) - st.at(7 + 2, 1, 0, 0) - st.at(7 + 0, 0, 0, 0);
+      const double edgeJy2 = +st.at(7 + 2, 0, 1, 0) + st.at(7 + 0, 0, 1, 1) - st.at(7 + 2, 1, 1, 0) - st.at(7 + 0, 0, 1, 0);
+      const double edgeJz1 = -st.at(7 + 1, 0, 0, 0) + st.at(7 + 0, 0, 0, 0) + st.at(7 + 1, 1, 0, 0) - st.at(7 + 0, 0, 1, 0);
+      const double edgeJz2 = -st.at(7 + 1, 0, 0, 1) + st.at(7 + 0, 0, 0, 1) + st.at(7 + 1, 1, 0, 1) - st.at(7 + 0, 0, 1, 1);
       double d = 1.0;
       double vw = 0.0;
       const double ne = rho / RHGPU_CHARGE_ELEMENTARY;
@@ -300,9 +302,8 @@ __global__ void __launch_bounds__(128, 8) k_node_fused(GridInfo g, Fields f, Fie
    double B[3];
    if (wsum > 0) {
       for (int l = 0; l < 3; ++l) {
-         const double* cbl = f.cellB + l * N;
-         B[l] = (w111 * cbl[c000] + w112 * cbl[c001] + w121 * cbl[c010] + w211 * cbl[c100] + w122 * cbl[c011] +
-                 w221 * cbl[c110] + w212 * cbl[c101] + w222 * cbl[c111]) / wsum;
+         B[l] = (w111 * st.at(l, 0, 0, 0) + w112 * st.at(l, 0, 0, 1) + w121 * st.at(l, 0, 1, 0) + w211 * st.at(l, 1, 0, 0) +
+                 w122 * st.at(l, 0, 1, 1) + w221 * st.at(l, 1, 1, 0) + w212 * st.at(l, 1, 0, 1) + w222 * st.at(l, 1, 1, 1)) / wsum;
       }
    } else {
       B[0] = B[1] = B[2] = 0.0;
@@ -313,7 +314,6 @@ __global__ void __launch_bounds__(128, 8) k_node_fused(GridInfo g, Fields f, Fie
    E[0] = -(Ue[1] * B[2] - Ue[2] * B[1]);
    E[1] = -(Ue[2] * B[0] - Ue[0] * B[2]);
    E[2] = -(Ue[0] * B[1] - Ue[1] * B[0]);
-   const double eta = f.nodeEta[n];
    E[0] += eta * Jn[0];
    E[1] += eta * Jn[1];
    E[2] += eta * Jn[2];
@@ -329,6 +329,48 @@ __global__ void __launch_bounds__(128, 8) k_node_fused(GridInfo g, Fields f, Fie
    countIf(eClamp, &cnt[CNT_MAX_E]);
    gridCount(f, GC_NODE_MAX_E, N, n, eClamp);
    for (int l = 0; l < 3; ++l) f.nodeE[l * N + n] = E[l];
+}
+
+__device__ __forceinline__ void ndStage(const GridInfo& g, const Fields& f, double* dst, int i0, int j0, int kz) {
+   const long long N = g.N;
+   stageLayer<ND_ARR, ND_Y>(
+       g,
+       [&](int a) {
+          return a < 3 ? f.cellB + a * N : a == 3 ? f.cellRho : a < 7 ? f.cellJi + (a - 4) * N : f.faceB + (a - 7) * N;
+       },
+       f.faceB, dst, i0, j0, kz);
+}
+
+__global__ void __launch_bounds__(32 * ND_Y, 3) k_node_fused(GridInfo g, Fields f, FieldParams fp, int nzb, unsigned long long* cnt) {
+   extern __shared__ __align__(16) double ndLayers[];
+   const int i0 = blockIdx.x * NT_X, j0 = blockIdx.y * ND_Y, k0 = blockIdx.z * nzb;
+   const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+   const int nk = min(nzb, g.nz - k0);
+   const bool mine = i < g.nx && j < g.ny;
+   ndStage(g, f, ndLayers, i0, j0, k0);
+   ndStage(g, f, ndLayers + ND_LAYER, i0, j0, k0 + 1);
+   cpAsyncCommit();
+   if (nk > 1) ndStage(g, f, ndLayers + 2 * ND_LAYER, i0, j0, k0 + 2);
+   cpAsyncCommit();
+   int a = 0, b = 1;   // slots of layers k and k + 1
+   for (int t = 0; t < nk; ++t) {
+      const int k = k0 + t;
+      const long long n = mine ? cidx(g, i, j, k) : 0;
+      // the node's own values, on their way during the wait for the layers
+      const double avg[3] = {f.cellAvgB[n], f.cellAvgB[g.N + n], f.cellAvgB[2 * g.N + n]}, eta = f.nodeEta[n];
+      cpAsyncWaitGroup<1>();   // cell layers k and k + 1 are in
+      __syncthreads();
+      NodeStencil st;
+      st.L = ndLayers + a * ND_LAYER;
+      st.U = ndLayers + b * ND_LAYER;
+      st.off = threadIdx.y * NT_LX + threadIdx.x;
+      if (mine) nodeFromStencil(g, f, fp, cnt, i, j, k, n, st, avg, eta);
+      __syncthreads();         // layer k is read by every thread: its slot takes layer k + 3
+      if (t + 2 < nk) ndStage(g, f, ndLayers + a * ND_LAYER, i0, j0, k + 3);
+      cpAsyncCommit();
+      a = b;
+      b = b == 2 ? 0 : b + 1;
+   }
 }
 
 }  // namespace rh

@@ -128,33 +128,46 @@ __global__ void k_faraday(GridInfo g, Fields f);
 //                 nodeJi), calcNodeJ (edge curls of faceB / (2 dx mu0 d), the
 //                 whistler limiter d), then calcNodeUe, upwindNodeB and calcNodeE;
 //                 the averaged nodeB that the whistler limiter reads stays in
-//                 registers, the upwind weights re-read the same eight cells
+//                 registers, the upwind weights re-read the same eight cells (staged)
 //   k_cell_tiled  per cell: node2Cell of nodeJ and calcCellUe, calcCellEp (the
 //                 gradient of face-averaged nodeRhoQi), and (FARADAY: no E
 //                 smoothing) faceCurl, faceB += dt curl E; none of them reads
 //                 what another writes
-// k_cell_tiled reads its eight-point stencils from node layers staged in shared
-// memory. The node pass reads its cells directly: its FP64 work per node (eight
-// square roots and divisions) keeps it issue-bound, and a staged version with
-// fewer resident warps took 0.42 ms against 0.33 ms for this one.
+// Both read their eight-point stencils from layers staged in shared memory, and
+// what a thread reads of its own cell or node is requested before it waits.
 // The cellUe Neumann pass (k_ext_cell_neumann3) follows k_cell_tiled; calcNodeUe
 // and calcNodeE do not read cellUe, so its place before them in the reference's
 // order does not matter.
 __global__ void k_ext_bc(GridInfo g, Fields f, FieldParams fp, const int* ext, int next);
-
-__global__ void __launch_bounds__(128, 8) k_node_fused(GridInfo g, Fields f, FieldParams fp, unsigned long long* cnt);
 
 // ---- the cell pass, its node stencil in shared memory ------------------------------------------
 // A block of 32 x 4 cells marches nzb planes along z; the node layers k - 1
 // and k that a plane of cells reads (nodeJ, nodeRhoQi, nodeE over 33 x 5 nodes
 // from (i0 - 1, j0 - 1)) sit in a ring of three layer slots, the next one
 // copied in with cp.async while the current plane is computed, so every node
-// value is loaded once per block instead of once per cell reading it.
+// value is loaded once per block instead of once per cell reading it. 120 x 160
+// x 160 cells: 136 us (4.7 TB/s of what it must move); 240 us with the cell's own
+// values loaded where they are used, 257 us with each staged value's place also
+// worked out by itself.
 constexpr int NT_X = 32, NT_Y = 4, NT_Z = 8;   // NT_Z: most planes of a block
 constexpr int NT_LX = NT_X + 1, NT_LY = NT_Y + 1;
 constexpr int CT_ARR = 7;    // nodeJ x 3, nodeRhoQi, nodeE x 3
 constexpr int CT_LAYER = CT_ARR * NT_LY * NT_LX;
 constexpr size_t CT_SMEM = 3 * CT_LAYER * sizeof(double);
+
+// The node pass: a block of 32 x ND_Y nodes marches nzb planes along z, the cell
+// layers k and k + 1 that a plane of nodes reads (cellB, cellRhoQi, cellJi, faceB
+// over 33 x (ND_Y + 1) cells from (i0, j0)) in a ring of three layer slots, the
+// next one copied in while the current plane is computed. It is bound by its
+// 16 IEEE square roots and divisions per node and the waits around them at the 24
+// warps per SM that 71 KB of layers leave. 120 x 160 x 160 nodes: 258 us; 326 us
+// with every value read from L1 and L2 by itself; 288 us without the early loads;
+// 308 us with 32 x 4 blocks; 275 us with rsqrt and Newton steps for the weights.
+constexpr int ND_Y = 8;
+constexpr int ND_ARR = 10;   // cellB x 3, cellRhoQi, cellJi x 3, faceB x 3
+constexpr int ND_LAYER = ND_ARR * (ND_Y + 1) * 33;
+constexpr size_t ND_SMEM = 3 * ND_LAYER * sizeof(double);
+__global__ void __launch_bounds__(32 * ND_Y, 3) k_node_fused(GridInfo g, Fields f, FieldParams fp, int nzb, unsigned long long* cnt);
 
 // node (dx, dy, dz) in {-1, 0}^3 of a cell's stencil, o = (dx + 1) + 2 (dy + 1) + 4 (dz + 1)
 struct CellStencil {
@@ -169,23 +182,67 @@ struct CellStencil {
    __device__ __forceinline__ double ne(int l, int o) const { return at(4 + l, o); }
 };
 
-__device__ __forceinline__ void ctStage(const GridInfo& g, const Fields& f, double* dst, int i0, int j0, int kz) {
-   int z = kz;
+// One layer z of NA arrays into shared memory with cp.async, values 0 where the
+// box has no cell: (32 + 1) x (TY + 1) values from (x0, y0), row (a, y) at (a * (TY
+// + 1) + y) * NT_LX. The block is 32 x TY threads; a warp copies its own y row of
+// every array with one offset, then the row TY of arrays ty, ty + TY, ...; the
+// last column goes to one thread per row. `arr(a)` is array a at cell 0.
+template <int NA, int TY, class ARR>
+__device__ __forceinline__ void stageLayer(const GridInfo& g, const ARR& arr, const double* none, double* dst, int x0,
+                                           int y0, int z) {
+   const int tx = threadIdx.x, ty = threadIdx.y;
    const bool zok = wrapc(z, g.nz, g.per[2]);
-   const long long N = g.N;
-   for (int e = threadIdx.x + NT_X * threadIdx.y; e < CT_LAYER; e += NT_X * NT_Y) {
-      const int a = e / (NT_LY * NT_LX), r = e - a * (NT_LY * NT_LX), jj = r / NT_LX, ii = r - jj * NT_LX;
-      int x = i0 - 1 + ii, y = j0 - 1 + jj;
-      const bool ok = zok && wrapc(x, g.nx, g.per[0]) && wrapc(y, g.ny, g.per[1]);
-      const double* arr = a < 3 ? f.nodeJ + a * N : a == 3 ? f.nodeRho : f.nodeE + (a - 4) * N;
-      cpAsync8(dst + e, ok ? arr + cidx(g, x, y, z) : f.faceB, ok ? 8 : 0);
+   int x = x0 + tx, y = y0 + ty, yl = y0 + TY;
+   const bool xok = wrapc(x, g.nx, g.per[0]) && zok;
+   const bool ok = wrapc(y, g.ny, g.per[1]) && xok, okl = wrapc(yl, g.ny, g.per[1]) && xok;
+   const int plane = g.nx * g.ny * z;
+   const int off = x + g.nx * y + plane, offl = x + g.nx * yl + plane;
+#pragma unroll
+   for (int a = 0; a < NA; ++a)
+      cpAsync8(dst + (a * (TY + 1) + ty) * NT_LX + tx, ok ? arr(a) + off : none, ok ? 8 : 0);
+#pragma unroll
+   for (int a0 = 0; a0 < NA; a0 += TY) {
+      const int a = a0 + ty;
+      if (a < NA) cpAsync8(dst + (a * (TY + 1) + TY) * NT_LX + tx, okl ? arr(a) + offl : none, okl ? 8 : 0);
+   }
+   const int r = tx + NT_X * ty;
+   if (r < NA * (TY + 1)) {
+      const int a = r / (TY + 1);
+      int xc = x0 + NT_X, yc = y0 + r - a * (TY + 1);
+      const bool okc = wrapc(xc, g.nx, g.per[0]) && wrapc(yc, g.ny, g.per[1]) && zok;
+      cpAsync8(dst + r * NT_LX + NT_X, okc ? arr(a) + (xc + g.nx * yc + plane) : none, okc ? 8 : 0);
    }
 }
+
+// the cell pass's node layer kz from (i0 - 1, j0 - 1)
+__device__ __forceinline__ void ctStage(const GridInfo& g, const Fields& f, double* dst, int i0, int j0, int kz) {
+   const long long N = g.N;
+   stageLayer<CT_ARR, NT_Y>(
+       g, [&](int a) { return a < 3 ? f.nodeJ + a * N : a == 3 ? f.nodeRho : f.nodeE + (a - 4) * N; }, f.faceB, dst, i0 - 1,
+       j0 - 1, kz);
+}
+
+// a cell's own values, loaded a plane ahead of their use
+template <bool FARADAY>
+struct CellOwn {
+   double rho, ji[3], fB[3];
+   unsigned char fl;
+   __device__ __forceinline__ void load(const Fields& f, long long N, long long n) {
+      rho = f.cellRho[n];
+#pragma unroll
+      for (int l = 0; l < 3; ++l) ji[l] = f.cellJi[l * N + n];
+      if (FARADAY) {
+#pragma unroll
+         for (int l = 0; l < 3; ++l) fB[l] = f.faceB[l * N + n];
+      }
+      fl = f.flags[n];
+   }
+};
 
 template <bool FARADAY>
 __device__ __forceinline__ void cellFromStencil(const GridInfo& g, const Fields& f, const FieldParams& fp, int useEp,
                                                 unsigned long long* cnt, int i, int j, int k, long long n,
-                                                const CellStencil& st) {
+                                                const CellStencil& st, const CellOwn<FARADAY>& own) {
    const long long N = g.N;
    const bool inner = allNb(g, i, j, k);
    bool clamp = false;
@@ -199,15 +256,15 @@ __device__ __forceinline__ void cellFromStencil(const GridInfo& g, const Fields&
          f.cellJ[l * N + n] = J[l];
       }
       double Ue[3];
-      const unsigned char fl = f.flags[n];
+      const unsigned char fl = own.fl;
       if (fl & RHGPU_FLAG_INNER_FIELD) {
          for (int l = 0; l < 3; ++l) Ue[l] = fp.obstacleUe[l];
       } else {
-         const double rho = f.cellRho[n];
+         const double rho = own.rho;
          for (int l = 0; l < 3; ++l) {
             if (fabs(rho) > 0) {
-               if (fp.use_hall) Ue[l] = -(J[l] - f.cellJi[l * N + n]) / rho;
-               else Ue[l] = f.cellJi[l * N + n] / rho;
+               if (fp.use_hall) Ue[l] = -(J[l] - own.ji[l]) / rho;
+               else Ue[l] = own.ji[l] / rho;
             } else {
                Ue[l] = 0.0;
             }
@@ -235,8 +292,8 @@ __device__ __forceinline__ void cellFromStencil(const GridInfo& g, const Fields&
             const double C = fp.ep_coeff;
             if (!fp.isothermal) {
                Ep[0] = -C * gx; Ep[1] = -C * gy; Ep[2] = -C * gz;
-            } else if (fabs(f.cellRho[n]) > 0) {
-               const double rho = f.cellRho[n];
+            } else if (fabs(own.rho) > 0) {
+               const double rho = own.rho;
                Ep[0] = -C * gx / rho; Ep[1] = -C * gy / rho; Ep[2] = -C * gz / rho;
             }
          }
@@ -260,21 +317,21 @@ __device__ __forceinline__ void cellFromStencil(const GridInfo& g, const Fields&
       const double n5y = st.ne(1, s5), n5z = st.ne(2, s5), n6y = st.ne(1, s6), n6z = st.ne(2, s6);
       const double n7y = st.ne(1, s7), n7z = st.ne(2, s7), n8y = st.ne(1, s8), n8z = st.ne(2, s8);
       const double curlX = 0.5 * (+n5z + n6z - n6y - n7y - n7z - n8z + n8y + n5y) / dx;
-      f.faceB[0 * N + n] += dt * curlX;
+      f.faceB[0 * N + n] = own.fB[0] + dt * curlX;
    }
    if (doY) {
       constexpr int s3 = 2, s4 = 6, s7 = 3, s8 = 7;
       const double n3x = st.ne(0, s3), n3z = st.ne(2, s3), n4x = st.ne(0, s4), n4z = st.ne(2, s4);
       const double n7x = st.ne(0, s7), n7z = st.ne(2, s7), n8x = st.ne(0, s8), n8z = st.ne(2, s8);
       const double curlY = 0.5 * (-n4x - n8x + n8z + n7z + n7x + n3x - n3z - n4z) / dx;
-      f.faceB[1 * N + n] += dt * curlY;
+      f.faceB[1 * N + n] = own.fB[1] + dt * curlY;
    }
    if (doZ) {
       constexpr int s1 = 4, s4 = 6, s5 = 5, s8 = 7;
       const double n1x = st.ne(0, s1), n1y = st.ne(1, s1), n4x = st.ne(0, s4), n4y = st.ne(1, s4);
       const double n5x = st.ne(0, s5), n5y = st.ne(1, s5), n8x = st.ne(0, s8), n8y = st.ne(1, s8);
       const double curlZ = 0.5 * (-n1x - n5x - n5y - n8y + n8x + n4x + n4y + n1y) / dx;
-      f.faceB[2 * N + n] += dt * curlZ;
+      f.faceB[2 * N + n] = own.fB[2] + dt * curlZ;
    }
 }
 
@@ -283,15 +340,15 @@ __device__ __forceinline__ void cellFromStencil(const GridInfo& g, const Fields&
 // the layer shared with the next block but is a plane more in a serial march.
 // (32^3 cells, 32 blocks of 8 planes: 60 us; 256 blocks of one: 17 us. 61 x 83 x
 // 70 cells: 62 -> 40 us. Grids that fill a wave with 8 planes keep them.)
-inline int cellPlanes(const GridInfo& g) {
-   const long long cols = (long long)((g.nx + NT_X - 1) / NT_X) * ((g.ny + NT_Y - 1) / NT_Y);
+inline int layerPlanes(const GridInfo& g, int ty) {
+   const long long cols = (long long)((g.nx + NT_X - 1) / NT_X) * ((g.ny + ty - 1) / ty);
    int nzb = NT_Z;
    while (nzb > 1 && cols * ((g.nz + nzb - 1) / nzb) < 148 * 8) nzb >>= 1;
    return nzb;
 }
 
 template <bool FARADAY>
-__global__ void __launch_bounds__(NT_X * NT_Y) k_cell_tiled(GridInfo g, Fields f, FieldParams fp, int useEp,
+__global__ void __launch_bounds__(NT_X * NT_Y, 6) k_cell_tiled(GridInfo g, Fields f, FieldParams fp, int useEp,
                                                             int nzb, unsigned long long* cnt) {
    extern __shared__ __align__(16) double ctLayers[];
    const int tx = threadIdx.x, ty = threadIdx.y;
@@ -299,6 +356,8 @@ __global__ void __launch_bounds__(NT_X * NT_Y) k_cell_tiled(GridInfo g, Fields f
    const int i = i0 + tx, j = j0 + ty;
    const int nk = min(nzb, g.nz - k0);
    const bool mine = i < g.nx && j < g.ny;
+   CellOwn<FARADAY> own, next;
+   if (mine) own.load(f, g.N, cidx(g, i, j, k0));
    ctStage(g, f, ctLayers, i0, j0, k0 - 1);
    ctStage(g, f, ctLayers + CT_LAYER, i0, j0, k0);
    cpAsyncCommit();
@@ -312,7 +371,9 @@ __global__ void __launch_bounds__(NT_X * NT_Y) k_cell_tiled(GridInfo g, Fields f
       st.U = ctLayers + ((t + 1) % 3) * CT_LAYER;
       st.off = ty * NT_LX + tx;
       const int k = k0 + t;
-      if (mine) cellFromStencil<FARADAY>(g, f, fp, useEp, cnt, i, j, k, cidx(g, i, j, k), st);
+      if (mine && t + 1 < nk) next.load(f, g.N, cidx(g, i, j, k + 1));
+      if (mine) cellFromStencil<FARADAY>(g, f, fp, useEp, cnt, i, j, k, cidx(g, i, j, k), st, own);
+      own = next;
       __syncthreads();         // layer k - 1 is read by every thread: its slot takes layer k + 2
       if (t + 3 <= nk) ctStage(g, f, ctLayers + (t % 3) * CT_LAYER, i0, j0, k0 + t + 2);
       cpAsyncCommit();

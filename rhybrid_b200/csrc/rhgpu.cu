@@ -176,6 +176,18 @@ int ensureKeyCapacity(rhgpu_ctx* c, long long n) {
    return RHGPU_OK;
 }
 
+// k_node_fused uses more than the 48 KB of static shared memory: its limit is
+// raised once per device
+int raiseNodeSmem(const rhgpu_ctx* c) {
+   static std::atomic<bool> raised[64] = {};
+   if (c->device < 0 || c->device >= 64) return fail(RHGPU_ERR_CUDA, "device index out of range");
+   if (!raised[c->device].load()) {
+      RH_CUDA(cudaFuncSetAttribute(k_node_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ND_SMEM));
+      raised[c->device].store(true);
+   }
+   return RHGPU_OK;
+}
+
 #define RH_FIELD_LAUNCH(name, grid, block, ...)              \
    do {                                                      \
       RH_TIME(c, #name);                                     \
@@ -193,11 +205,18 @@ int fieldsAll(rhgpu_ctx* c) {
    const bool smooth = c->P.n_linear_smoothings_nodeE > 0 || c->P.use_gaussian_smoothing_nodeE;
    RH_FIELD_LAUNCH(k_face2cell, G, B, g, c->f);
    if (c->next > 0) RH_FIELD_LAUNCH(k_ext_bc, EB, 128, g, c->f, c->fp, c->ext, c->next);
-   RH_FIELD_LAUNCH(k_node_fused, G, B, g, c->f, c->fp, c->cntU);
+   {
+      RH_TIME(c, "k_node_fused");
+      const int nzb = layerPlanes(g, ND_Y);
+      const dim3 NG((g.nx + NT_X - 1) / NT_X, (g.ny + ND_Y - 1) / ND_Y, (g.nz + nzb - 1) / nzb);
+      if (const int rc = raiseNodeSmem(c)) return rc;
+      k_node_fused<<<NG, dim3(NT_X, ND_Y), ND_SMEM, c->stream>>>(g, c->f, c->fp, nzb, c->cntU);
+      RH_LAUNCHED(c);
+   }
    c->gridAvgCounter += 1;
    {
       RH_TIME(c, "k_cell_tiled");
-      const int nzb = cellPlanes(g);
+      const int nzb = layerPlanes(g, NT_Y);
       const dim3 NG((g.nx + NT_X - 1) / NT_X, (g.ny + NT_Y - 1) / NT_Y, (g.nz + nzb - 1) / nzb);
       if (smooth)
          k_cell_tiled<false><<<NG, dim3(NT_X, NT_Y), CT_SMEM, c->stream>>>(g, c->f, c->fp, c->P.use_electron_pressure,
