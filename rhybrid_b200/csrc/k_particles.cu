@@ -1,6 +1,7 @@
 // Definitions of the kernels declared in k_particles.cuh (each declaration there says
 // what its kernel does); the template kernels stay in the header.
 #include "k_particles.cuh"
+#include "k_fast.cuh"
 
 namespace rh {
 
@@ -141,35 +142,31 @@ __global__ void k_set_alive_from_count(long long N, const long long* cnt, int* a
 }
 
 __global__ void __launch_bounds__(32 * DEP_WARPS, 4) k_deposit_cell(GridInfo g, PStore P, double q, double* S, unsigned* err) {
-   __shared__ double sw[DEP_WARPS][32][11];                // w8[0..7], v[0..2] of a batch's particles
-   __shared__ int soct[DEP_WARPS][32];                     // octant (i + 2j + 4k) of the corner-000 entry, 8 if invalid
-   __shared__ double stage[DEP_WARPS][DEP_ENTRIES + 1];    // the group's sums, per cell
+   // entry (a, b, c) of the 3x3x3 sums at (a + 6 b + 18 c) * 4: the corners of a
+   // particle's lower and upper four entries fall on different banks
+   constexpr int ROW = 6, PLANE = 18, SUMS = 3 * PLANE * 4;
+   __shared__ double sw[DEP_WARPS][32][13];      // w8[0..7], then 1, vx, vy, vz of a batch's particles
+   __shared__ int sat[DEP_WARPS][32];            // the corner-000 entry's place in the sums, -1 if invalid
+   __shared__ double sums[DEP_WARPS][SUMS];
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   // per entry t: its value (-1 charge, 0..2 current) and its corner map,
-   // nibble o = the corner of a particle of octant o landing on the entry, 8
-   // for none (nibble 8: a particle without a valid octant)
-   unsigned long long cmap[4];
-   int el[4];
-   const int ne = lane < 12 ? 4 : 3;
+   const int corner = lane >> 2, moment = lane & 3;
+   double* const acc = sums[warp] + ((corner & 1) + ROW * ((corner >> 1) & 1) + PLANE * (corner >> 2)) * 4 + moment;
+   // the entries that this thread writes out (rows threadIdx.x / 8 + 32 k of cell threadIdx.x % 8)
+   const int ow = threadIdx.x % DEP_WARPS;
+   int place[4];
 #pragma unroll
-   for (int t = 0; t < 4; ++t) {
-      const int e = lane + 32 * t;
-      int ind, l;
-      if (e < 27) { ind = e; l = -1; } else { ind = (e - 27) / 3; l = (e - 27) % 3; }
-      const int ea = ind % 3, eb = (ind / 3) % 3, ec = ind / 9;
-      unsigned long long m = 8ull << 32;
-      for (int o = 0; o < 8; ++o) {
-         const int ox = ea - (o & 1), oy = eb - ((o >> 1) & 1), oz = ec - (o >> 2);
-         const bool on = (unsigned)ox <= 1u && (unsigned)oy <= 1u && (unsigned)oz <= 1u;
-         m |= (unsigned long long)(on ? ox + 2 * oy + 4 * oz : 8) << (4 * o);
-      }
-      cmap[t] = m;
-      el[t] = l;
+   for (int k = 0; k < 4; ++k) {
+      const int e = threadIdx.x / DEP_WARPS + 32 * k;
+      const int ind = e < 27 ? e : (e - 27) / 3, m = e < 27 ? 0 : 1 + (e - 27) % 3;
+      place[k] = e < DEP_ENTRIES ? (ind % 3 + ROW * ((ind / 3) % 3) + PLANE * (ind / 9)) * 4 + m : -1;
    }
+   for (int e = lane; e < SUMS; e += 32) sums[warp][e] = 0.0;
+   __syncwarp();
+   const double hdx = 0.5 * g.dx;
+   const unsigned long long inCell = (unsigned long long)__double_as_longlong(g.dx);   // bits of [0, dx) are below
    const long long groups = (g.N + DEP_WARPS - 1) / DEP_WARPS;
    for (long long grp = blockIdx.x; grp < groups; grp += gridDim.x) {
       const long long c = grp * DEP_WARPS + warp;
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
       if (c < g.N) {
          const long long a0 = P.start[c];
          const int na = P.alive[c];
@@ -180,44 +177,44 @@ __global__ void __launch_bounds__(32 * DEP_WARPS, 4) k_deposit_cell(GridInfo g, 
                const double x = P.a[0][p], y = P.a[1][p], z = P.a[2][p];
                const double wq = P.a[6][p] * q;
                double w8[8];
-               int ind[8];
-               cicWeights(x, y, z, wq, g, w8, ind);
-               int oct = 8;
-               const int i0 = ind[0] % 3, j0 = (ind[0] / 3) % 3, k0 = ind[0] / 9;
-               if (ind[0] >= 0 && ind[0] < 27 && i0 <= 1 && j0 <= 1 && k0 <= 1) oct = i0 + 2 * j0 + 4 * k0;
-               else raiseError(err, RHGPU_DEVERR_NAN_PARTICLE);
+               int at = -1;
+               if ((unsigned long long)__double_as_longlong(x) < inCell && (unsigned long long)__double_as_longlong(y) < inCell &&
+                   (unsigned long long)__double_as_longlong(z) < inCell) {
+                  cicWeightsLocal(x, y, z, wq, g, w8);   // as after a migration: the octant is the half of each axis
+                  at = ((x < hdx ? 0 : 1) + ROW * (y < hdx ? 0 : 1) + PLANE * (z < hdx ? 0 : 1)) * 4;
+               } else {
+                  int ind[8];
+                  cicWeights(x, y, z, wq, g, w8, ind);
+                  const int i0 = ind[0] % 3, j0 = (ind[0] / 3) % 3, k0 = ind[0] / 9;
+                  if (ind[0] >= 0 && ind[0] < 27 && i0 <= 1 && j0 <= 1 && k0 <= 1) at = (i0 + ROW * j0 + PLANE * k0) * 4;
+                  else raiseError(err, RHGPU_DEVERR_NAN_PARTICLE);
+               }
 #pragma unroll
                for (int o = 0; o < 8; ++o) sw[warp][lane][o] = w8[o];
-               sw[warp][lane][8] = P.a[3][p];
-               sw[warp][lane][9] = P.a[4][p];
-               sw[warp][lane][10] = P.a[5][p];
-               soct[warp][lane] = oct;
+               sw[warp][lane][8] = 1.0;
+               sw[warp][lane][9] = P.a[3][p];
+               sw[warp][lane][10] = P.a[4][p];
+               sw[warp][lane][11] = P.a[5][p];
+               sat[warp][lane] = at;
             }
             __syncwarp();
-#pragma unroll 2
+#pragma unroll 4
             for (int j = 0; j < nb; ++j) {
-               const int sh = 4 * soct[warp][j];
-               const double* r = sw[warp][j];
-#pragma unroll
-               for (int t = 0; t < 4; ++t) {
-                  if (t >= ne) break;
-                  const unsigned corner = (unsigned)(cmap[t] >> sh) & 15u;
-                  const double w = r[corner & 7u];
-                  const double v = el[t] < 0 ? w : w * r[8 + (el[t] < 0 ? 0 : el[t])];
-                  acc[t] += corner < 8u ? v : 0.0;
-               }
+               const double v = sw[warp][j][corner] * sw[warp][j][8 + moment];
+               const int at = sat[warp][j];
+               if (at >= 0) acc[at] += v;   // lanes own their entries of this particle
+               __syncwarp();                // the next particle's lanes may own them differently
             }
-            __syncwarp();
          }
       }
-#pragma unroll
-      for (int t = 0; t < 4; ++t)
-         if (t < ne) stage[warp][lane + 32 * t] = acc[t];
       __syncthreads();
-      for (int idx = threadIdx.x; idx < DEP_ENTRIES * DEP_WARPS; idx += 32 * DEP_WARPS) {
-         const int e = idx / DEP_WARPS, w = idx - e * DEP_WARPS;
-         const long long cc = grp * DEP_WARPS + w;
-         if (cc < g.N) S[(long long)e * g.N + cc] = stage[w][e];
+      const long long cc = grp * DEP_WARPS + ow;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+         if (place[k] < 0) continue;
+         double* const p = &sums[ow][place[k]];
+         if (cc < g.N) S[(long long)(threadIdx.x / DEP_WARPS + 32 * k) * g.N + cc] = *p;
+         *p = 0.0;
       }
       __syncthreads();
    }

@@ -83,22 +83,19 @@ __device__ inline void cicWeights(double x, double y, double z, double wq, const
 }
 
 // Per cell, the 3x3x3 CIC sums of accumulateCell in particle order, one warp
-// per cell: lane L owns the accumulator entries e = L, L+32, L+64, L+96
-// (e < 27: charge of 3x3x3 entry e; e = 27 + 3*entry + l: current l). The
-// particles of the cell are taken 32 at a time, each lane computing one
-// particle's CIC weights into shared memory; then every lane walks those
-// particles in order and adds the contribution that falls on its entries, so
-// each entry is the same sequential sum as in the reference. Each entry keeps
-// a map from the particle's octant (the 3x3x3 index of its corner 000 is one
-// of the 8 of {0,1}^3) to the corner landing on the entry, or none; an entry
-// no corner lands on adds +0.0, which leaves every sum unchanged (a sum that
-// starts at +0.0 is never -0.0, so x + 0.0 == x for each of its values), so
-// the walk has no branches and each sum is still the reference's sequence.
-// S[e*N + c] receives the 108 sums of cell c. A block takes DEP_WARPS
-// consecutive cells at a time (one per warp) and writes their sums row by row
-// through shared memory, DEP_WARPS cells contiguous per row; the blocks, one
-// resident wave of DEP_GRID, stride over the groups of cells, so each warp
-// builds its corner maps once.
+// per cell: a particle contributes to 8 of the 27 entries, charge and three
+// currents each, one product per lane (lane = 4 corner + moment). The sums stay
+// in shared memory, so that a particle costs a warp two operand loads, a
+// product and one read-add-write; each entry's sum is the same sequence of
+// additions as in the reference. The particles of the cell are taken 32 at a
+// time, each lane computing one particle's CIC weights into shared memory.
+// S[e*N + c] receives the 108 sums of cell c (e < 27: charge of entry e; e = 27 +
+// 3*entry + l: current l). A block takes DEP_WARPS consecutive cells at a time
+// (one per warp) and writes their sums row by row, DEP_WARPS cells contiguous
+// per row; the blocks, one resident wave of DEP_GRID, stride over the groups of
+// cells. 64 x 48 x 40 cells of 20 ions: 161 us; 250 us with the 108 sums held in
+// registers, four per lane, every lane adding a contribution or +0.0 for every
+// particle.
 constexpr int DEP_WARPS = 8;
 constexpr int DEP_ENTRIES = 108;
 constexpr int DEP_GRID = 148 * 4;   // 4 blocks of 256 threads at 64 registers per SM
