@@ -106,8 +106,8 @@ __host__ __device__ inline double dnJFactor(int vel, double rsj, double rho) {
 // TRANSPOSED, the data gradient with mirrored taps and W transposed, no bias,
 // masked by the ReLU derivative.
 //
-// A block owns a column of 30 x 8 output voxels in (x, y) and TC_ZC of its
-// z-slices. Input z-slices of 32 x-positions x 10 y-rows (one voxel of halo
+// A block owns a column of 30 x 8 output voxels in (x, y) and zc of its
+// z-slices (tcSlices). Input z-slices of 32 x-positions x 10 y-rows (one voxel of halo
 // each side) stream through a ring of 4 slots in shared memory, one plane per
 // 8-channel half with 16 bytes per voxel: any run of positions is a K-major,
 // unswizzled UMMA operand (core matrices of 8 consecutive positions x 16 bytes,
@@ -137,7 +137,7 @@ __host__ __device__ inline double dnJFactor(int vel, double rsj, double rho) {
 // mbarrier wait is bounded: on expiry the kernel raises RHGPU_DEVERR_DENOISER
 // in `err`, stops issuing, waits (bounded again) for the last commit of the
 // MMAs it issued, and still frees its tensor memory.
-constexpr int TC_HX = 32, TC_BY = 8, TC_ZC = 8;
+constexpr int TC_HX = 32, TC_BY = 8;
 constexpr int TC_HY = TC_BY + 2;
 constexpr int TC_BX = TC_HX - 2;                             // output voxels per x-row
 constexpr int TC_SPOS = TC_HX * TC_HY;                       // positions of one staged slice
@@ -350,15 +350,32 @@ __device__ __forceinline__ void tcIssue(unsigned tmem, unsigned aHi, unsigned aL
    }
 }
 
+// output slices per block: a block's time goes with its input slices, two more
+// than these, and its set-up (about three slices'), and the blocks run in waves of
+// 4 per SM, so the number with the shortest waves x slices is taken: at 64^3
+// voxels 3 (a training iteration 0.40 -> 0.36 ms, with 8 only 192 blocks ran), at
+// 120 x 160 x 160 12 (the three layers of a step 469 -> 451 us).
+inline int tcSlices(const DnGrid& g) {
+   const long long cols = (long long)((g.nx + TC_BX - 1) / TC_BX) * ((g.ny + TC_BY - 1) / TC_BY);
+   int best = 1;
+   long long least = -1;
+   for (int zc = 1; zc <= 16; ++zc) {
+      const long long waves = (cols * ((g.nz + zc - 1) / zc) + 4 * 148 - 1) / (4 * 148);
+      const long long cost = waves * (zc + 5);
+      if (least < 0 || cost <= least) { least = cost; best = zc; }
+   }
+   return best;
+}
+
 template <bool TRANSPOSED>
 __global__ void __launch_bounds__(TC_THREADS)
-k_dn_conv_tc(DnGrid g, const unsigned* in, const __nv_bfloat16* bimg, const float* bias, int mode, unsigned* out,
+k_dn_conv_tc(DnGrid g, int zc, const unsigned* in, const __nv_bfloat16* bimg, const float* bias, int mode, unsigned* out,
              const unsigned* mask, float* out32, const float* res, DnMoments mom, unsigned* err) {
    extern __shared__ __align__(16) unsigned char tcSmemRaw[];
    TcShared& sh = *reinterpret_cast<TcShared*>(tcSmemRaw);
    const int tid = threadIdx.x, warp = tid >> 5;
-   const int x0 = blockIdx.x * TC_BX, y0 = blockIdx.y * TC_BY, z0 = blockIdx.z * TC_ZC;
-   const int nzc = min(TC_ZC, g.nz - z0);
+   const int x0 = blockIdx.x * TC_BX, y0 = blockIdx.y * TC_BY, z0 = blockIdx.z * zc;
+   const int nzc = min(zc, g.nz - z0);
    const int nin = nzc + 2;   // input slices z0 - 1 .. z0 + nzc; input i is slice z0 - 1 + i, in slot i % 4
    const unsigned planeBase = (unsigned)__cvta_generic_to_shared(&sh.plane[0][0]);
    const unsigned bimgBase = (unsigned)__cvta_generic_to_shared(&sh.bimg[0]);

@@ -26,13 +26,14 @@ int dnConv(rhgpu_dn* d, cudaStream_t st, bool transposed, int l, const unsigned*
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
       raised[d->device][transposed] = true;
    }
+   const int zc = tcSlices(d->g);
    const dim3 grid((unsigned)((d->g.nx + TC_BX - 1) / TC_BX), (unsigned)((d->g.ny + TC_BY - 1) / TC_BY),
-                   (unsigned)((d->g.nz + TC_ZC - 1) / TC_ZC));
+                   (unsigned)((d->g.nz + zc - 1) / zc));
    const __nv_bfloat16* img = d->bimg + (size_t)((transposed ? 3 : 0) + l) * (TC_BIMG / 2);
    if (transposed)
-      k_dn_conv_tc<true><<<grid, TC_THREADS, TC_SMEM, st>>>(d->g, in, img, bias, mode, out, mask, out32, res, mom, err);
+      k_dn_conv_tc<true><<<grid, TC_THREADS, TC_SMEM, st>>>(d->g, zc, in, img, bias, mode, out, mask, out32, res, mom, err);
    else
-      k_dn_conv_tc<false><<<grid, TC_THREADS, TC_SMEM, st>>>(d->g, in, img, bias, mode, out, mask, out32, res, mom, err);
+      k_dn_conv_tc<false><<<grid, TC_THREADS, TC_SMEM, st>>>(d->g, zc, in, img, bias, mode, out, mask, out32, res, mom, err);
    RH_CUDA(cudaGetLastError());
    return RHGPU_OK;
 }

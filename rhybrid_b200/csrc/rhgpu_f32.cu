@@ -218,11 +218,11 @@ int f32Upload(rhgpu_ctx* c, int s, const uint32_t* counts, const double* particl
       k_iota<<<blocks1d(n, 256), 256, 0, c->stream>>>(idxIn, n);
       RH_CUDA(cudaGetLastError());
       size_t sb = 0;
-      cub::DeviceRadixSort::SortPairs(nullptr, sb, keyIn, keyOut, idxIn, idxOut, (int)n, 0, 32, c->stream);
+      cub::DeviceRadixSort::SortPairs(nullptr, sb, keyIn, keyOut, idxIn, idxOut, (int)n, 0, bitsFor(NS), c->stream);
       rc = ensureSortTmp(c, sb);
       if (rc) return rc;
       sb = c->sortTmpBytes;
-      RH_CUDA(cub::DeviceRadixSort::SortPairs(c->sortTmp, sb, keyIn, keyOut, idxIn, idxOut, (int)n, 0, 32, c->stream));
+      RH_CUDA(cub::DeviceRadixSort::SortPairs(c->sortTmp, sb, keyIn, keyOut, idxIn, idxOut, (int)n, 0, bitsFor(NS), c->stream));
    }
    k_sorted_bounds<<<blocks1d(n + 1, 256), 256, 0, c->stream>>>(keyOut, n, NS, c->ffirst);
    k_bounds_counts<<<blocks1d(NS, 256), 256, 0, c->stream>>>(c->ffirst, NS, h.cnt[h.cur]);
@@ -283,11 +283,11 @@ int f32Download(rhgpu_ctx* c, int s, uint32_t* counts, double* particles, long l
       k_iota<<<blocks1d(tot, 256), 256, 0, c->stream>>>(idxIn, tot);
       RH_CUDA(cudaGetLastError());
       size_t sb = 0;
-      cub::DeviceRadixSort::SortPairs(nullptr, sb, keyIn, keyOut, idxIn, idxOut, (int)tot, 0, 32, c->stream);
+      cub::DeviceRadixSort::SortPairs(nullptr, sb, keyIn, keyOut, idxIn, idxOut, (int)tot, 0, bitsFor(N), c->stream);
       rc = ensureSortTmp(c, sb);
       if (rc) return rc;
       sb = c->sortTmpBytes;
-      RH_CUDA(cub::DeviceRadixSort::SortPairs(c->sortTmp, sb, keyIn, keyOut, idxIn, idxOut, (int)tot, 0, 32, c->stream));
+      RH_CUDA(cub::DeviceRadixSort::SortPairs(c->sortTmp, sb, keyIn, keyOut, idxIn, idxOut, (int)tot, 0, bitsFor(N), c->stream));
       k_sorted_bounds<<<blocks1d(tot + 1, 256), 256, 0, c->stream>>>(keyOut, tot, N, c->ftmpCellStart);
       k_bounds_counts<<<blocks1d(N, 256), 256, 0, c->stream>>>(c->ftmpCellStart, N, cellCnt);
       if (particles32)
