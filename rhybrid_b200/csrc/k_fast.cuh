@@ -46,11 +46,6 @@ namespace rh {
 
 constexpr int FAST_MAX_SPECIES = 8;
 constexpr int SEG = RHGPU_FAST_SEGMENT;   // dual cells per segment
-constexpr int FT = 256;                   // threads of k_fast_avg_deposit (one chunk of particles)
-constexpr int FW = FT / 32;
-constexpr int REC = 11;                   // its doubles per deposit record: w8[8], v[3]
-static_assert(SEG == 32 && SEG * 8 == FT, "its deposit sums map (dual cell, corner) to one thread");
-
 struct SegBuf {
    double* a[7];        // x, y, z (cell-local), vx, vy, vz, weight: planes of one array
    long long plane;     // their distance in elements
@@ -477,6 +472,19 @@ __device__ __forceinline__ double cicFraction(double x, const GridInfo& g, doubl
    return fma(fma(-q, g.dx, r), g.rdx, q);
 }
 
+// one deposit record: the eight CIC weights (the products of cicWeightsLocal, in
+// its order), then 1 and the velocity
+__device__ __forceinline__ void writeRecord(double* rec, double w_x, double w_y, double w_z, double wq, double vx,
+                                            double vy, double vz) {
+   double2* const r = reinterpret_cast<double2*>(rec);
+   r[0] = make_double2((1 - w_x) * (1 - w_y) * (1 - w_z) * wq, w_x * (1 - w_y) * (1 - w_z) * wq);
+   r[1] = make_double2((1 - w_x) * w_y * (1 - w_z) * wq, w_x * w_y * (1 - w_z) * wq);
+   r[2] = make_double2((1 - w_x) * (1 - w_y) * w_z * wq, w_x * (1 - w_y) * w_z * wq);
+   r[3] = make_double2((1 - w_x) * w_y * w_z * wq, w_x * w_y * w_z * wq);
+   r[4] = make_double2(1.0, vx);
+   r[5] = make_double2(vy, vz);
+}
+
 // migration of one axis (migrateAxis); a coordinate inside [0, dx) is told by
 // one unsigned comparison of its bits (negative values and NaN compare above)
 __device__ __forceinline__ int migrateAxisBits(double& x, int& off, const GridInfo& g, bool& nan) {
@@ -719,14 +727,7 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
       unsigned long long mb = 0;
       if (lm && lane == __ffs(lm) - 1) mb = atomicAdd(fb.nmovers, (unsigned long long)__popc(lm));
       if (rec) {
-         double2* const r = reinterpret_cast<double2*>(sh.rec + recPos * PD_REC);
-         const double wq = st[6] * FS.sp[s].q;
-         r[0] = make_double2((1 - w_x) * (1 - w_y) * (1 - w_z) * wq, w_x * (1 - w_y) * (1 - w_z) * wq);
-         r[1] = make_double2((1 - w_x) * w_y * (1 - w_z) * wq, w_x * w_y * (1 - w_z) * wq);
-         r[2] = make_double2((1 - w_x) * (1 - w_y) * w_z * wq, w_x * (1 - w_y) * w_z * wq);
-         r[3] = make_double2((1 - w_x) * w_y * w_z * wq, w_x * w_y * w_z * wq);
-         r[4] = make_double2(1.0, st[3]);
-         r[5] = make_double2(st[4], st[5]);
+         writeRecord(sh.rec + recPos * PD_REC, w_x, w_y, w_z, st[6] * FS.sp[s].q, st[3], st[4], st[5]);
       }
       __syncthreads();
       if (stay) {

@@ -511,7 +511,7 @@ int fastAverages(rhgpu_ctx* c) {
       switch (perMask(c->g)) {
 #define RH_FAST_AVG(M)                                                                                         \
    case M:                                                                                                      \
-      k_fast_avg_deposit<M><<<(unsigned)c->fg.NS, FT, 0, c->stream>>>(c->g, c->fg, stay, mask, A);              \
+      k_fast_avg_deposit<M><<<(unsigned)c->fg.NS, PD_T, 0, c->stream>>>(c->g, c->fg, stay, mask, A);              \
       break;
          RH_FAST_AVG(0) RH_FAST_AVG(1) RH_FAST_AVG(2) RH_FAST_AVG(3) RH_FAST_AVG(4) RH_FAST_AVG(5) RH_FAST_AVG(6)
          RH_FAST_AVG(7)
