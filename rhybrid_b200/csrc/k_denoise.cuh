@@ -203,29 +203,73 @@ __device__ __forceinline__ bool tcWait(unsigned bar, unsigned parity) {
    return false;
 }
 
-// input slice zz into ring slot `slot`: 32 x 10 positions from (x0 - 1, y0 - 1),
-// zeros outside a non-periodic box, wrapped on periodic axes
-__device__ __forceinline__ void tcStageSlice(TcShared& sh, const DnGrid& g, const unsigned* in, const DnMoments& mom,
-                                             int x0, int y0, int zz, int slot) {
+// staging of the 32 x 10 positions of an input slice from (x0 - 1, y0 - 1), zeros
+// outside a non-periodic box, wrapped on periodic axes. What a thread copies
+// keeps its place in every slice: an activation's (16-byte half tid & 1 of five
+// positions, 64 apart) or, from the moments, whole positions (three, 128 apart),
+// so their offsets in a plane of voxels are formed once. The first layer's moments
+// are loaded before the wait on the tensor cores and stored after it, the last
+// layer's own moments likewise: the block's 4 warps wait on their own memory and
+// barriers, not on the tensor cores. Three layers of 120 x 160 x 160 voxels: 364
+// us; 451 us with every place worked out per slice and loads where they are used.
+constexpr int TC_ACT = 2 * TC_SPOS / TC_THREADS;                   // halves per thread
+constexpr int TC_MOM = (TC_SPOS + TC_THREADS - 1) / TC_THREADS;    // positions per thread
+static_assert(TC_ACT * TC_THREADS == 2 * TC_SPOS && TC_THREADS % TC_HX == 0, "whole rows per turn");
+struct TcPlaces {
+   int at[TC_ACT];   // voxel in its plane, -1 outside
+};
+__device__ __forceinline__ TcPlaces tcPlaces(const DnGrid& g, bool moments, int x0, int y0) {
+   TcPlaces P;
+   const int p0 = moments ? (int)threadIdx.x : (int)threadIdx.x >> 1, dp = moments ? TC_THREADS : TC_THREADS / 2;
+   const int x = dnWrap(x0 - 1 + p0 % TC_HX, g.nx, g.per[0]);
+#pragma unroll
+   for (int k = 0; k < TC_ACT; ++k) {
+      const int p = p0 + k * dp;
+      const int y = p < TC_SPOS ? dnWrap(y0 - 1 + p / TC_HX, g.ny, g.per[1]) : -1;
+      P.at[k] = x >= 0 && y >= 0 ? x + g.nx * y : -1;
+   }
+   return P;
+}
+
+// input slice zz of an activation into ring slot `slot` (cp.async)
+__device__ __forceinline__ void tcStageSlice(TcShared& sh, const DnGrid& g, const unsigned* in, const TcPlaces& P, int zz,
+                                             int slot) {
+   const int z = dnWrap(zz, g.nz, g.per[2]), h = threadIdx.x & 1;
+   unsigned char* const dst = &sh.plane[h][slot * TC_SLOT + 16 * (TC_PAD + (threadIdx.x >> 1))];
+   const uint4* const src = reinterpret_cast<const uint4*>(in) + ((long long)g.nx * g.ny * max(z, 0)) * 2 + h;
+#pragma unroll
+   for (int k = 0; k < TC_ACT; ++k) {
+      const bool ok = P.at[k] >= 0 && z >= 0;
+      cpAsync16(dst + 16 * (TC_THREADS / 2) * k, ok ? src + 2 * P.at[k] : src, ok ? 16 : 0);
+   }
+}
+
+// the moments of slice zz: loaded into registers, and, once they are there,
+// normalized into the first plane of ring slot `slot` (the second stays zero)
+struct TcRaw {
+   double v[TC_MOM][4];
+};
+__device__ __forceinline__ void tcLoadMoments(TcRaw& R, const DnGrid& g, const DnMoments& mom, const TcPlaces& P, int zz) {
    const int z = dnWrap(zz, g.nz, g.per[2]);
-   for (int e = threadIdx.x; e < 2 * TC_SPOS; e += TC_THREADS) {
-      const int p = e >> 1, h = e & 1;
-      const int hx = p % TC_HX, hy = p / TC_HX;
-      const int x = dnWrap(x0 - 1 + hx, g.nx, g.per[0]), y = dnWrap(y0 - 1 + hy, g.ny, g.per[1]);
-      unsigned char* dst = &sh.plane[h][slot * TC_SLOT + 16 * (TC_PAD + p)];
-      const bool ok = x >= 0 && y >= 0 && z >= 0;
-      const long long gv = ok ? (long long)x + (long long)g.nx * ((long long)y + (long long)g.ny * z) : 0;
-      if (in) {
-         cpAsync16(dst, reinterpret_cast<const uint4*>(in) + (gv * 2 + h), ok ? 16 : 0);
-      } else {
-         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-         if (ok && h == 0) {
-            const double r = mom.rho[gv], fj = dnJFactor(mom.vel, mom.rsj, r);
-            v = make_uint4(packBf16((float)(r * mom.rsr), (float)(mom.J[gv] * fj)),
-                           packBf16((float)(mom.J[mom.N + gv] * fj), (float)(mom.J[2 * mom.N + gv] * fj)), 0u, 0u);
-         }
-         *reinterpret_cast<uint4*>(dst) = v;
-      }
+   const long long plane = (long long)g.nx * g.ny * z;
+#pragma unroll
+   for (int k = 0; k < TC_MOM; ++k) {
+      const bool ok = P.at[k] >= 0 && z >= 0;
+      const long long gv = ok ? plane + P.at[k] : 0;
+      R.v[k][0] = ok ? mom.rho[gv] : 0.0;
+#pragma unroll
+      for (int l = 0; l < 3; ++l) R.v[k][1 + l] = ok ? mom.J[l * mom.N + gv] : 0.0;
+   }
+}
+__device__ __forceinline__ void tcStoreMoments(TcShared& sh, const TcRaw& R, const DnMoments& mom, int slot) {
+#pragma unroll
+   for (int k = 0; k < TC_MOM; ++k) {
+      const int p = (int)threadIdx.x + k * TC_THREADS;
+      if (p >= TC_SPOS) break;
+      const double r = R.v[k][0], fj = dnJFactor(mom.vel, mom.rsj, r);
+      *reinterpret_cast<uint4*>(&sh.plane[0][slot * TC_SLOT + 16 * (TC_PAD + p)]) =
+          make_uint4(packBf16((float)(r * mom.rsr), (float)(R.v[k][1] * fj)),
+                     packBf16((float)(R.v[k][2] * fj), (float)(R.v[k][3] * fj)), 0u, 0u);
    }
 }
 
@@ -241,10 +285,28 @@ __device__ __forceinline__ void tcPublish() {
    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// the moments that output slice z of the last layer adds to (mode 4), loaded ahead
+// of its epilogue
+struct TcOwn {
+   double v[TC_TILES][4];
+};
+__device__ __forceinline__ void tcLoadOwn(TcOwn& O, const DnGrid& g, int x0, int y0, int z, const DnMoments& mom) {
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+   for (int j = 0; j < TC_TILES; ++j) {
+      const int x = x0 - 1 + lane, y = y0 + 4 * j + warp;
+      if (lane < 1 || lane > TC_BX || x >= g.nx || y >= g.ny) continue;
+      const long long v = (long long)x + (long long)g.nx * ((long long)y + (long long)g.ny * z);
+      O.v[j][0] = mom.rho[v];
+#pragma unroll
+      for (int l = 0; l < 3; ++l) O.v[j][1 + l] = mom.J[l * mom.N + v];
+   }
+}
+
 template <bool TRANSPOSED>
 __device__ __forceinline__ void tcEpilogue(const DnGrid& g, unsigned tmem, int group, int x0, int y0, int z,
                                            const float* bias, int mode, unsigned* out, const unsigned* mask,
-                                           float* out32, const float* res, const DnMoments& mom) {
+                                           float* out32, const float* res, const DnMoments& mom, const TcOwn& own) {
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    unsigned rr[TC_TILES][16];
 #pragma unroll
@@ -289,12 +351,12 @@ __device__ __forceinline__ void tcEpilogue(const DnGrid& g, unsigned tmem, int g
       if (mode == 4) {
          if (mom.keep && mom.keep[v]) continue;
          // the velocity form writes back J = rho' u' from the denoised density and velocity
-         const double rin = mom.rho[v], fj = dnJFactor(mom.vel, mom.rsj, rin);
+         const double rin = own.v[j][0], fj = dnJFactor(mom.vel, mom.rsj, rin);
          double r0 = (double)(c[0] + (float)(rin * mom.rsr)) * mom.sr;
          if (r0 < mom.minRho) r0 = mom.minRho;
-         double j0 = (double)(c[1] + (float)(mom.J[v] * fj)) * mom.sj;
-         double j1 = (double)(c[2] + (float)(mom.J[mom.N + v] * fj)) * mom.sj;
-         double j2 = (double)(c[3] + (float)(mom.J[2 * mom.N + v] * fj)) * mom.sj;
+         double j0 = (double)(c[1] + (float)(own.v[j][1] * fj)) * mom.sj;
+         double j1 = (double)(c[2] + (float)(own.v[j][2] * fj)) * mom.sj;
+         double j2 = (double)(c[3] + (float)(own.v[j][3] * fj)) * mom.sj;
          if (mom.vel) { j0 *= r0; j1 *= r0; j2 *= r0; }
          mom.rho[v] = r0;
          mom.J[v] = j0;
@@ -379,6 +441,9 @@ k_dn_conv_tc(DnGrid g, int zc, const unsigned* in, const __nv_bfloat16* bimg, co
    const int nin = nzc + 2;   // input slices z0 - 1 .. z0 + nzc; input i is slice z0 - 1 + i, in slot i % 4
    const unsigned planeBase = (unsigned)__cvta_generic_to_shared(&sh.plane[0][0]);
    const unsigned bimgBase = (unsigned)__cvta_generic_to_shared(&sh.bimg[0]);
+   const TcPlaces places = tcPlaces(g, in == nullptr, x0, y0);
+   TcRaw raw;
+   TcOwn own;
    // tensor memory (one warp), mbarriers (one thread)
    if (warp == 0) {
       const unsigned dst = (unsigned)__cvta_generic_to_shared(&sh.tmemBase);
@@ -402,7 +467,17 @@ k_dn_conv_tc(DnGrid g, int zc, const unsigned* in, const __nv_bfloat16* bimg, co
          const int pos = k < TC_PAD ? k : TC_PAD + TC_SPOS + (k - TC_PAD);
          *reinterpret_cast<uint4*>(&sh.plane[h][slot * TC_SLOT + 16 * pos]) = make_uint4(0u, 0u, 0u, 0u);
       }
-      for (int k = 0; k < 3; ++k) tcStageSlice(sh, g, in, mom, x0, y0, z0 - 1 + k, k);
+      if (in) {
+         for (int k = 0; k < 3; ++k) tcStageSlice(sh, g, in, places, z0 - 1 + k, k);
+      } else {
+         for (int e = tid; e < TC_RING * TC_SPOS; e += TC_THREADS)
+            *reinterpret_cast<uint4*>(&sh.plane[1][(e / TC_SPOS) * TC_SLOT + 16 * (TC_PAD + e % TC_SPOS)]) =
+                make_uint4(0u, 0u, 0u, 0u);
+         for (int k = 0; k < 3; ++k) {
+            tcLoadMoments(raw, g, mom, places, z0 - 1 + k);
+            tcStoreMoments(sh, raw, mom, k);
+         }
+      }
       cpAsyncCommit();
    }
    tcPublish<0>();
@@ -433,6 +508,9 @@ k_dn_conv_tc(DnGrid g, int zc, const unsigned* in, const __nv_bfloat16* bimg, co
          const unsigned b = (unsigned)__cvta_generic_to_shared(&sh.bar[i & 1]);
          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(b) : "memory");
       }
+      const bool more = i + 3 < nin;
+      if (!in && more) tcLoadMoments(raw, g, mom, places, z0 + 2 + i);
+      if (mode == 4 && i >= 3) tcLoadOwn(own, g, x0, y0, z0 + i - 3, mom);
       if (i > 0) {
          // input i - 1's MMAs done: output slice i - 3 is complete, slot (i - 1) % 4 is free
          const int pb = (i - 1) & 1;
@@ -441,17 +519,21 @@ k_dn_conv_tc(DnGrid g, int zc, const unsigned* in, const __nv_bfloat16* bimg, co
             timedOut = true;
          } else {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (i + 3 < nin) tcStageSlice(sh, g, in, mom, x0, y0, z0 + 2 + i, (i + 3) % TC_RING);
+            if (more) {
+               if (in) tcStageSlice(sh, g, in, places, z0 + 2 + i, (i + 3) % TC_RING);
+               else tcStoreMoments(sh, raw, mom, (i + 3) % TC_RING);
+            }
             const int o = i - 3, grp = (i + 3) & 3;   // (o + 2) & 3
-            if (o >= 0) tcEpilogue<TRANSPOSED>(g, tmem, grp, x0, y0, z0 + o, bias, mode, out, mask, out32, res, mom);
+            if (o >= 0) tcEpilogue<TRANSPOSED>(g, tmem, grp, x0, y0, z0 + o, bias, mode, out, mask, out32, res, mom, own);
             if (i + 1 < nin) {   // the group's next output slice, o + 4, takes its first MMA from input i + 1
 #pragma unroll
                for (int j = 0; j < TC_TILES; ++j) tcZero16(tmem + lanes + (unsigned)(j * TC_TCOLS + 16 * grp));
                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             }
          }
-      } else if (3 < nin) {
-         tcStageSlice(sh, g, in, mom, x0, y0, z0 + 2, 3);   // slot 3 is still free
+      } else if (more) {   // slot 3 is still free
+         if (in) tcStageSlice(sh, g, in, places, z0 + 2, 3);
+         else tcStoreMoments(sh, raw, mom, 3);
       }
       cpAsyncCommit();   // one group per iteration, empty or not
       timedOut = __syncthreads_or(timedOut);
@@ -463,7 +545,8 @@ k_dn_conv_tc(DnGrid g, int zc, const unsigned* in, const __nv_bfloat16* bimg, co
          timedOut = true;
       } else {
          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-         tcEpilogue<TRANSPOSED>(g, tmem, (nzc + 1) & 3, x0, y0, z0 + nzc - 1, bias, mode, out, mask, out32, res, mom);
+         if (mode == 4) tcLoadOwn(own, g, x0, y0, z0 + nzc - 1, mom);
+         tcEpilogue<TRANSPOSED>(g, tmem, (nzc + 1) & 3, x0, y0, z0 + nzc - 1, bias, mode, out, mask, out32, res, mom, own);
       }
    }
    if (timedOut) {
