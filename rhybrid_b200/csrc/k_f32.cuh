@@ -330,8 +330,9 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
          }
          bool removed = !inside || !all;
          if (removed) {
-            atomicAdd(&cntd[4 * s + 0], FS.w[s]);
-            atomicAdd(&cntd[4 * s + 1], FS.w[s] * ((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]));
+            double* const q = removedSums(cntd, S, s);
+            atomicAdd(&q[0], FS.w[s]);
+            atomicAdd(&q[1], FS.w[s] * ((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]));
          }
          if (inside) {
             if (PER & 1) wrapc(ti, g.nx, 1);
@@ -358,9 +359,9 @@ k_f32_push_deposit(GridInfo gIn, Fields f, FastGeom fg, F32Set FS, F32Params pp,
                const float zp = (float)blockOrigin(g.z_min, tk, g.dx) + o[2] * pp.dx;
                if (xp * xp + yp * yp + zp * zp < FS.R2obs[s]) {
                   removed = true;
-                  atomicAdd(&cntd[4 * s + 2], FS.w[s]);
-                  atomicAdd(&cntd[4 * s + 3],
-                            FS.w[s] * ((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]));
+                  double* const q = removedSums(cntd, S, s);
+                  atomicAdd(&q[2], FS.w[s]);
+                  atomicAdd(&q[3], FS.w[s] * ((double)v[0] * v[0] + (double)v[1] * v[1] + (double)v[2] * v[2]));
                }
             }
             if (!removed) {

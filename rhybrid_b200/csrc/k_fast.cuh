@@ -632,8 +632,9 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
          bool removed = !inside || !all;
          if (removed) {
             const double ke = st[6] * (sq(st[3]) + sq(st[4]) + sq(st[5]));
-            atomicAdd(&cntd[4 * s + 0], st[6]);
-            atomicAdd(&cntd[4 * s + 1], ke);
+            double* const q = removedSums(cntd, S, s);
+            atomicAdd(&q[0], st[6]);
+            atomicAdd(&q[1], ke);
          }
          if (inside) {
             // the new dual cell relative to the segment's first, and to its row
@@ -660,8 +661,9 @@ k_fast_push_deposit(GridInfo gIn, Fields f, FastGeom fg, FastSpecies FS, PushPar
                   if (sq(xp) + sq(yp) + sq(zp) < FS.sp[s].R2obs) {
                      removed = true;
                      const double ke = st[6] * (sq(st[3]) + sq(st[4]) + sq(st[5]));
-                     atomicAdd(&cntd[4 * s + 2], st[6]);
-                     atomicAdd(&cntd[4 * s + 3], ke);
+                     double* const q = removedSums(cntd, S, s);
+                     atomicAdd(&q[2], st[6]);
+                     atomicAdd(&q[3], ke);
                   }
                }
             }

@@ -81,8 +81,9 @@ __global__ void k_push(GridInfo g, Fields f, PStore P, SpeciesDev sp, PushParams
    P.a[3][p] = vx; P.a[4][p] = vy; P.a[5][p] = vz;
    if (st || !inside) {
       const double w = P.a[6][p];
-      atomicAdd(&cntd[4 * sidx + 0], w);
-      atomicAdd(&cntd[4 * sidx + 1], w * (sq(vx) + sq(vy) + sq(vz)));
+      double* const q = removedSums(cntd, blockIdx.x, sidx);
+      atomicAdd(&q[0], w);
+      atomicAdd(&q[1], w * (sq(vx) + sq(vy) + sq(vz)));
       key[p] = -1;
       return;
    }
@@ -269,8 +270,9 @@ __global__ void k_bc_exterior(GridInfo g, PStore P, const int* ext, int next, do
       P.pcell[p] = -1;
    }
    if (na > 0) {
-      atomicAdd(&cntd[4 * sidx + 0], sw);
-      atomicAdd(&cntd[4 * sidx + 1], se);
+      double* const q = removedSums(cntd, blockIdx.x, sidx);
+      atomicAdd(&q[0], sw);
+      atomicAdd(&q[1], se);
    }
    P.alive[c] = 0;
 }
@@ -301,8 +303,9 @@ __global__ void k_bc_obstacle(GridInfo g, PStore P, const int* cells, int ncells
    }
    for (int t = cur; t < P.alive[c]; ++t) P.pcell[a + t] = -1;
    if (sw != 0.0 || se != 0.0) {
-      atomicAdd(&cntd[4 * sidx + 2], sw);
-      atomicAdd(&cntd[4 * sidx + 3], se);
+      double* const q = removedSums(cntd, blockIdx.x, sidx);
+      atomicAdd(&q[2], sw);
+      atomicAdd(&q[3], se);
    }
    P.alive[c] = cur;
 }

@@ -331,7 +331,7 @@ int rhgpu_create(const rhgpu_params* params, int32_t n_species, const rhgpu_spec
    alloc((void**)&c->inPrefix, sizeof(int) * 27 * N);
    alloc((void**)&c->newCount, sizeof(long long) * (N + 1));
    alloc((void**)&c->cntU, sizeof(unsigned long long) * NCNT_U);
-   alloc((void**)&c->cntD, sizeof(double) * 4 * MAX_SPECIES);
+   alloc((void**)&c->cntD, sizeof(double) * REMOVED_COPIES * REMOVED_STRIDE);
    alloc((void**)&c->err, sizeof(unsigned));
    // fast-path geometry and buffers
    FastGeom& fg = c->fg;
@@ -822,10 +822,12 @@ int rhgpu_get_counters(rhgpu_ctx* c, double* out, int32_t n) {
    if (!c || !out) return fail(RHGPU_ERR_ARG, "get_counters: bad arguments");
    RH_CUDA(cudaSetDevice(c->device));
    unsigned long long u[NCNT_U];
-   double d[4 * MAX_SPECIES];
+   double d[REMOVED_COPIES * REMOVED_STRIDE];
    RH_CUDA(cudaStreamSynchronize(c->stream));
    RH_CUDA(cudaMemcpy(u, c->cntU, sizeof u, cudaMemcpyDeviceToHost));
    RH_CUDA(cudaMemcpy(d, c->cntD, sizeof d, cudaMemcpyDeviceToHost));
+   for (int i = 1; i < REMOVED_COPIES; ++i)
+      for (int k = 0; k < REMOVED_STRIDE; ++k) d[k] += d[i * REMOVED_STRIDE + k];
    std::vector<double> v(RHGPU_NUM_FIELD_COUNTERS + RHGPU_CNT_PER_SPECIES * c->ns, 0.0);
    for (int i = 0; i < RHGPU_NUM_FIELD_COUNTERS; ++i) v[i] = (double)u[i];
    v[RHGPU_CNT_GRID_AVERAGE_COUNTER] = c->gridAvgCounter;

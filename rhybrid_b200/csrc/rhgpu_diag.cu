@@ -142,7 +142,7 @@ int diagnostics(rhgpu_ctx* c, double* out, bool withScales) {
 // the log counters back to zero (logWriteParticleField, diagnostics.h:777-800)
 int zeroLogCounters(rhgpu_ctx* c) {
    RH_CUDA(cudaMemsetAsync(c->cntU, 0, sizeof(unsigned long long) * NCNT_U, c->stream));
-   RH_CUDA(cudaMemsetAsync(c->cntD, 0, sizeof(double) * 4 * MAX_SPECIES, c->stream));
+   RH_CUDA(cudaMemsetAsync(c->cntD, 0, sizeof(double) * REMOVED_COPIES * REMOVED_STRIDE, c->stream));
    if (c->injCnt) RH_CUDA(cudaMemsetAsync(c->injCnt, 0, sizeof(double) * 3 * MAX_SPECIES, c->stream));
    RH_CUDA(cudaStreamSynchronize(c->stream));
    return RHGPU_OK;

@@ -52,6 +52,7 @@ int fail(int code, const std::string& msg);
    } while (0)
 
 const int MAX_SPECIES = 8;
+static_assert(4 * MAX_SPECIES <= REMOVED_STRIDE, "a copy of the removed sums holds every species");
 const int NCNT_U = 32;   // field counters 0..15, species MaxVi at 16+s
 
 struct TimerRec { int cls; int ea, eb; };
