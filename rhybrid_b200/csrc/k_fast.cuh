@@ -509,11 +509,12 @@ __device__ __forceinline__ int migrateAxisBits(double& x, int& off, const GridIn
 // reservation's round trip overlaps the chunk's remaining work.
 //
 // It is bound by issue slots and the waits between them at the 32 warps per SM
-// that 64 registers and 57 KB of shared memory leave (62 % of cycles issue, 67 %
+// that 64 registers and 56 KB of shared memory leave (62 % of cycles issue, 59 %
 // of the shared-memory wavefronts), not by memory.
-// Mars run, 9.25e7 ions, 120 x 160 x 160 cells: 4.33 ms per step = 2300 GB/s of
-// its 104 bytes per ion and cell; 4.62 ms with species packed within a chunk,
-// eleven 8-byte accesses per record and one corner x four moments per thread;
+// Mars run, 9.25e7 ions, 120 x 160 x 160 cells: 4.27 ms per step = 2330 GB/s of
+// its 104 bytes per ion and cell; 4.33 ms with a pointer per plane; 4.62 ms with
+// species packed within a chunk, eleven 8-byte accesses per record and one corner
+// x four moments per thread;
 // 5.35 ms with two particles per thread at 16 warps per SM.
 template <int PER, bool EXTRA>
 __global__ void __launch_bounds__(PD_T, 4)
