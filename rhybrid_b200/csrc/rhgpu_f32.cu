@@ -345,6 +345,7 @@ int f32Push(rhgpu_ctx* c) {
    if (c->P.initial_flow_through_period < c->t && c->useIFT) c->useIFT = 0;
    const long long NS = c->fg.NS;
    if ((rc = migBegin(c)) != RHGPU_OK) return rc;
+   if ((rc = fixedRestart(c)) != RHGPU_OK) return rc;
    {
       RH_TIME(c, "f32_push_deposit");
       const F32Set FS = f32Set(c);
@@ -392,7 +393,9 @@ int f32Gather(rhgpu_ctx* c) {
       k_f32_gather<false><<<gatherGrid(c->g), 2 * GA_CELLS, 0, c->stream>>>(c->g, c->f, c->fg, c->f32b, hiR, loR, hiJ,
                                                                         loJ, scale, c->P.min_ion_charge_density, c->cntU);
    RH_LAUNCHED(c);
-   return fixedClear(c, c->f32b.MMlo, c->f32b.MMhi);
+   if (const int rc_ = fixedClear(c, c->f32b.MMlo, c->f32b.MMhi)) return rc_;
+   c->fixedDirty = false;
+   return RHGPU_OK;
 }
 
 }  // namespace rhh

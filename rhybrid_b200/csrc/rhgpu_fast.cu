@@ -561,6 +561,7 @@ int fastPush(rhgpu_ctx* c) {
    pp.maxVi2 = c->P.max_ion_speed2;
    pp.avgList = c->avgGroups > 0;
    if (const int rc = migBegin(c)) return rc;
+   if (const int rc = fixedRestart(c)) return rc;
    {
       RH_TIME(c, "fast_push_deposit");
       const FastSpecies FS = fastSpecies(c);
@@ -605,6 +606,15 @@ int fixedClear(rhgpu_ctx* c, unsigned long long* lo, unsigned long long* hi) {
    return RHGPU_OK;
 }
 
+// the sums of a push that was never gathered (a second rhgpu_push, or a step
+// refused in between) are dropped: a gather takes the last push's deposit
+int fixedRestart(rhgpu_ctx* c) {
+   if (c->fixedDirty)
+      if (const int rc = fixedClear(c, c->fb.MMlo, c->fb.MMhi)) return rc;
+   c->fixedDirty = true;
+   return RHGPU_OK;
+}
+
 int fastGather(rhgpu_ctx* c) {
    RH_TIME(c, "fast_gather");
    const double hiR = std::ldexp(1.0, 64 - c->kR), loR = std::ldexp(1.0, -c->kR);
@@ -616,7 +626,9 @@ int fastGather(rhgpu_ctx* c) {
       k_fast_gather<false><<<gatherGrid(c->g), 2 * GA_CELLS, 0, c->stream>>>(c->g, c->f, c->fg, c->fb, hiR, loR, hiJ, loJ,
                                                                          c->P.min_ion_charge_density, c->cntU);
    RH_LAUNCHED(c);
-   return fixedClear(c, c->fb.MMlo, c->fb.MMhi);
+   if (const int rc_ = fixedClear(c, c->fb.MMlo, c->fb.MMhi)) return rc_;
+   c->fixedDirty = false;
+   return RHGPU_OK;
 }
 
 template int moverPass<Mover32, F32Set>(rhgpu_ctx*, const Mover32*, long long, const F32Set&, int, unsigned,

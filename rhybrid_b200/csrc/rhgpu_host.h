@@ -161,6 +161,7 @@ struct rhgpu_ctx {
    cudaEvent_t migEvent = nullptr;
    bool migPending = false;             // a push's movers wait for migFinish
    bool migDirty = false;               // finc may hold counts of a step that did not finish
+   bool fixedDirty = false;             // MMlo / MMhi hold the movers' sums of a push that no gather has taken
    long long migLast = -1;              // movers of the last step (-1: none yet): the next one's launch sizes
    int kR = 0, kJ = 0;
    void* sortTmp = nullptr;
@@ -319,6 +320,7 @@ int fastDownload(rhgpu_ctx* c, int s, uint32_t* counts, double* particles, long 
 int fastPush(rhgpu_ctx* c);
 int fastGather(rhgpu_ctx* c);
 int fixedClear(rhgpu_ctx* c, unsigned long long* lo, unsigned long long* hi);
+int fixedRestart(rhgpu_ctx* c);
 
 // ---- FP32 form (rhgpu_f32.cu)
 F32Buf f32View(const F32Host& h, int which);
