@@ -761,7 +761,6 @@ int rhgpu_push(rhgpu_ctx* c) {
    if (!c) return fail(RHGPU_ERR_ARG, "null context");
    RH_CUDA(cudaSetDevice(c->device));
    int rc = phasePush(c);
-   if (!rc) rc = migFinish(c);
    if (rc) return rc;
    return checkDeviceError(c);
 }
@@ -802,9 +801,6 @@ int rhgpu_step(rhgpu_ctx* c, int32_t nsteps) {
       if (!rc && c->dnOn) rc = dnApplyCtx(c);
       if (!rc) rc = phaseBoundaries(c);
       if (!rc) rc = fieldsAll(c);
-      // the movers' placement touches the particle storage only: the host looks
-      // at it once the gather and the field update are on the stream
-      if (!rc) rc = migFinish(c);
       if (rc) return rc;
    }
    return checkDeviceError(c);

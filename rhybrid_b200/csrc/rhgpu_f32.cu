@@ -337,7 +337,6 @@ int f32RelayoutNext(rhgpu_ctx* c, unsigned mask) {
 
 int f32Push(rhgpu_ctx* c) {
    int rc = f32Init(c);
-   if (!rc) rc = migFinish(c);
    // a relayout of the last step may have grown the particle storage
    if (!rc) rc = f32MoverBuffers(c);
    if (rc) return rc;
@@ -375,8 +374,12 @@ int f32Push(rhgpu_ctx* c) {
                      c->f32b.scaleR, c->f32b.scaleJ, true);
       if (rc) return rc;
    }
-   RH_TIME(c, "f32_migrate");
-   return migLaunch(c, c->f32b.movers, c->f32b.moverCap, f32Set(c));
+   {
+      RH_TIME(c, "f32_migrate");
+      rc = migLaunch(c, c->f32b.movers, c->f32b.moverCap, f32Set(c));
+      if (rc) return rc;
+   }
+   return migFinish(c);
 }
 
 int f32Gather(rhgpu_ctx* c) {

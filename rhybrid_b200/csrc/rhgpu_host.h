@@ -159,7 +159,6 @@ struct rhgpu_ctx {
    MigCtl* mig = nullptr;               // the step's migration state (fb.nmovers is its nm)
    MigCtl* migHost = nullptr;           // pinned copy, valid after migEvent
    cudaEvent_t migEvent = nullptr;
-   bool migPending = false;             // a push's movers wait for migFinish
    bool migDirty = false;               // finc may hold counts of a step that did not finish
    bool fixedDirty = false;             // MMlo / MMhi hold the movers' sums of a push that no gather has taken
    long long migLast = -1;              // movers of the last step (-1: none yet): the next one's launch sizes
@@ -343,8 +342,8 @@ void freeInjector(InjHost& h);
 // the movers' deposit and placement (rhgpu_fast.cu; instantiated for the fast
 // path's and the FP32 form's movers) and the particle sources of a step
 // appended to a mover list. migBegin clears the step's migration state,
-// moverPass and migLaunch put the whole step on the stream, migFinish waits for
-// migLaunch's state and does what the device could not.
+// moverPass and migLaunch put the deposit and the placement on the stream,
+// migFinish ends the push: it waits for the state and does what the device could not.
 int migBegin(rhgpu_ctx* c);
 template <class MV, class SET>
 int moverPass(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS, int need, unsigned smask, unsigned long long* lo,
