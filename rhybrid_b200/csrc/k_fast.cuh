@@ -816,7 +816,8 @@ k_mover_pass(GridInfo g, FastGeom fg, SET FS, const MV* mv, const MigCtl* ctl, l
              unsigned long long* lo, unsigned long long* hi, double scaleR, double scaleJ, int* inc, unsigned* rank) {
    __shared__ long long term[MP_THREADS / 32][32][4];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, o = lane & 7;
-   const long long nm = min((long long)ctl->nm, cap);
+   const long long nm = (long long)ctl->nm;
+   if (nm > cap) return;   // more movers than the list holds: the host ends the step with an error
    const long long step = (long long)gridDim.x * (MP_THREADS / 8);
    for (long long m0 = ((long long)blockIdx.x * (MP_THREADS / 32) + warp) * 4; m0 < nm; m0 += step) {
       const long long m = m0 + (lane >> 3);

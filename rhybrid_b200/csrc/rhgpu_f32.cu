@@ -377,6 +377,7 @@ int f32Push(rhgpu_ctx* c) {
    {
       RH_TIME(c, "f32_migrate");
       rc = migLaunch(c, c->f32b.movers, c->f32b.moverCap, f32Set(c));
+      if (!rc) rc = migPlace(c, c->f32b.movers, c->f32b.moverCap, f32Set(c), 0);
       if (rc) return rc;
    }
    return migFinish(c);

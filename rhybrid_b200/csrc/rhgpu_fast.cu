@@ -201,8 +201,8 @@ int migPlace(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS, int force
    return RHGPU_OK;
 }
 
-// the counted movers' places in the list, as far as the device can take them;
-// the migration state is on its way to the host before the list is filled
+// the counted movers listed by destination; the migration state is on its way to
+// the host before the list is filled
 template <class MV, class SET>
 int migLaunch(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS) {
    const int NS = (int)c->fg.NS;
@@ -212,7 +212,16 @@ int migLaunch(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS) {
    RH_CUDA(cudaEventRecord(c->migEvent, c->stream));
    k_mig_list<<<moverBlocks(c, 256), 256, 0, c->stream>>>(mv, c->mig, cap, 0, NS, c->foffInc, c->mbkt, c->mkey, c->mval);
    RH_LAUNCHED(c);
-   return migPlace(c, mv, cap, FS, 0);
+   return RHGPU_OK;
+}
+
+// the step's movers fit the list; if not, k_mover_pass has deposited none and the
+// push stops here, before anything has taken its deposit
+int migFits(rhgpu_ctx* c) {
+   RH_CUDA(cudaEventSynchronize(c->migEvent));
+   const long long cap = c->path == RHGPU_PATH_FP32 ? c->f32b.moverCap : c->fb.moverCap;
+   if ((long long)c->migHost->nm > cap) return fail(RHGPU_ERR_CAPACITY, "mover list overflow");
+   return RHGPU_OK;
 }
 
 FastSpecies setOf(rhgpu_ctx* c, const Mover*) { return fastSpecies(c); }
@@ -286,10 +295,9 @@ int migResolve(rhgpu_ctx* c, const MV* mv, long long cap) {
 // box of 20 ions per cell (202 -> 205 us) than a wait after the field update,
 // nothing measurable at 16^3 cells or above 2e6 ions.
 int migFinish(rhgpu_ctx* c) {
-   RH_CUDA(cudaEventSynchronize(c->migEvent));
+   if (const int rc = migFits(c)) return rc;
    const bool f32 = c->path == RHGPU_PATH_FP32;
    const long long cap = f32 ? c->f32b.moverCap : c->fb.moverCap, nm = (long long)c->migHost->nm;
-   if (nm > cap) return fail(RHGPU_ERR_CAPACITY, "mover list overflow");
    c->migLast = nm;
    if (c->migHost->over || c->migHost->maxInc > MIG_RANK) {
       const int rc = f32 ? migResolve(c, c->f32b.movers, cap) : migResolve(c, c->fb.movers, cap);
@@ -590,13 +598,18 @@ int fastPush(rhgpu_ctx* c) {
                                c->fb.scaleR, c->fb.scaleJ, true);
       if (rc) return rc;
    }
-   if (c->avgGroups) {
-      const int rc = fastAverages(c);
-      if (rc) return rc;
-   }
    {
       RH_TIME(c, "fast_migrate");
       const int rc = migLaunch(c, c->fb.movers, c->fb.moverCap, fastSpecies(c));
+      if (rc) return rc;
+   }
+   if (c->avgGroups) {   // before the placement: the averages read the stayers alone
+      if (const int rc = migFits(c)) return rc;
+      if (const int rc = fastAverages(c)) return rc;
+   }
+   {
+      RH_TIME(c, "fast_migrate");
+      const int rc = migPlace(c, c->fb.movers, c->fb.moverCap, fastSpecies(c), 0);
       if (rc) return rc;
    }
    return migFinish(c);
@@ -638,6 +651,7 @@ int fastGather(rhgpu_ctx* c) {
 template int moverPass<Mover32, F32Set>(rhgpu_ctx*, const Mover32*, long long, const F32Set&, int, unsigned,
                                         unsigned long long*, unsigned long long*, double, double, bool);
 template int migLaunch<Mover32, F32Set>(rhgpu_ctx*, const Mover32*, long long, const F32Set&);
+template int migPlace<Mover32, F32Set>(rhgpu_ctx*, const Mover32*, long long, const F32Set&, int);
 template int injectAll<Mover>(rhgpu_ctx*, Mover*, long long);
 template int injectAll<Mover32>(rhgpu_ctx*, Mover32*, long long);
 

@@ -342,14 +342,17 @@ void freeInjector(InjHost& h);
 // the movers' deposit and placement (rhgpu_fast.cu; instantiated for the fast
 // path's and the FP32 form's movers) and the particle sources of a step
 // appended to a mover list. migBegin clears the step's migration state,
-// moverPass and migLaunch put the deposit and the placement on the stream,
-// migFinish ends the push: it waits for the state and does what the device could not.
+// moverPass, migLaunch and migPlace put the deposit, the list and the placement on
+// the stream, migFinish ends the push: it waits for the state and does what the
+// device could not.
 int migBegin(rhgpu_ctx* c);
 template <class MV, class SET>
 int moverPass(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS, int need, unsigned smask, unsigned long long* lo,
               unsigned long long* hi, double scaleR, double scaleJ, bool count);
 template <class MV, class SET>
 int migLaunch(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS);
+template <class MV, class SET>
+int migPlace(rhgpu_ctx* c, const MV* mv, long long cap, const SET& FS, int force);
 template <class MV>
 int migResolve(rhgpu_ctx* c, const MV* mv, long long cap);
 int migFinish(rhgpu_ctx* c);
