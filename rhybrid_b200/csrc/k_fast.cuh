@@ -871,11 +871,14 @@ k_mover_pass(GridInfo g, FastGeom fg, SET FS, const MV* mv, const MigCtl* ctl, l
 // FP32 and FP64 form), depending on its vector width and resident warps, where
 // the gather and the fill together take 0.13 (FP32) and 0.15 (FP64).
 constexpr int GA_CELLS = 64;   // cells of a block of 128 threads, consecutive in x
-inline dim3 gatherGrid(const GridInfo& g) { return dim3((g.nx + GA_CELLS - 1) / GA_CELLS, g.ny, g.nz); }
+// the blocks of a row and the rows share the launch's x axis: its y axis ends at
+// 65535 blocks, and ny may be more
+inline dim3 gatherGrid(const GridInfo& g) { return dim3((g.nx + GA_CELLS - 1) / GA_CELLS * g.ny, 1, g.nz); }
 #define RH_GATHER_PROLOGUE                                        \
-   const int i = blockIdx.x * GA_CELLS + (threadIdx.x >> 1);      \
+   const int nxb = (g.nx + GA_CELLS - 1) / GA_CELLS;              \
+   const int j = (int)blockIdx.x / nxb, k = blockIdx.z;           \
+   const int i = ((int)blockIdx.x - j * nxb) * GA_CELLS + (threadIdx.x >> 1); \
    const int h = threadIdx.x & 1;                                 \
-   const int j = blockIdx.y, k = blockIdx.z;                      \
    if (i >= g.nx) return;                                         \
    const long long n = cidx(g, i, j, k);                          \
    const long long N = g.N;

@@ -291,9 +291,9 @@ int migResolve(rhgpu_ctx* c, const MV* mv, long long cap) {
 // the push's movers placed, its "next" buffers become the current ones: the last
 // part of a push, so that no step leaves a migration behind, whatever its later
 // phases return. The host waits for the state that k_mig_buckets leaves, with the
-// list and the placement on the stream behind it: 2.7 us more per step of a 32^3
-// box of 20 ions per cell (202 -> 205 us) than a wait after the field update,
-// nothing measurable at 16^3 cells or above 2e6 ions.
+// list and the placement on the stream behind it: 1.4 to 2.2 us more per step of
+// a 32^3 box of 20 ions per cell (107 us) than a wait after the field update,
+// nothing measurable at 2e6 ions and more.
 int migFinish(rhgpu_ctx* c) {
    if (const int rc = migFits(c)) return rc;
    const bool f32 = c->path == RHGPU_PATH_FP32;
