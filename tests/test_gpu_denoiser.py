@@ -147,6 +147,39 @@ def test_gradients_match_oracle():
         d.close()
 
 
+# sizes (nx, ny, nz) and the output slices that a block of the convolutions streams there (test_cpu_block_rules.py holds
+# them to the rule): the last block has fewer; two columns of blocks in x at one of them; 14 to 107 rows of gradient
+# partials
+SLICES = [((3, 173, 27), 2), ((31, 213, 11), 2), ((3, 1581, 5), 3), ((3, 1581, 15), 8), ((3, 1581, 23), 12)]
+
+
+@pytest.mark.parametrize("dims,periodic", [(d, (1, 0, 1) if q % 2 else (0, 1, 0)) for q, (d, _) in enumerate(SLICES)])
+def test_streamed_slices_match_oracle(dims, periodic):
+    """Forward (in place, from the moments) and gradients where a block streams
+    several slices, to the bounds of the small grid's tests."""
+    nx, ny, nz = dims
+    rng = np.random.default_rng(nz)
+    d = abi.Denoiser(abi.gpu_library(), nx, ny, nz, periodic)
+    try:
+        d.set_scales(2.0, 3.0)
+        p = random_params(rng)
+        d.set_params(p)
+        x = rng.normal(0, 1, (nz, ny, nx, 4)).astype(np.float32)
+        ro, jo = d.apply(*to_abi(x, 2.0, 3.0))
+        got = np.concatenate([(ro / 2.0).reshape(nz, ny, nx, 1), (jo / 3.0).reshape(nz, ny, nx, 3)], axis=-1)
+        want, _ = odn.forward(p, x, periodic, bf16_mode=True)
+        assert np.abs(got - want).max() < 1e-2 * np.abs(want).max()
+        t = rng.normal(0, 1, x.shape).astype(np.float32)
+        loss, g = d.loss_grad(*to_abi(x, 2.0, 3.0), *to_abi(t, 2.0, 3.0))
+        lw, gw = odn.loss_grad(p, x, t, periodic, bf16_mode=True)
+        assert abs(loss - lw) <= 1e-3 * lw
+        for l in range(3):
+            sl = slice(l * odn.LAYER, (l + 1) * odn.LAYER)
+            assert np.linalg.norm(g[sl] - gw[sl]) < 2e-2 * np.linalg.norm(gw[sl]), l
+    finally:
+        d.close()
+
+
 def test_training_on_method_pairs_gains_on_held_out_pairs():
     """Mars-like geometry (2 % of the cells) at 256 ppc; pairs at 8 ppc (1 in
     32 particles) from 6 states; after training, the denoised moments of a
