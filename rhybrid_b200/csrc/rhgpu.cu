@@ -524,7 +524,7 @@ int rhgpu_download_array(rhgpu_ctx* c, int32_t id, double* host) {
 int rhgpu_upload_cell_flags(rhgpu_ctx* c, const uint8_t* host) {
    if (!c || !host) return fail(RHGPU_ERR_ARG, "upload_cell_flags: bad arguments");
    RH_CUDA(cudaSetDevice(c->device));
-   RH_CUDA(cudaMemcpy(c->flags, host, c->g.N, cudaMemcpyHostToDevice));
+   if (const int rc = copyOnStream(c, c->flags, host, (size_t)c->g.N)) return rc;
    std::vector<int> ob;
    for (long long n = 0; n < c->g.N; ++n)
       if (host[n] & RHGPU_FLAG_INNER_PARTICLE) ob.push_back((int)n);
@@ -556,14 +556,13 @@ int rhgpu_upload_cell_flags(rhgpu_ctx* c, const uint8_t* host) {
             si[(size_t)S] = hit ? 1 : 0;
          }
       }
-      RH_CUDA(cudaMemcpy(c->segInnerDev, si.data(), (size_t)fg.NS, cudaMemcpyHostToDevice));
+      if (const int rc = copyOnStream(c, c->segInnerDev, si.data(), (size_t)fg.NS)) return rc;
    }
    cudaFree(c->obst);
    c->obst = nullptr;
    c->nobst = (int)ob.size();
    RH_CUDA(cudaMalloc(&c->obst, sizeof(int) * (ob.size() + 1)));
-   if (!ob.empty()) RH_CUDA(cudaMemcpy(c->obst, ob.data(), sizeof(int) * ob.size(), cudaMemcpyHostToDevice));
-   return RHGPU_OK;
+   return ob.empty() ? RHGPU_OK : copyOnStream(c, c->obst, ob.data(), sizeof(int) * ob.size());
 }
 
 namespace {
@@ -607,8 +606,8 @@ int rhgpu_upload_particles(rhgpu_ctx* c, int32_t s, const uint32_t* counts, cons
       const long long cap = std::max<long long>(c->capHint[s], (long long)n + n / 8 + 1024);
       freeStore(c->ps[s]);
       freeStore(c->alt[s]);
-      int rc0 = allocStore(c->ps[s], cap, N);
-      if (!rc0) rc0 = allocStore(c->alt[s], cap, N);
+      int rc0 = allocStore(c, c->ps[s], cap);
+      if (!rc0) rc0 = allocStore(c, c->alt[s], cap);
       if (rc0) return rc0;
    }
    int rc = ensureStaging(c, sizeof(double) * 7 * (size_t)(n > 0 ? n : 1) + sizeof(uint32_t) * (size_t)N + 64);

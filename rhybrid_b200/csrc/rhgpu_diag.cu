@@ -256,8 +256,8 @@ int rhgpu_set_population_averages(rhgpu_ctx* c, int32_t n_groups, const int32_t*
    RH_CUDA(cudaMalloc(&c->avgN, sizeof(double) * n_groups * N));
    RH_CUDA(cudaMalloc(&c->avgV, sizeof(double) * 3 * n_groups * N));
    RH_CUDA(cudaMalloc(&c->avgOut, sizeof(double) * 4 * N));
-   RH_CUDA(cudaMemset(c->avgN, 0, sizeof(double) * n_groups * N));
-   RH_CUDA(cudaMemset(c->avgV, 0, sizeof(double) * 3 * n_groups * N));
+   if (const int rc = clearOnStream(c, c->avgN, sizeof(double) * n_groups * N)) return rc;
+   if (const int rc = clearOnStream(c, c->avgV, sizeof(double) * 3 * n_groups * N)) return rc;
    for (int s = 0; s < c->ns; ++s) c->avgGroupOf[s] = group_of_species[s];
    c->avgGroups = n_groups;
    return RHGPU_OK;
@@ -315,7 +315,7 @@ int rhgpu_set_grid_counters(rhgpu_ctx* c, int32_t enable) {
       return RHGPU_OK;
    }
    if (!c->gridCnt) RH_CUDA(cudaMalloc(&c->gridCnt, sizeof(double) * GC_PLANES * N));
-   RH_CUDA(cudaMemset(c->gridCnt, 0, sizeof(double) * GC_PLANES * N));
+   if (const int rc = clearOnStream(c, c->gridCnt, sizeof(double) * GC_PLANES * N)) return rc;
    c->f.gc = c->gridCnt;
    return RHGPU_OK;
 }

@@ -17,16 +17,16 @@ constexpr int NOALLOC_MAX_DEVICES = 64;
 // looks the address up and stores the same value
 std::atomic<double*> g_noallocPtr[NOALLOC_MAX_DEVICES] = {};
 
-int allocStore(PStore& s, long long cap, long long N) {
+int allocStore(rhgpu_ctx* c, PStore& s, long long cap) {
+   const long long N = c->g.N;
    s.cap = cap;
    s.nslots = 0;
    for (int a = 0; a < 7; ++a) RH_CUDA(cudaMalloc(&s.a[a], sizeof(double) * (cap > 0 ? cap : 1)));
    RH_CUDA(cudaMalloc(&s.pcell, sizeof(int) * (cap > 0 ? cap : 1)));
    RH_CUDA(cudaMalloc(&s.start, sizeof(long long) * (N + 1)));
    RH_CUDA(cudaMalloc(&s.alive, sizeof(int) * N));
-   RH_CUDA(cudaMemset(s.start, 0, sizeof(long long) * (N + 1)));
-   RH_CUDA(cudaMemset(s.alive, 0, sizeof(int) * N));
-   return RHGPU_OK;
+   const int rc = clearOnStream(c, s.start, sizeof(long long) * (N + 1));
+   return rc ? rc : clearOnStream(c, s.alive, sizeof(int) * N);
 }
 
 void freeStore(PStore& s) {

@@ -488,22 +488,37 @@ int injectAll(rhgpu_ctx* c, MV* movers, long long moverCap) {
    return RHGPU_OK;
 }
 
+// the averages' sums, allocated at their first step: all of them or none
+int averageBuffers(rhgpu_ctx* c) {
+   FastBufs& A = c->avgFB;
+   if (A.RP) return RHGPU_OK;
+   const size_t rp = sizeof(double) * 16 * c->fg.nrows * c->g.nx, rpb = sizeof(double) * 16 * c->fg.nrows * c->fg.nseg,
+                mm = sizeof(unsigned long long) * 4 * c->g.N;
+   FastBufs n = {};
+   cudaError_t e = cudaMalloc(&n.RP, rp);
+   if (e == cudaSuccess) e = cudaMalloc(&n.RPB, rpb);
+   if (e == cudaSuccess) e = cudaMalloc(&n.MMlo, mm);
+   if (e == cudaSuccess) e = cudaMalloc(&n.MMhi, mm);
+   int rc = e == cudaSuccess ? clearOnStream(c, n.RPB, rpb)
+                             : fail(RHGPU_ERR_CUDA, std::string("population averages: ") + cudaGetErrorString(e));
+   if (!rc) rc = fixedClear(c, n.MMlo, n.MMhi);
+   if (rc) {
+      cudaGetLastError();
+      cudaFree(n.RP); cudaFree(n.RPB); cudaFree(n.MMlo); cudaFree(n.MMhi);
+      return rc;
+   }
+   A.RP = n.RP; A.RPB = n.RPB; A.MMlo = n.MMlo; A.MMhi = n.MMhi;
+   return RHGPU_OK;
+}
+
 // fast path: each output population's share of this step's deposit added to
 // its averages: the stayers (the next buffer before the arrivals are placed)
 // by segment, then every deposited mover (left its segment, or deposited in it
 // and removed by a boundary)
 int fastAverages(rhgpu_ctx* c) {
    const long long N = c->g.N;
+   if (const int rc = averageBuffers(c)) return rc;
    FastBufs& A = c->avgFB;
-   if (!A.RP) {
-      RH_CUDA(cudaMalloc(&A.RP, sizeof(double) * 16 * c->fg.nrows * c->g.nx));
-      RH_CUDA(cudaMalloc(&A.RPB, sizeof(double) * 16 * c->fg.nrows * c->fg.nseg));
-      RH_CUDA(cudaMalloc(&A.MMlo, sizeof(unsigned long long) * 4 * N));
-      RH_CUDA(cudaMalloc(&A.MMhi, sizeof(unsigned long long) * 4 * N));
-      RH_CUDA(cudaMemset(A.RPB, 0, sizeof(double) * 16 * c->fg.nrows * c->fg.nseg));
-      RH_CUDA(cudaMemset(A.MMlo, 0, sizeof(unsigned long long) * 4 * N));
-      RH_CUDA(cudaMemset(A.MMhi, 0, sizeof(unsigned long long) * 4 * N));
-   }
    A.scaleR = c->fb.scaleR;
    A.scaleJ = c->fb.scaleJ;
    const double hiR = std::ldexp(1.0, 64 - c->kR), loR = std::ldexp(1.0, -c->kR);

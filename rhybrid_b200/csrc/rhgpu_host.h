@@ -255,6 +255,18 @@ struct KScope {
 };
 #define RH_TIME(c, name) KScope rh_scope_(c, name)
 
+// device memory cleared, or filled from host memory that may go, in the order of
+// the context's stream (which does not wait for the default stream's work)
+inline int clearOnStream(rhgpu_ctx* c, void* p, size_t bytes) {
+   RH_CUDA(cudaMemsetAsync(p, 0, bytes, c->stream));
+   return RHGPU_OK;
+}
+inline int copyOnStream(rhgpu_ctx* c, void* dst, const void* host, size_t bytes) {
+   RH_CUDA(cudaMemcpyAsync(dst, host, bytes, cudaMemcpyHostToDevice, c->stream));
+   RH_CUDA(cudaStreamSynchronize(c->stream));
+   return RHGPU_OK;
+}
+
 #define RH_LAUNCHED(c) do { int rc_ = checkLaunch(c); if (rc_) return rc_; } while (0)
 
 template <class T>
@@ -292,7 +304,7 @@ int checkDeviceError(rhgpu_ctx* c);
 int fieldsAll(rhgpu_ctx* c);
 
 // ---- exact path (rhgpu_exact.cu)
-int allocStore(PStore& s, long long cap, long long N);
+int allocStore(rhgpu_ctx* c, PStore& s, long long cap);
 void freeStore(PStore& s);
 int pushAll(rhgpu_ctx* c);
 // species whose particles the exact-path deposit adds (accumulating, particles uploaded)

@@ -281,7 +281,7 @@ int buildInjector(rhgpu_ctx* c, const rhgpu_injector& J, long long& keyBase, Inj
       if (rc) return rc;
       if (!rates.empty()) {
          RH_CUDA(cudaMalloc(&h.rates, sizeof(double) * rates.size()));
-         RH_CUDA(cudaMemcpy(h.rates, rates.data(), sizeof(double) * rates.size(), cudaMemcpyHostToDevice));
+         if (const int rc2 = copyOnStream(c, h.rates, rates.data(), sizeof(double) * rates.size())) return rc2;
       }
       h.rateCells = cells;
       h.rateValues = rates;
@@ -300,7 +300,7 @@ int buildInjector(rhgpu_ctx* c, const rhgpu_injector& J, long long& keyBase, Inj
    keyBase += (long long)cells.size();
    if (!cells.empty()) {
       RH_CUDA(cudaMalloc(&h.cells, sizeof(int) * cells.size()));
-      RH_CUDA(cudaMemcpy(h.cells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice));
+      if (const int rc = copyOnStream(c, h.cells, cells.data(), sizeof(int) * cells.size())) return rc;
    }
    h.d.cells = h.cells;
    return RHGPU_OK;
@@ -315,7 +315,7 @@ int rhgpu_set_injectors(rhgpu_ctx* c, int32_t n, const rhgpu_injector* inj) {
    RH_CUDA(cudaStreamSynchronize(c->stream));
    if (!c->injCnt) {
       RH_CUDA(cudaMalloc(&c->injCnt, sizeof(double) * 3 * MAX_SPECIES));
-      RH_CUDA(cudaMemset(c->injCnt, 0, sizeof(double) * 3 * MAX_SPECIES));
+      if (const int rc = clearOnStream(c, c->injCnt, sizeof(double) * 3 * MAX_SPECIES)) return rc;
    }
    long long keyBase = c->fg.NS > 0 ? c->fg.NS : 1;
    std::vector<InjHost> built;
