@@ -144,8 +144,8 @@ k_fast_avg_deposit(GridInfo gIn, FastGeom fg, FastSpecies FS, unsigned mask, Fas
    segPartialsOut<PD_T>(g, fg, fb.RP, fb.RPB, s_rec, row, gseg, u0, u1);
 }
 
-// fast path: row partials + fixed-point part added to the population's sums;
-// the fixed-point sums restart
+// fast path: row partials + fixed-point part added to the population's sums; the
+// host clears the fixed-point sums after it
 __global__ void __launch_bounds__(2 * GA_CELLS)
 k_fast_avg_gather(GridInfo g, FastGeom fg, FastBufs fb, double hiR, double loR, double hiJ, double loJ, double* nSum,
                   double* vSum);

@@ -572,11 +572,11 @@ k_dn_conv_tc(DnGrid g, int zc, const unsigned* in, const __nv_bfloat16* bimg, co
 // B[vox][co] (mma), then the 4 warps are added in order and the block's part of
 // its partial row (DN_LAYER values) written. A warp stages a k-step's voxels as
 // 16-byte halves in shared memory, where ldmatrix transposes them into operands;
-// the next k-step's are loaded meanwhile. 52 us for 64^3 voxels; bound by the
-// L2 reads of X, three times per row of taps. A training iteration at 64^3, with
-// one tap per block, 2-byte operand loads, the partial rows added one load after
-// another, 21 launches and a read-back: 0.98 ms; with this, rows added 16 loads at
-// a time, 14 launches and the losses read every 64 iterations: 0.40 ms.
+// the next k-step's are loaded meanwhile. 52 us for 64^3 voxels; bound by the L2
+// reads: X once per tap, 27 times, and dY ten times. A training iteration at 64^3,
+// with one tap per block, 2-byte operand loads, the partial rows added one load
+// after another, 26 launches and a read-back: 0.98 ms; with this, rows added 16
+// loads at a time, 15 launches and the losses read every 64 iterations: 0.40 ms.
 constexpr int DN_WGRAD_ROWS = 9;   // (dy, dz) pairs
 __global__ void __launch_bounds__(32 * DN_WARPS)
 k_dn_wgrad(DnGrid g, const unsigned* X, const unsigned* dY, float* part);

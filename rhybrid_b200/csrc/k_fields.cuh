@@ -335,11 +335,16 @@ __device__ __forceinline__ void cellFromStencil(const GridInfo& g, const Fields&
    }
 }
 
-// planes per block: fewer than NT_Z while the grid would leave SMs without one
-// resident wave of blocks (8 of 27.7 KB per SM); a plane more per block saves
-// the layer shared with the next block but is a plane more in a serial march.
-// (32^3 cells, 32 blocks of 8 planes: 60 us; 256 blocks of one: 17 us. 61 x 83 x
-// 70 cells: 62 -> 40 us. Grids that fill a wave with 8 planes keep them.)
+// planes per block of the node and of the cell pass: NT_Z, halved while the grid
+// has fewer than 148 * 8 blocks. A plane more per block saves the layer shared
+// with the next block but is a plane more in a serial march. The count is the
+// cell pass's (6 blocks of 27.7 KB per SM, 888 in a wave); the node pass (3 of 71
+// KB, 444) shares it. us with 1, 2, 4, 8 planes, the rule's choice in brackets:
+//    cells            node pass                     cell pass
+//    32^3             [12.5]  16.6   24.7   41.4    [9.0]   10.5   14.5   20.6
+//    61 x 83 x 70     [39.0]  38.0   38.0   51.6    20.8   [20.1]  18.9   21.3
+//    60 x 80 x 80     [39.5]  39.4   37.2   51.6    27.0   [24.9]  23.5   27.0
+//    120 x 160 x 160  258.5   250.2  255.2 [256.0]  151.2   137.7  133.5 [137.4]
 inline int layerPlanes(const GridInfo& g, int ty) {
    const long long cols = (long long)((g.nx + NT_X - 1) / NT_X) * ((g.ny + ty - 1) / ty);
    int nzb = NT_Z;

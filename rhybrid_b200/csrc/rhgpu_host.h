@@ -152,7 +152,7 @@ struct rhgpu_ctx {
    int* finc = nullptr;                 // arrivals per (species, segment)
    unsigned long long* mkey = nullptr;  // migration sort: 2 x mcap mover keys
    unsigned* mval = nullptr;            // 2 x mcap mover indices
-   unsigned* mbkt = nullptr;            // 2 x mcap destination buckets
+   unsigned* mbkt = nullptr;            // 2 x mcap: a mover's place among its destination's arrivals; the radix order: destination buckets
    long long mcap = 0;
    int* fmaxInc = nullptr;              // count of the buckets above MIG_RANK arrivals
    int* fover = nullptr;                // 16 bytes
